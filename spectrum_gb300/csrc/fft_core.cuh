@@ -650,17 +650,12 @@ SPX_DEV void local_fft(float2* s, const FftGeom& g, const Load& load, const floa
   local_passes<EPT>(s, g, 1, tw, tid, T);
 }
 
-// local_fft with the natural-order result handed to out(i, z), i < M: from
-// the last pass's registers for the compile-time plans, else read back from
-// shared memory after the last pass.  Ends without a barrier.
+// The runtime plan's local FFT with the natural-order result handed to
+// out(i, z), i < M, read back from shared memory after the last pass.  Ends
+// without a barrier.
 template <int EPT, typename Load, typename Out>
 SPX_DEV void local_fft_out(float2* s, const FftGeom& g, const Load& load, const float2* __restrict__ tw,
                            uint32_t tid, uint32_t T, const Out& out) {
-  if constexpr (EPT == 16) {
-    if (g.M == 16384 && T == 1024) return ct_local_fft_out<16384>(s, load, tw, tid, out);
-    if (g.M == 8192 && T == 512) return ct_local_fft_out<8192>(s, load, tw, tid, out);
-    if (g.M == 4096 && T == 256) return ct_local_fft_out<4096>(s, load, tw, tid, out);
-  }
   first_pass_dispatch<EPT>(s, g, load, tid, T);
   local_passes<EPT>(s, g, 1, tw, tid, T);
   for (uint32_t i = tid; i < g.M; i += T) out(i, s[sw(i)]);

@@ -1,0 +1,498 @@
+// fft_pair.cuh — local FFTs of power-of-two size (1024 .. 16384 points) whose
+// threads transform two neighbouring butterflies at once with packed FP32
+// arithmetic (add/mul/fma on two values per instruction, sm_100 and later).
+//
+// The compile-time plans of fft_core.cuh (CtPlan: same radix order, same
+// twiddle values, same operations in the same order on every element), so the
+// results are the bits of ct_local_fft; what changes is the data layout:
+//   * a register pair holds the same component of elements 2p and 2p + 1 (C2:
+//     both real parts, both imaginary parts), so every addition,
+//     multiplication and rotation by -i of two butterflies j = 2m, 2m + 1 is
+//     one instruction (or none), and a twiddle product is four;
+//   * shared memory holds 16-byte slots {re 2p, re 2p+1, im 2p, im 2p+1},
+//     moved by 128-bit accesses: half the shared-memory instructions and
+//     addresses per point;
+//   * twiddle tables hold the pair W^{r k}, W^{r (k+1)} (k even) in the same
+//     form, one 128-bit load for two points.
+// In every pass but the first the outputs of butterflies 2m, 2m + 1 (an even
+// stride) are neighbouring elements again; the first pass (stride 1) pairs the
+// outputs r, r + 1 of one butterfly when it stores.
+//
+// Why: the scalar passes issue ~85 instructions per point and reach 45-55 % of
+// the issue slots, with the FP32 pipe 30 % busy (ncu): issue slots and latency
+// bound them, not memory.  The packed forms run at the FP32 pipe's full rate
+// in half the issue slots (measured: 64 pair operations per clock and SM for
+// add, mul and fma, operand negation free).
+//
+// Contraction: spx_device.cuh's Dft leaves mul/add contraction to the
+// compiler; the forms below spell out the fused operations it chose (checked
+// bit for bit on the GPU by tests/test_gpu_pair_fft.py against the scalar
+// kernels).
+#pragma once
+
+#include "fft_core.cuh"
+
+namespace spx {
+
+// ---- packed arithmetic -------------------------------------------------------
+SPX_DEV float2 pk(float k) { return make_float2(k, k); }
+SPX_DEV float2 pneg(float2 a) { return make_float2(-a.x, -a.y); }
+SPX_DEV float2 padd(float2 a, float2 b) { return __fadd2_rn(a, b); }
+SPX_DEV float2 psub(float2 a, float2 b) { return __fadd2_rn(a, pneg(b)); }
+SPX_DEV float2 pmul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+SPX_DEV float2 pfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+
+// Two complex values: real parts and imaginary parts of elements 2p, 2p + 1.
+struct C2 {
+  float2 x, y;
+};
+SPX_DEV C2 c2add(C2 a, C2 b) { return C2{padd(a.x, b.x), padd(a.y, b.y)}; }
+SPX_DEV C2 c2sub(C2 a, C2 b) { return C2{psub(a.x, b.x), psub(a.y, b.y)}; }
+// a * w, the operations of cmul on both values
+SPX_DEV C2 c2mul(C2 a, C2 w) {
+  return C2{pfma(a.x, w.x, pneg(pmul(a.y, w.y))), pfma(a.x, w.y, pmul(a.y, w.x))};
+}
+// a * (wx + i wy), constants
+SPX_DEV C2 c2mulc(C2 a, float wx, float wy) {
+  return C2{pfma(a.x, pk(wx), pmul(a.y, pk(-wy))), pfma(a.x, pk(wy), pmul(a.y, pk(wx)))};
+}
+
+SPX_DEV void pdft4_tail(C2 s02, C2 d02, C2 s13, C2 d13, C2& a0, C2& a1, C2& a2, C2& a3) {
+  a0 = c2add(s02, s13);
+  a2 = c2sub(s02, s13);
+  a1 = C2{padd(d02.x, d13.y), psub(d02.y, d13.x)};  // d02 - i*d13
+  a3 = C2{psub(d02.x, d13.y), padd(d02.y, d13.x)};  // d02 + i*d13
+}
+SPX_DEV void pdft4(C2& a0, C2& a1, C2& a2, C2& a3) {
+  pdft4_tail(c2add(a0, a2), c2sub(a0, a2), c2add(a1, a3), c2sub(a1, a3), a0, a1, a2, a3);
+}
+
+template <int R>
+struct PDft;
+
+template <>
+struct PDft<2> {
+  static SPX_DEV void run(C2* v) {
+    const C2 t = v[0];
+    v[0] = c2add(t, v[1]);
+    v[1] = c2sub(t, v[1]);
+  }
+};
+template <>
+struct PDft<4> {
+  static SPX_DEV void run(C2* v) { pdft4(v[0], v[1], v[2], v[3]); }
+};
+template <>
+struct PDft<8> {
+  static SPX_DEV void run(C2* v) {
+    C2 e0 = v[0], e1 = v[2], e2 = v[4], e3 = v[6];
+    C2 o0 = v[1], o1 = v[3], o2 = v[5], o3 = v[7];
+    pdft4(e0, e1, e2, e3);
+    pdft4(o0, o1, o2, o3);
+    // o1 (1 - i)/sqrt2 = k t1, o2 (-i), o3 (-1 - i)/sqrt2 = k (t3.x, -t3.y)
+    const C2 t1{padd(o1.x, o1.y), psub(o1.y, o1.x)};
+    const C2 t3{psub(o3.y, o3.x), padd(o3.x, o3.y)};
+    const float2 k = pk(kS2), nk = pk(-kS2);
+    v[0] = c2add(e0, o0);
+    v[4] = c2sub(e0, o0);
+    v[1] = C2{pfma(t1.x, k, e1.x), pfma(t1.y, k, e1.y)};
+    v[5] = C2{pfma(t1.x, nk, e1.x), pfma(t1.y, nk, e1.y)};
+    v[2] = C2{padd(e2.x, o2.y), psub(e2.y, o2.x)};
+    v[6] = C2{psub(e2.x, o2.y), padd(e2.y, o2.x)};
+    v[3] = C2{pfma(t3.x, k, e3.x), pfma(t3.y, nk, e3.y)};
+    v[7] = C2{pfma(t3.x, nk, e3.x), pfma(t3.y, k, e3.y)};
+  }
+};
+template <>
+struct PDft<16> {
+  static SPX_DEV void run(C2* v) {
+    // columns n2: v[n2], v[n2 + 4], v[n2 + 8], v[n2 + 12] -> b[n2][k1] in place
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) pdft4(v[n2], v[4 + n2], v[8 + n2], v[12 + n2]);
+    const float2 k = pk(kS2), nk = pk(-kS2);
+    auto b = [&](int n2, int k1) -> C2& { return v[4 * k1 + n2]; };
+    b(1, 1) = c2mulc(b(1, 1), kC16, -kS16);
+    b(1, 3) = c2mulc(b(1, 3), kS16, -kC16);
+    b(3, 1) = c2mulc(b(3, 1), kS16, -kC16);
+    b(3, 3) = c2mulc(b(3, 3), -kC16, kS16);
+    // the rotations by odd multiples of pi/4 leave their factor k to the sums
+    C2 o[4][4];
+    {  // k1 = 0
+      C2 a0 = b(0, 0), a1 = b(1, 0), a2 = b(2, 0), a3 = b(3, 0);
+      pdft4(a0, a1, a2, a3);
+      o[0][0] = a0; o[0][1] = a1; o[0][2] = a2; o[0][3] = a3;
+    }
+    {  // k1 = 1: a2 = k (t.x, t.y)
+      const C2 z = b(2, 1), a0 = b(0, 1);
+      const C2 t{padd(z.x, z.y), psub(z.y, z.x)};
+      pdft4_tail(C2{pfma(t.x, k, a0.x), pfma(t.y, k, a0.y)}, C2{pfma(t.x, nk, a0.x), pfma(t.y, nk, a0.y)},
+                 c2add(b(1, 1), b(3, 1)), c2sub(b(1, 1), b(3, 1)), o[1][0], o[1][1], o[1][2], o[1][3]);
+    }
+    {  // k1 = 2: a1 = k (P.x, P.y), a2 = -i z, a3 = k (Q.x, -Q.y)
+      const C2 z1 = b(1, 2), z = b(2, 2), z3 = b(3, 2), a0 = b(0, 2);
+      const C2 P{padd(z1.x, z1.y), psub(z1.y, z1.x)}, Q{psub(z3.y, z3.x), padd(z3.x, z3.y)};
+      const float2 qx = pmul(Q.x, k), qy = pmul(Q.y, k);
+      pdft4_tail(C2{padd(a0.x, z.y), psub(a0.y, z.x)}, C2{psub(a0.x, z.y), padd(a0.y, z.x)},
+                 C2{pfma(P.x, k, qx), pfma(P.y, k, pneg(qy))}, C2{pfma(P.x, k, pneg(qx)), pfma(P.y, k, qy)},
+                 o[2][0], o[2][1], o[2][2], o[2][3]);
+    }
+    {  // k1 = 3: a2 = k (t.x, -t.y)
+      const C2 z = b(2, 3), a0 = b(0, 3);
+      const C2 t{psub(z.y, z.x), padd(z.x, z.y)};
+      pdft4_tail(C2{pfma(t.x, k, a0.x), pfma(t.y, nk, a0.y)}, C2{pfma(t.x, nk, a0.x), pfma(t.y, k, a0.y)},
+                 c2add(b(1, 3), b(3, 3)), c2sub(b(1, 3), b(3, 3)), o[3][0], o[3][1], o[3][2], o[3][3]);
+    }
+#pragma unroll
+    for (int k1 = 0; k1 < 4; ++k1)
+#pragma unroll
+      for (int k2 = 0; k2 < 4; ++k2) v[k1 + 4 * k2] = o[k1][k2];
+  }
+};
+
+// ---- shared-memory layout ------------------------------------------------------
+// Slot p (elements 2p, 2p + 1) at ps(p) = p + p/16: a quarter-warp's eight
+// 128-bit accesses hit eight different 16-byte banks for unit strides (every
+// pass's loads and the stores of strides >= 16) and for the stride-16 stores
+// of a first radix-16 pass.
+SPX_DEV uint32_t ps(uint32_t p) { return p + (p >> 4); }
+// 16-byte slots of an M-point local FFT (the bytes of sw_len(M) elements).
+constexpr uint32_t ps_len(uint32_t M) { return M / 2 + M / 32; }
+// Element i of the natural-order result in shared memory.
+SPX_DEV float2 pair_elem(const float4* s, uint32_t i) {
+  const float* f = reinterpret_cast<const float*>(s + ps(i >> 1)) + (i & 1u);
+  return make_float2(f[0], f[2]);
+}
+
+// ---- plans -----------------------------------------------------------------------
+// Entries (float4) of a pass's pair table: per twiddle row, Ns / 2 pairs; a
+// split radix-4 pass holds 32 pairs W^l, W^{l+1} (l < 64), then W^{64 j}
+// twice over (both values the same).
+constexpr uint32_t pair_tw_entries(uint32_t R, uint32_t Ns) {
+  return Ns < 2 ? 0u : tw_split(R, Ns) ? 32u + Ns / 64u : tw_rows(R) * (Ns / 2);
+}
+constexpr bool pair_size(uint32_t M) { return M >= 1024 && M <= 16384 && (M & (M - 1)) == 0; }
+
+template <int M>
+struct PairPlan : CtPlan<M> {
+  static_assert(pair_size((uint32_t)M), "power of two, 1024 .. 16384");
+  using P0 = CtPlan<M>;
+  static constexpr int T = M / 32;  // threads: two radix-16 butterflies each
+  static constexpr int ptwoff(int p) {
+    return p == 0 ? 0 : ptwoff(p - 1) + (int)pair_tw_entries((uint32_t)P0::radix(p - 1), (uint32_t)P0::ns(p - 1));
+  }
+};
+
+// ---- loads -------------------------------------------------------------------------
+SPX_DEV float4 ld_stream4(const float2* p) {
+  float4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
+
+// Samples n, n + 1 (n even) of a beam: window applied (load_sample's rounded
+// multiplies), zero beyond n_point.  16-byte loads when the beam starts on a
+// 16-byte boundary and n_point is even (no pair then straddles the end), else
+// two 8-byte loads that keep the line in L1 for the second.
+struct SamplePairs {
+  const float2* __restrict__ x;
+  uint32_t n_point;
+  const float* __restrict__ win;
+  bool vec;
+  SPX_DEV SamplePairs(const float2* x_, uint32_t n, const float* w)
+      : x(x_), n_point(n), win(w), vec(((reinterpret_cast<uintptr_t>(x_) & 15u) | (n & 1u)) == 0) {}
+  template <int R>
+  SPX_DEV void load(C2 (&v)[R], uint32_t n0, uint32_t step) const {
+    float4 a[R];
+    if (vec) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const uint32_t n = n0 + r * step;
+        a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (n < n_point) a[r] = ld_stream4(x + n);
+      }
+      if (win) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const uint32_t n = n0 + r * step;
+          if (n < n_point) {
+            const float2 w = __ldg(reinterpret_cast<const float2*>(win + n));
+            a[r] = make_float4(__fmul_rn(a[r].x, w.x), __fmul_rn(a[r].y, w.x), __fmul_rn(a[r].z, w.y),
+                               __fmul_rn(a[r].w, w.y));
+          }
+        }
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const uint32_t n = n0 + r * step;
+        const float2 b = n < n_point ? __ldg(x + n) : make_float2(0.f, 0.f);
+        const float2 c = n + 1 < n_point ? __ldg(x + n + 1) : make_float2(0.f, 0.f);
+        a[r] = make_float4(b.x, b.y, c.x, c.y);
+        if (win) {
+          const float w0 = n < n_point ? __ldg(win + n) : 0.f, w1 = n + 1 < n_point ? __ldg(win + n + 1) : 0.f;
+          a[r] = make_float4(__fmul_rn(b.x, w0), __fmul_rn(b.y, w0), __fmul_rn(c.x, w1), __fmul_rn(c.y, w1));
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = C2{make_float2(a[r].x, a[r].z), make_float2(a[r].y, a[r].w)};
+  }
+};
+
+// Elements n, n + 1 of a row written earlier by other CTAs (exchange slots):
+// L2-coherent 16-byte loads (rows start on 16-byte boundaries).
+struct ExchangePairs {
+  const float2* row;
+  template <int R>
+  SPX_DEV void load(C2 (&v)[R], uint32_t n0, uint32_t step) const {
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const float4 a = __ldcg(reinterpret_cast<const float4*>(row + n0 + r * step));
+      v[r] = C2{make_float2(a.x, a.z), make_float2(a.y, a.w)};
+    }
+  }
+};
+
+// ---- passes ------------------------------------------------------------------------
+template <int M, int T, typename Load>
+SPX_DEV void pair_first(float4* s, const Load& load, uint32_t tid) {
+  constexpr int R = CtPlan<M>::radix(0), B = M / R, Q = B / 2 / T;
+  static_assert(R % 2 == 0 && Q * 2 * T == B, "whole pairs");
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const uint32_t m = tid + q * T;
+    C2 v[R];
+    load.load(v, 2 * m, B);
+    PDft<R>::run(v);
+    // butterflies 2m, 2m + 1: slots m R + r/2 and m R + R/2 + r/2 (r even);
+    // R = 16: ps(16 m + c) = 17 m + c (c < 16); R = 8: 8 m + m/2 + c (c < 8)
+    static_assert(R == 16 || R == 8, "first radix");
+    float4* d = s + (R == 16 ? 17 * m : 8 * m + (m >> 1));
+#pragma unroll
+    for (int r = 0; r < R; r += 2) {
+      d[r / 2] = make_float4(v[r].x.x, v[r + 1].x.x, v[r].y.x, v[r + 1].y.x);
+      d[R / 2 + r / 2] = make_float4(v[r].x.y, v[r + 1].x.y, v[r].y.y, v[r + 1].y.y);
+    }
+  }
+  __syncthreads();
+}
+
+SPX_DEV C2 ld_tw(const float4* __restrict__ t) {
+  const float4 w = __ldg(t);
+  return C2{make_float2(w.x, w.y), make_float2(w.z, w.w)};
+}
+
+// Loads and twiddles of the butterflies 2m, 2m + 1 of pass P, then their DFT.
+template <int M, int P>
+SPX_DEV void pair_load(const float4* s, C2* v, uint32_t m) {
+  constexpr int R = CtPlan<M>::radix(P), H = M / R / 2;  // slots between inputs
+  static_assert(H % 16 == 0, "constant slot offsets");
+  const float4* p = s + ps(m);
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const float4 a = p[r * (H + H / 16)];
+    v[r] = C2{make_float2(a.x, a.y), make_float2(a.z, a.w)};
+  }
+}
+template <int M, int P>
+SPX_DEV void pair_butterfly(C2* v, const float4* __restrict__ tw, uint32_t m) {
+  constexpr int R = CtPlan<M>::radix(P), Ns = CtPlan<M>::ns(P);
+  const uint32_t kk = m & (Ns / 2 - 1);  // k / 2
+  const float4* t = tw + PairPlan<M>::ptwoff(P);
+  if constexpr (R == 4) {
+    C2 w1;
+    if constexpr (tw_split(4, Ns))
+      w1 = c2mul(ld_tw(t + 32 + (kk >> 5)), ld_tw(t + (kk & 31u)));
+    else
+      w1 = ld_tw(t + kk);
+    const C2 w2 = c2mul(w1, w1);
+    v[1] = c2mul(v[1], w1);
+    v[2] = c2mul(v[2], w2);
+    v[3] = c2mul(v[3], c2mul(w2, w1));
+  } else {
+#pragma unroll
+    for (int r = 1; r < R; ++r) v[r] = c2mul(v[r], ld_tw(t + (r - 1) * (Ns / 2) + kk));
+  }
+  PDft<R>::run(v);
+}
+
+// Pass P (not the first, not the last) in shared memory.
+template <int M, int P, int T>
+SPX_DEV void pair_pass(float4* s, const float4* __restrict__ tw, uint32_t tid) {
+  constexpr int R = CtPlan<M>::radix(P), Ns = CtPlan<M>::ns(P), Q = M / R / 2 / T, H = Ns / 2;
+  static_assert(Q == 1, "one pair of butterflies per thread");
+  C2 v[R];
+  pair_load<M, P>(s, v, tid);
+  __syncthreads();
+  pair_butterfly<M, P>(v, tw, tid);
+  // slot of output r: ((j - k) R + k) / 2 + r H with j = 2m; H divides 16 or is a multiple of it
+  const uint32_t kk = tid & (H - 1);
+  float4* d = s + ps((tid - kk) * R + kk);
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+    d[r * H + ((r * H) >> 4)] = make_float4(v[r].x.x, v[r].x.y, v[r].y.x, v[r].y.y);
+  __syncthreads();
+}
+template <int M, int P, int T>
+SPX_DEV void pair_passes_until_last(float4* s, const float4* __restrict__ tw, uint32_t tid) {
+  if constexpr (P + 1 < CtPlan<M>::npass) {
+    pair_pass<M, P, T>(s, tw, tid);
+    pair_passes_until_last<M, P + 1, T>(s, tw, tid);
+  }
+}
+
+// Last pass: out(i, z) takes elements i, i + 1 (i even) of the natural-order
+// result; consecutive threads get consecutive pairs.  Ends without a barrier.
+template <int M, int T, typename Out>
+SPX_DEV void pair_last(const float4* s, const float4* __restrict__ tw, uint32_t tid, const Out& out) {
+  constexpr int P = CtPlan<M>::npass - 1;
+  constexpr int R = CtPlan<M>::radix(P), B = M / R, Q = B / 2 / T;
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    const uint32_t m = tid + q * T;
+    C2 v[R];
+    pair_load<M, P>(s, v, m);
+    pair_butterfly<M, P>(v, tw, m);
+#pragma unroll
+    for (int r = 0; r < R; ++r) out(2 * m + r * B, v[r]);
+  }
+}
+
+// The whole local FFT (M / 32 threads): first pass from `load`, the result
+// handed to out(i, z) (pair_last); ends without a barrier.
+template <int M, typename Load, typename Out>
+SPX_DEV void pair_local_fft_out(float4* s, const Load& load, const float4* __restrict__ tw, uint32_t tid,
+                                const Out& out) {
+  constexpr int T = PairPlan<M>::T;
+  pair_first<M, T>(s, load, tid);
+  pair_passes_until_last<M, 1, T>(s, tw, tid);
+  pair_last<M, T>(s, tw, tid, out);
+}
+
+// Result back into the slots it was read from (element i at pair_elem(s, i)).
+struct SlotOut {
+  float4* s;
+  SPX_DEV void operator()(uint32_t i, C2 z) const { s[ps(i >> 1)] = make_float4(z.x.x, z.x.y, z.y.x, z.y.y); }
+};
+template <int M, typename Load>
+SPX_DEV void pair_local_fft(float4* s, const Load& load, const float4* __restrict__ tw, uint32_t tid) {
+  pair_local_fft_out<M>(s, load, tw, tid, SlotOut{s});
+  __syncthreads();
+}
+
+// ---- outputs -------------------------------------------------------------------------
+SPX_DEV float2 first_of(C2 z) { return make_float2(z.x.x, z.y.x); }
+SPX_DEV float2 second_of(C2 z) { return make_float2(z.x.y, z.y.y); }
+
+// Output of bins i, i + 1 of one beam's natural-order spectrum (the layouts
+// of store_bin); `out` is 16-byte aligned (8 bytes for magnitudes).
+template <int M, int MODE>
+struct BinOutPairs;
+constexpr int kPairComplex = 0, kPairMag = 1, kPairMagPhase = 2, kPairReversed = 3, kPairOther = 4;
+
+template <int M>
+struct BinOutPairs<M, kPairComplex> {
+  float4* row;
+  SPX_DEV BinOutPairs(void* out, uint32_t, float, const FftGeom&, uint32_t beam)
+      : row(reinterpret_cast<float4*>(out) + (size_t)beam * (M / 2)) {}
+  SPX_DEV void operator()(uint32_t i, C2 z) const { row[i >> 1] = make_float4(z.x.x, z.y.x, z.x.y, z.y.y); }
+};
+template <int M>
+struct BinOutPairs<M, kPairMag> {  // |X| or |X|^2, times scale
+  float2* row;
+  bool squared;
+  float scale;
+  SPX_DEV BinOutPairs(void* out, uint32_t mode, float sc, const FftGeom&, uint32_t beam)
+      : row(reinterpret_cast<float2*>(out) + (size_t)beam * (M / 2)), squared(mode == SPX_OUT_MAG2), scale(sc) {}
+  SPX_DEV void operator()(uint32_t i, C2 z) const {
+    float a = mag2_rn(first_of(z)), b = mag2_rn(second_of(z));
+    if (!squared) {
+      a = __fsqrt_rn(a);
+      b = __fsqrt_rn(b);
+    }
+    row[i >> 1] = make_float2(__fmul_rn(a, scale), __fmul_rn(b, scale));
+  }
+};
+template <int M>
+struct BinOutPairs<M, kPairMagPhase> {
+  float4* row;
+  SPX_DEV BinOutPairs(void* out, uint32_t, float, const FftGeom&, uint32_t beam)
+      : row(reinterpret_cast<float4*>(out) + (size_t)beam * (M / 2)) {}
+  SPX_DEV void operator()(uint32_t i, C2 z) const {
+    const float2 a = first_of(z), b = second_of(z);
+    row[i >> 1] = make_float4(mag_rn(a), atan2f(a.y, a.x), mag_rn(b), atan2f(b.y, b.x));
+  }
+};
+// Inverse transform: bin k goes to element (M - k) mod M, scaled.  A pair of
+// elements (p, p + 1), p even, holds bins i + 2 and i + 1 (p = M - i - 2): the
+// first comes from the next lane; the warp's ends are stored alone.
+template <int M>
+struct BinOutPairs<M, kPairReversed> {
+  float2* row;
+  float scale;
+  SPX_DEV BinOutPairs(void* out, uint32_t, float sc, const FftGeom&, uint32_t beam)
+      : row(reinterpret_cast<float2*>(out) + (size_t)beam * M), scale(sc) {}
+  SPX_DEV void operator()(uint32_t i, C2 z) const {
+    const uint32_t lane = threadIdx.x & 31u;
+    const float2 a = make_float2(__fmul_rn(z.x.x, scale), __fmul_rn(z.y.x, scale));
+    const float2 b = make_float2(__fmul_rn(z.x.y, scale), __fmul_rn(z.y.y, scale));
+    const float nx = __shfl_down_sync(0xffffffffu, a.x, 1), ny = __shfl_down_sync(0xffffffffu, a.y, 1);
+    if (lane == 0) row[i == 0 ? 0u : M - i] = a;
+    if (lane == 31)
+      row[M - i - 1] = b;
+    else
+      *reinterpret_cast<float4*>(row + (M - i - 2)) = make_float4(nx, ny, b.x, b.y);
+  }
+};
+template <int M>
+struct BinOutPairs<M, kPairOther> {  // any mode, any alignment
+  void* out;
+  uint32_t mode, beam;
+  float scale;
+  const FftGeom& g;
+  SPX_DEV BinOutPairs(void* o, uint32_t m, float sc, const FftGeom& gg, uint32_t b)
+      : out(o), mode(m), beam(b), scale(sc), g(gg) {}
+  SPX_DEV void operator()(uint32_t i, C2 z) const {
+    store_bin(out, mode, scale, g, beam, i, first_of(z));
+    store_bin(out, mode, scale, g, beam, i + 1, second_of(z));
+  }
+};
+
+// ---- cross stage -----------------------------------------------------------------------
+// cross_stage_exchange for two neighbouring columns n2, n2 + 1 per thread
+// (CR a power of two, M / CR even): the same operations on each column.
+template <int CR, int M, int T>
+SPX_DEV void pair_cross_stage(float2* __restrict__ slot, uint32_t c, const SamplePairs& load,
+                              const float2* __restrict__ twc, uint32_t tid) {
+  constexpr uint32_t S = M / CR;
+  static_assert(S % 2 == 0 && (S / 2) % T == 0, "whole pairs of columns");
+#pragma unroll 1
+  for (uint32_t q = tid; q < S / 2; q += T) {
+    const uint32_t n2 = c * S + 2 * q;
+    C2 v[CR];
+    load.load(v, n2, M);
+    const float4 t = __ldg(reinterpret_cast<const float4*>(twc + n2));
+    PDft<CR>::run(v);
+    auto put = [&](int k1, C2 z) {
+      __stcg(reinterpret_cast<float4*>(slot + (size_t)k1 * M + n2), make_float4(z.x.x, z.y.x, z.x.y, z.y.y));
+    };
+    put(0, v[0]);
+    C2 w[CR];
+    w[1] = C2{make_float2(t.x, t.z), make_float2(t.y, t.w)};
+#pragma unroll
+    for (int k1 = 2; k1 < CR; ++k1) w[k1] = (k1 % 2 == 0) ? c2mul(w[k1 / 2], w[k1 / 2]) : c2mul(w[k1 - 1], w[1]);
+#pragma unroll
+    for (int k1 = 1; k1 < CR; ++k1) put(k1, c2mul(v[k1], w[k1]));
+  }
+}
+
+// Elements i, i + 1 into a 16-byte aligned row of device memory.
+struct RowOutPairs {
+  float2* row;
+  SPX_DEV void operator()(uint32_t i, C2 z) const {
+    __stcg(reinterpret_cast<float4*>(row + i), make_float4(z.x.x, z.y.x, z.x.y, z.y.y));
+  }
+};
+
+}  // namespace spx

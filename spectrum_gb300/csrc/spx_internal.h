@@ -19,6 +19,7 @@ namespace spx {
 struct FftPlan {
   FftGeom g{};
   float2* d_tw_local = nullptr;  // M - 1 entries (>= 1 allocated)
+  float4* d_tw_pair = nullptr;   // the same twiddles in pairs (fft_pair.cuh; sizes of pair_size, else null)
   float2* d_tw_cross = nullptr;  // W_N^{n2}, M entries (big plans: W_N^{n2 k1} as [k1][n2], then W_Cb^e)
   bool big = false;              // three-launch transform (2^19, 2^20, 2^21 points)
   // Sizes without a direct plan: Bluestein's chirp-z transform through a
@@ -46,7 +47,9 @@ bool is_smooth23(uint32_t n);
 // per pass, tw_rows(R) rows of W_{Ns R}^{r k}, or the two factors of a split
 // radix-4 table (tw_split); g.twoff gives each pass's first entry.
 void fill_local_twiddles(const FftGeom& g, float2* twl);
-
+// Uploads plan->g's local twiddles in pairs (plan->d_tw_pair) where the pair
+// kernels of fft_pair.cuh take its local size.
+cudaError_t upload_pair_twiddles(FftPlan* plan, const float2* twl);
 
 }  // namespace spx
 

@@ -1,0 +1,63 @@
+"""GPU checks of the packed power-of-two kernels (fft_pair.cuh).
+
+They run the plans of the scalar kernels with two butterflies per thread, so
+every output is compared bit for bit with the scalar kernels, which a context
+tuned to 32 points per thread still runs (spx_set_fft_tuning): lengths that
+fill the transform, fall one short (odd: 8-byte loads), end inside it, and
+samples that start off a 16-byte boundary.
+"""
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+SIZES = [1024, 2048, 4096, 8192, 16384, 32768, 131072, 262144]
+MODES = ("complex", "mag", "mag2", "magphase")
+
+
+def _samples(beams, n, offset, seed):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(seed)
+    f = torch.randn(beams * n + offset, 2, generator=g, device="cuda")
+    return torch.view_as_complex(f)[offset:].reshape(beams, n)
+
+
+@pytest.fixture(scope="module")
+def scalar(spx):
+    """A context whose power-of-two transforms run the scalar kernels."""
+    from spectrum_gb300._capi import lib
+    c = spx.Context(0)
+    for nfft in SIZES:
+        c.check(lib.spx_set_fft_tuning(c.h, nfft, 32, 0))
+    return c
+
+
+def _same(a, b):
+    import torch
+    return torch.equal(a.view(torch.int32), b.view(torch.int32))
+
+
+@pytest.mark.parametrize("nfft", SIZES)
+def test_outputs_equal_the_scalar_kernels(spx, scalar, nfft):
+    for n, offset, window in ((nfft, 0, spx.WINDOW_HANN), (nfft - 1, 0, spx.WINDOW_BLACKMAN),
+                              (nfft // 2 + 2, 0, spx.WINDOW_NONE), (nfft - 2, 1, spx.WINDOW_HAMMING), (1, 1, 0)):
+        x = _samples(5, n, offset, nfft + n)
+        for out in MODES:
+            a, b = (spx.fft(x, nfft, window, out, 0.25, ctx=c) for c in (None, scalar))
+            assert _same(a, b), (nfft, n, offset, out)
+
+
+@pytest.mark.parametrize("nfft", SIZES)
+def test_inverse_and_unaligned_output_equal_the_scalar_kernels(spx, scalar, nfft):
+    import torch
+    x = _samples(3, nfft, 0, nfft)
+    ref = spx.ifft(x, ctx=scalar)
+    assert _same(spx.ifft(x), ref)
+    y = torch.empty(3 * nfft + 1, dtype=torch.complex64, device="cuda")[1:].reshape(3, nfft)
+    assert _same(spx.ifft(x, out=y), ref)
+    z = x.clone()
+    spx.ifft(z, out=z)
+    assert _same(z, ref)
+    half, full = (spx.fft_r2c(x.real.contiguous(), nfft, spx.WINDOW_HANN, f) for f in (False, True))
+    assert _same(half, spx.fft_r2c(x.real.contiguous(), nfft, spx.WINDOW_HANN, False, ctx=scalar))
+    assert _same(full, spx.fft_r2c(x.real.contiguous(), nfft, spx.WINDOW_HANN, True, ctx=scalar))
