@@ -101,15 +101,13 @@ fft_xl_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __re
     local_fft_out<EPT>(s, g, ExchangeLoader{row}, tw_local, tid, T, RowOut{row});
 }
 
-// The same transform as fft_xl_kernel for power-of-two local sizes M (M / 32
-// threads) and C in {2, 4, 8, 16}, on all SMs: a persistent cooperative
-// launch of G groups of C CTAs (one CTA per SM for M = 16384), group q
-// transforming beams q, q + G, ...; a bounded device-memory barrier per beam
-// (group_barrier) replaces the cluster barrier (clusters of 8 one-SM CTAs fit
-// on 120 of the 152 SMs).  Each CTA leaves its spectrum row in the beam's
-// exchange slot; rows_transpose_kernel then writes the output (the stride-C
-// stores of a direct epilogue cost more than the extra pass: 0.332 vs 0.313 ms
-// for 256 x 131072 points).
+// The same transform as fft_xl_kernel for local sizes of 4096 and 8192 points
+// (set by spx_set_fft_tuning; the default 16384-point plans of power-of-two
+// transforms run fft_mid.cu) and C in {2, 4, 8, 16}, on all SMs: a persistent
+// cooperative launch of G groups of C CTAs, group q transforming beams q,
+// q + G, ...; a bounded device-memory barrier per beam (group_barrier)
+// replaces the cluster barrier.  Each CTA leaves its spectrum row in the beam's
+// exchange slot; rows_transpose_kernel then writes the output.
 template <int M>
 __global__ void __launch_bounds__(M / 32, 16384 / M)
 fft_group_out_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __restrict__ win,
@@ -182,8 +180,7 @@ spx_status launch_rows_transpose(spx_ctx* ctx, const FftGeom& g, const float2* r
 }
 
 bool group_geometry(const FftGeom& g) {
-  return g.C > 1 && (g.C & (g.C - 1)) == 0 && g.ept == 16 && (g.M == 4096 || g.M == 8192 || g.M == 16384) &&
-         g.T == g.M / 16;
+  return g.C > 1 && (g.C & (g.C - 1)) == 0 && g.ept == 16 && (g.M == 4096 || g.M == 8192) && g.T == g.M / 16;
 }
 
 // ---------------------------------------------------------------------------
@@ -292,6 +289,7 @@ cudaError_t upload_pair_twiddles(FftPlan* plan, const float2* twl) {
 
 FftPlan::~FftPlan() {
   if (d_tw_pair) cudaFree(d_tw_pair);
+  if (d_tw_rows) cudaFree(d_tw_rows);
   if (d_tw_local) cudaFree(d_tw_local);
   if (d_tw_cross) cudaFree(d_tw_cross);
   if (d_chirp) cudaFree(d_chirp);
@@ -343,6 +341,7 @@ spx_status get_plan(spx_ctx* ctx, uint32_t nfft, const FftPlan** out) {
   e = cudaMemcpy(plan->d_tw_local, twl.data(), twl.size() * sizeof(float2), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemcpy(twiddles)");
   e = upload_pair_twiddles(plan.get(), twl.data());
+  if (e == cudaSuccess) e = upload_mid_twiddles(plan.get(), twl.data());
   if (e != cudaSuccess) return cuda_fail(ctx, e, "pair twiddles");
   if (g.C > 1) {  // W_N^{n2}, n2 < M: the cross stage raises it to W_N^{n2 k1}
     std::vector<float2> twc((size_t)g.M);
@@ -553,6 +552,11 @@ spx_status launch_fft_out(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
     if (e != cudaSuccess) return cuda_fail(ctx, e, "launch fft_out_kernel");
     return SPX_OK;
   }
+  // power-of-two sizes at the default local size: two launches of small CTAs
+  // against the beam groups and the transpose, 2^25 points in all:
+  // 32768 0.323 -> 0.247 ms, 65536 0.324 -> 0.230, 131072 0.326 -> 0.233,
+  // 262144 0.354 -> 0.250
+  if (plan.d_tw_rows) return launch_fft_mid(ctx, plan, d_in, beams, n_point, d_win, out_mode, scale, d_out);
   const size_t xch_bytes = ((size_t)beams * g.nfft * sizeof(float2) + 255) & ~(size_t)255;
   void* xch = nullptr;
   spx_status st = get_scratch(ctx, kSlotExchange, xch_bytes + (size_t)beams * sizeof(uint32_t), &xch);
@@ -562,9 +566,7 @@ spx_status launch_fft_out(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
     uint32_t* arrive = reinterpret_cast<uint32_t*>(static_cast<char*>(xch) + xch_bytes);
     e = cudaMemsetAsync(arrive, 0, (size_t)beams * sizeof(uint32_t), ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemsetAsync(group barriers)");
-    const void* kfn = g.M == 16384 ? (const void*)fft_group_out_kernel<16384>
-                      : g.M == 8192 ? (const void*)fft_group_out_kernel<8192>
-                                    : (const void*)fft_group_out_kernel<4096>;
+    const void* kfn = g.M == 8192 ? (const void*)fft_group_out_kernel<8192> : (const void*)fft_group_out_kernel<4096>;
     e = configure_kernel(kfn, kMaxFftSmem);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "configure fft_group_out_kernel");
     const uint32_t T = g.M / 32;

@@ -18,18 +18,22 @@
 // spx_topk: the same FFT code, |X| = sqrt_rn(re*re + im*im), the same
 // histogram-median threshold and the same comparisons.
 //
-// C > 1 (the beam's bins k = c + C*i are spread over the cluster): the
-// cluster FFT writes the bins of the search window into its exchange slot in
-// row layout (row c holds X[c + C*i]; the slot's rows are dead by then) and
-// maxima_cluster_kernel, one small cluster per beam and several clusters per
-// SM, loads |X| of contiguous bin ranges into shared memory, merges their
-// noise histograms through distributed shared memory, and classifies and
-// ranks the maxima.  Two launches instead of one: the per-beam threshold is a
-// dependency across the whole beam, and resolving it inside the FFT cluster
-// (one CTA per SM) left the SMs idle on barriers for ~40 % of the launch.
+// C > 1: the transform leaves the bins of the search window in device memory
+// (power-of-two sizes: the rows of fft_mid.cu; 3-smooth sizes and tuned local
+// sizes: row c of the cluster's or group's exchange slot holds X[c + C*i], the
+// slot's rows being dead by then) and maxima_cluster_kernel, one small cluster
+// per beam and several clusters per SM, loads |X| of contiguous bin ranges into
+// shared memory, merges their noise histograms through distributed shared
+// memory, and classifies and ranks the maxima.  A search of its own because the
+// per-beam threshold is a dependency across the whole beam: resolving it inside
+// the FFT cluster (one CTA per SM) left the SMs idle on barriers for ~40 % of
+// the launch.
 #include <cuda/atomic>
 
+#include <algorithm>
+
 #include "fft_core.cuh"
+#include "fft_pair.cuh"
 #include "mlp_device.cuh"
 #include "spx_internal.h"
 
@@ -42,6 +46,7 @@ struct FusedArgs {
   const float* win;
   const float2* tw_local;
   const float2* tw_cross;
+  const float4* tw_pair;    // local twiddles in pairs (packed kernels)
   float2* xch;              // exchange slots (C > 1), one per beam; then the window's bins
   uint32_t* arrive;         // [beams] group-barrier arrivals (C > 1), zeroed by the host
   uint32_t* err;            // device error word
@@ -361,12 +366,18 @@ SPX_DEV void write_window_row(float2* row, const float2* s, const FftGeom& g, ui
   discard_outside_window(row, g, w, tid, T);
 }
 
-// Output of the last local pass straight into the window part of the row.
-struct WindowRowOut {
+// Output of the last packed local pass straight into the window part of the
+// row (rows start on 16-byte boundaries).
+struct WindowRowOutPairs {
   float2* row;
   WindowRows w;
-  SPX_DEV void operator()(uint32_t i, float2 z) const {
-    if (i >= w.ilo && i < w.ihi) __stcg(row + i, z);
+  SPX_DEV void operator()(uint32_t i, C2 z) const {
+    if (i >= w.ilo && i + 1 < w.ihi) {
+      __stcg(reinterpret_cast<float4*>(row + i), make_float4(z.x.x, z.y.x, z.x.y, z.y.y));
+    } else {
+      if (i >= w.ilo && i < w.ihi) __stcg(row + i, first_of(z));
+      if (i + 1 >= w.ilo && i + 1 < w.ihi) __stcg(row + i + 1, second_of(z));
+    }
   }
 };
 
@@ -411,29 +422,28 @@ fft_peaks_kernel(FftGeom g, FusedArgs a) {
   write_window_row(row, s, g, c, a.start, a.end, tid, T);
 }
 
-// C > 1 with a power-of-two local size M (4096, 8192, 16384; M / 16 threads)
-// and C in {2, 4, 8, 16}: a persistent cooperative launch of G groups of C
-// CTAs (one CTA per SM); group q transforms beams q, q + G, ...  Per beam:
-// the cross stage into the beam's exchange slot, a group barrier, the local
-// FFT of row c, the window's bins into row c.  Clusters of 8 one-SM CTAs
-// fit on 120 of the 152 SMs; groups use all of them.
+// C > 1 with a local size M of 4096 or 8192 (spx_set_fft_tuning; M / 32
+// threads) and C in {2, 4, 8, 16}: a persistent cooperative launch of G groups
+// of C CTAs; group q transforms beams q, q + G, ...  Per beam: the cross stage
+// into the beam's exchange slot, a group barrier, the local FFT of row c, the
+// window's bins into row c.  Both stages run in packed arithmetic (fft_pair.cuh).
 template <int M>
-__global__ void __launch_bounds__(M / 16, 16384 / M)
+__global__ void __launch_bounds__(M / 32, 16384 / M)
 fft_group_kernel(FftGeom g, FusedArgs a, uint32_t groups) {
-  extern __shared__ float2 s[];
-  constexpr uint32_t T = M / 16;
+  extern __shared__ float4 s4[];
+  constexpr uint32_t T = M / 32;
   const uint32_t tid = threadIdx.x;
   const uint32_t grp = blockIdx.x / g.C, c = blockIdx.x - grp * g.C;
   // cross stage of a beam into its exchange slot, then this CTA's arrival
   auto cross = [&](uint32_t beam) {
     float2* slot = a.xch + (size_t)beam * g.nfft;
-    const SampleLoader ld{a.in + (size_t)beam * a.n_point, a.n_point, a.win};
+    const SamplePairs ld(a.in + (size_t)beam * a.n_point, a.n_point, a.win);
     prefetch_future_beam(g, a.in, a.n_point, beam, c, tid, T);
     switch (g.C) {
-      case 2: cross_stage_exchange<2>(slot, c, M, ld, a.tw_cross, tid, T); break;
-      case 4: cross_stage_exchange<4>(slot, c, M, ld, a.tw_cross, tid, T); break;
-      case 8: cross_stage_exchange<8>(slot, c, M, ld, a.tw_cross, tid, T); break;
-      default: cross_stage_exchange<16>(slot, c, M, ld, a.tw_cross, tid, T); break;
+      case 2: pair_cross_stage<2, M, T>(slot, c, ld, a.tw_cross, tid); break;
+      case 4: pair_cross_stage<4, M, T>(slot, c, ld, a.tw_cross, tid); break;
+      case 8: pair_cross_stage<8, M, T>(slot, c, ld, a.tw_cross, tid); break;
+      default: pair_cross_stage<16, M, T>(slot, c, ld, a.tw_cross, tid); break;
     }
     group_arrive(a.arrive + beam);
   };
@@ -449,9 +459,9 @@ fft_group_kernel(FftGeom g, FusedArgs a, uint32_t groups) {
     // the last pass writes the window's bins of the row straight from its
     // registers (no store to shared memory, barrier and reload)
     const WindowRows w = window_rows(g, c, a.start, a.end);
-    ct_local_fft_out<M>(s, ExchangeLoader{row}, a.tw_local, tid, WindowRowOut{row, w});
+    pair_local_fft_out<M>(s4, ExchangePairs{row}, a.tw_pair, tid, WindowRowOutPairs{row, w});
     discard_outside_window(row, g, w, tid, T);
-  }  // (the next beam's group_arrive barrier orders these reads of s before its first pass)
+  }  // (the next beam's group_arrive barrier orders these reads of s4 before its first pass)
 }
 
 // Self-test of the bounded wait: a single CTA arrives at a barrier that
@@ -483,6 +493,13 @@ spx_status launch_group_timeout_probe(spx_ctx* ctx, uint32_t* d_count) {
 //     this CTA; records written for ranks below the capacity.
 // The spectrum of beam b holds bin k at spec[b*nfft + (k mod C1)*M1 + k div C1]
 // (C1 = 1: natural order; C1 > 1: the cluster FFT's row layout).
+//
+// ROWS (C1 a power of two >= 32, the rows of fft_mid.cu): a CTA owns kw whole
+// columns q, bins q C1 .. q C1 + C1 - 1 each.  It reads them along the rows, two
+// columns per 16-byte load, keeps |X| as [row][column] in shared memory (every
+// access runs over the columns: no bank conflicts) and tests 32 consecutive
+// bins of one column per bitmap word.  Reading bin by bin would touch a line
+// per lane.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kMxThreads = 256;
 constexpr uint32_t kMxMinBlocks = 5;  // CTAs per SM the kernel is built for (<= 48 registers)
@@ -501,6 +518,7 @@ struct MxArgs {
   uint32_t c1shift;      // log2(C1) when C1 is a power of two, else 32
   uint32_t c1magic;      // ceil(2^32 / C1) (C1 not a power of two)
   uint32_t nfft, start, end, cap, refine, chunk;
+  uint32_t kw;           // rows form: columns per CTA (a power of two), chunk = C1 kw bins
   float fs, factor;      // factor <= 0: no threshold
 };
 
@@ -520,11 +538,20 @@ SPX_DEV float2 mx_load(const MxArgs& a, const float2* __restrict__ sb, uint32_t 
 // Shared memory (32-bit words): |X| [chunk + 2] | maxima bits [chunk/32] |
 // reductions [64] | with a threshold: 16-bit histogram [kHist/2] | merged
 // window [kMxMerge].
-static size_t mx_smem_words(uint32_t chunk, bool thr) {
-  return (size_t)chunk + 2 + (chunk + 31) / 32 + 64 + (thr ? kHist / 2 + kMxMerge : 0);
+static size_t mx_smem_words(uint32_t chunk, bool thr, bool rows) {
+  return (size_t)chunk + 2 + (chunk + 31) / 32 + 64 + (thr ? (rows ? kHist : kHist / 2) + kMxMerge : 0);
 }
 
-__global__ void __launch_bounds__(kMxThreads, kMxMinBlocks)
+// The largest of three values, NaN when one is: m > max3_nan(l, r, t) is
+// m > l && m > r && m > t, NaN included.
+SPX_DEV float max3_nan(float a, float b, float c) {
+  float d;
+  asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+  return d;
+}
+
+template <bool ROWS>
+__global__ void __launch_bounds__(kMxThreads, ROWS ? 4 : kMxMinBlocks)
 maxima_cluster_kernel(MxArgs a) {
   extern __shared__ uint32_t smx[];
   cg::cluster_group cl = cg::this_cluster();
@@ -534,14 +561,28 @@ maxima_cluster_kernel(MxArgs a) {
   float* smag = reinterpret_cast<float*>(smx);         // [chunk + 2]: bins lo - 1 .. hi
   uint32_t* bits = smx + a.chunk + 2;                   // [chunk / 32]
   uint32_t* red = bits + (a.chunk + 31) / 32;           // [64]
-  uint32_t* hist = red + 64;                            // [kHist / 2]: bucket b in half b & 1 of word b / 2
-  uint32_t* merged = hist + kHist / 2;                  // [kMxMerge]
-  const uint32_t lo = min(a.start + c * a.chunk, a.end);
-  const uint32_t hi = min(lo + a.chunk, a.end);
+  uint32_t* hist = red + 64;                            // [kHist / 2]: bucket b in half b & 1 of word b / 2 (ROWS: [kHist])
+  uint32_t* merged = hist + (ROWS ? kHist : kHist / 2);  // [kMxMerge]
+  // ROWS: whole columns from the even one at or below the window's start
+  const uint32_t lo = ROWS ? ((((a.start >> a.c1shift) & ~1u) + c * a.kw) << a.c1shift)
+                           : min(a.start + c * a.chunk, a.end);
+  const uint32_t hi = ROWS ? max(lo, min(lo + a.chunk, ((a.end + a.C1 - 1) >> a.c1shift) << a.c1shift))
+                           : min(lo + a.chunk, a.end);
   const uint32_t nb = hi - lo;
+  const uint32_t kwshift = ROWS ? 31u - __clz(a.kw) : 0u;
+  float* edge = smag + a.chunk;  // ROWS: |X| of bins lo - 1 and hi
+  // |X| of bin lo + i, -1 <= i <= nb
+  auto mag_at = [&](uint32_t i) {
+    if constexpr (ROWS) {
+      if (i >= nb) return edge[i == nb ? 1 : 0];
+      return smag[((i & (a.C1 - 1)) << kwshift) + (i >> a.c1shift)];
+    } else {
+      return smag[i + 1];
+    }
+  };
   const float2* sb = a.spec + (size_t)beam * a.nfft;
   if (thr_on) {
-    for (uint32_t b = tid; b < kHist / 2; b += kMxThreads) hist[b] = 0;
+    for (uint32_t b = tid; b < (ROWS ? kHist : kHist / 2); b += kMxThreads) hist[b] = 0;
     if (tid == 0) {
       red[0] = kHist;
       red[1] = 0;
@@ -551,7 +592,12 @@ maxima_cluster_kernel(MxArgs a) {
   // 1. (loads issued kMxBatch at a time per thread, so that enough bytes
   //    are in flight to cover the device-memory latency)
   uint32_t bmin = kHist, bmax = 0;
-  if (nb && tid < 2) smag[tid ? nb + 1 : 0] = mag_rn(mx_load(a, sb, tid ? hi : lo - 1));  // neighbours
+  if constexpr (ROWS) {  // the neighbours outside the chunk (defined where a bin of the window needs them)
+    if (nb && tid == 0 && lo >= a.start) edge[0] = mag_rn(mx_load(a, sb, lo - 1));
+    if (nb && tid == 1 && hi <= a.end) edge[1] = mag_rn(mx_load(a, sb, hi));
+  } else {
+    if (nb && tid < 2) smag[tid ? nb + 1 : 0] = mag_rn(mx_load(a, sb, tid ? hi : lo - 1));  // neighbours
+  }
   auto take = [&](uint32_t i, float2 z) {  // |X| of bin lo + i into shared memory and the histogram
     const float m = mag_rn(z);
     smag[i + 1] = m;
@@ -562,6 +608,83 @@ maxima_cluster_kernel(MxArgs a) {
       bmax = max(bmax, b);
     }
   };
+  if constexpr (ROWS) {
+    // column pair p of rows r0, r0 + step, ...: 2^hshift pairs per row
+    const uint32_t q0 = lo >> a.c1shift, nq = nb >> a.c1shift, hshift = kwshift - 1;
+    const uint32_t p = tid & ((1u << hshift) - 1), r0 = tid >> hshift, step = kMxThreads >> hshift;
+    const float2* src = sb + (size_t)r0 * a.M1 + q0 + 2 * p;
+    float* dst = smag + (r0 << kwshift) + 2 * p;
+    const size_t ds = (size_t)step * a.M1;
+    uint32_t umin = 0xFFFFFFFFu, umax = 0;  // smallest and largest |X|, as bits
+    // 32-bit counters: a bucket's byte offset is two instructions from the bits
+    auto count = [&](float m) {
+      atomicAdd(reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(hist) + ((__float_as_uint(m) >> 17) & (4 * kHist - 4))), 1u);
+    };
+    auto mags = [](float4 z) {  // both |X| (mag_rn's operations)
+      const float2 a2 = __fmul2_rn(make_float2(z.x, z.y), make_float2(z.x, z.y));
+      const float2 b2 = __fmul2_rn(make_float2(z.z, z.w), make_float2(z.z, z.w));
+      return make_float2(__fsqrt_rn(__fadd_rn(a2.x, a2.y)), __fsqrt_rn(__fadd_rn(b2.x, b2.y)));
+    };
+    if (nb == a.chunk) {
+      // whole columns: every bin counted without a test, the few outside the
+      // window taken out again
+      // (C1 / step = chunk / 512 is a multiple of 4; the next batch of loads is
+      // in flight while the current one is converted and counted)
+      float4 z[kMxBatch];
+#pragma unroll
+      for (uint32_t j = 0; j < kMxBatch; ++j) z[j] = __ldcs(reinterpret_cast<const float4*>(src + j * ds));
+      for (uint32_t r = r0; r < a.C1; r += kMxBatch * step, dst += kMxBatch * 2 * kMxThreads) {
+        src += kMxBatch * ds;
+        const bool more = r + kMxBatch * step < a.C1;
+        float4 zn[kMxBatch];
+#pragma unroll
+        for (uint32_t j = 0; j < kMxBatch; ++j)
+          if (more) zn[j] = __ldcs(reinterpret_cast<const float4*>(src + j * ds));
+#pragma unroll
+        for (uint32_t j = 0; j < kMxBatch; ++j) {
+          const float2 m = mags(z[j]);
+          *reinterpret_cast<float2*>(dst + j * 2 * kMxThreads) = m;
+          if (thr_on) {
+            count(m.x);
+            count(m.y);
+            umin = __vimin3_u32(umin, __float_as_uint(m.x), __float_as_uint(m.y));
+            umax = __vimax3_u32(umax, __float_as_uint(m.x), __float_as_uint(m.y));
+          }
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < kMxBatch; ++j) z[j] = zn[j];
+      }
+      if (thr_on && (lo < a.start || hi > a.end)) {
+        __syncthreads();
+        auto drop = [&](uint32_t k) {
+          atomicSub(reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(hist) +
+                                                ((__float_as_uint(mag_at(k - lo)) >> 17) & (4 * kHist - 4))), 1u);
+        };
+        for (uint32_t k = lo + tid; k < min(a.start, hi); k += kMxThreads) drop(k);
+        for (uint32_t k = max(a.end, lo) + tid; k < hi; k += kMxThreads) drop(k);
+      }
+    } else if (2 * p < nq) {
+      for (uint32_t r = r0; r < a.C1; r += step, src += ds, dst += 2 * kMxThreads) {
+        const float2 m = mags(__ldcs(reinterpret_cast<const float4*>(src)));
+        *reinterpret_cast<float2*>(dst) = m;
+        const uint32_t k = lo + ((2 * p) << a.c1shift) + r;
+        auto one = [&](uint32_t kk, float v) {
+          if (kk < a.start || kk >= a.end) return;
+          count(v);
+          umin = min(umin, __float_as_uint(v));
+          umax = max(umax, __float_as_uint(v));
+        };
+        if (thr_on) {
+          one(k, m.x);
+          one(k + a.C1, m.y);
+        }
+      }
+    }
+    if (umin <= umax) {
+      bmin = (umin & 0x7fffffffu) >> 19;
+      bmax = (umax & 0x7fffffffu) >> 19;
+    }
+  } else {
   // Power-of-two C1 divides kMxThreads: the kMxBatch bins lo + i0 + j*256 + tid
   // of a full batch lie in one row, 256 / C1 columns apart.
   const bool rows_fixed = a.c1shift < 32;
@@ -587,6 +710,7 @@ maxima_cluster_kernel(MxArgs a) {
       const uint32_t i = i0 + j * kMxThreads + tid;
       if (i < nb) take(i, z[j]);
     }
+  }
   }
   float thr = -INFINITY;
   if (thr_on) {
@@ -628,7 +752,9 @@ maxima_cluster_kernel(MxArgs a) {
         uint32_t sum = 0;
 #pragma unroll
         for (uint32_t cc = 0; cc < kMxMaxC2; ++cc)
-          if (cc < C2) sum += (cl.map_shared_rank(hist, cc)[b >> 1] >> ((b & 1u) * 16)) & 0xFFFFu;
+          if (cc < C2)
+            sum += ROWS ? cl.map_shared_rank(hist, cc)[b]
+                        : (cl.map_shared_rank(hist, cc)[b >> 1] >> ((b & 1u) * 16)) & 0xFFFFu;
         merged[t] = sum;
       }
       __syncthreads();
@@ -645,6 +771,29 @@ maxima_cluster_kernel(MxArgs a) {
   //    16-byte and one 8-byte load of |X| (bin i is smag[i + 1]); the 8
   //    lanes of a group of 32 bins merge their 4-bit pieces into the word.
   const uint32_t words = (nb + 31) / 32;
+  if constexpr (ROWS) {
+    // word (column q, rows 32 part .. + 31); consecutive threads, consecutive columns
+    const uint32_t parts = a.C1 / 32, nq = nb >> a.c1shift;
+    for (uint32_t i = tid; i < parts << kwshift; i += kMxThreads) {
+      const uint32_t q = i & (a.kw - 1), part = i >> kwshift;
+      if (q >= nq) continue;
+      const uint32_t b0 = (q << a.c1shift) + 32 * part;  // first bin of the word, from lo
+      const float* col = smag + ((32 * part) << kwshift) + q;
+      float l = mag_at(b0 - 1), m = col[0];
+      const uint32_t k0 = lo + b0;
+      uint32_t word = 0;
+#pragma unroll 8
+      for (uint32_t j = 0; j < 32; ++j) {
+        const float r = j < 31 ? col[(j + 1) << kwshift] : mag_at(b0 + 32);
+        if (m > max3_nan(l, r, thr)) word |= 1u << j;
+        l = m;
+        m = r;
+      }
+      if (k0 < a.start) word = a.start - k0 >= 32 ? 0u : word & (0xFFFFFFFFu << (a.start - k0));
+      if (k0 + 32 > a.end) word = k0 >= a.end ? 0u : word & (0xFFFFFFFFu >> (32 - (a.end - k0)));
+      bits[q * parts + part] = word;
+    }
+  } else
   for (uint32_t u = 0; u * 4 * kMxThreads < nb; ++u) {
     const uint32_t i = 4 * (u * kMxThreads + tid);
     uint32_t piece = 0;
@@ -708,7 +857,7 @@ maxima_cluster_kernel(MxArgs a) {
   for (uint32_t w = w0; w < w1 && rank < a.cap; ++w) {
     for (uint32_t t = bits[w]; t && rank < a.cap; t &= t - 1) {
       const uint32_t i = 32 * w + (__ffs(t) - 1), k = lo + i;
-      o[rank++] = fused_max(k, mx_load(a, sb, k), smag[i], smag[i + 1], smag[i + 2], bw, a.refine);
+      o[rank++] = fused_max(k, mx_load(a, sb, k), mag_at(i - 1), mag_at(i), mag_at(i + 1), bw, a.refine);
     }
   }
 }
@@ -736,6 +885,9 @@ static bool mx_geometry(uint32_t span, uint32_t* C2, uint32_t* chunk) {
   return true;
 }
 
+// Row layouts the ROWS form takes: 32 .. 256 rows, a power of two (fft_mid.cu).
+static bool mx_rows(uint32_t C1) { return C1 >= 32 && C1 <= 256 && (C1 & (C1 - 1)) == 0; }
+
 bool fused_mlp_supported(const FftGeom& g, uint32_t K) {
   return g.C == 1 && fused_supported(g, SPX_PEAK_TOPK) && K >= 1 && K <= 32 &&
          2 * (size_t)g.Mpad >= mlp_fused_words(g.T / 32, K);
@@ -758,6 +910,15 @@ spx_status launch_maxima_cluster(spx_ctx* ctx, const float2* d_spec, uint32_t C1
   if (!mx_geometry(end > start ? end - start : 0u, &C2, &chunk))
     return fail(ctx, SPX_ERR_INVALID_ARG, "maxima: search window too long");
   MxArgs a{};
+  const bool rows = mx_rows(C1);
+  if (rows) {  // 8192 bins per CTA, or the power of two times that which leaves <= 8 CTAs
+    const uint32_t q0 = (start / C1) & ~1u, q1 = end > start ? (end + C1 - 1) / C1 : q0;
+    uint32_t kw = 8192 / C1;
+    while ((q1 - q0 + kw - 1) / kw > kMxMaxC2) kw *= 2;
+    a.kw = kw;
+    chunk = kw * C1;
+    C2 = std::max<uint32_t>((q1 - q0 + kw - 1) / kw, 1u);
+  }
   a.spec = d_spec;
   a.ccount = d_ccount;
   a.out = reinterpret_cast<MaxValueDev*>(d_out);
@@ -774,8 +935,9 @@ spx_status launch_maxima_cluster(spx_ctx* ctx, const float2* d_spec, uint32_t C1
   a.chunk = chunk;
   a.fs = fs;
   a.factor = factor;
-  const size_t smem = mx_smem_words(chunk, factor > 0.0f) * sizeof(uint32_t);
-  cudaError_t e = configure_kernel((const void*)maxima_cluster_kernel, 227 * 1024);
+  const size_t smem = mx_smem_words(chunk, factor > 0.0f, rows) * sizeof(uint32_t);
+  const void* kfn = rows ? (const void*)maxima_cluster_kernel<true> : (const void*)maxima_cluster_kernel<false>;
+  cudaError_t e = configure_kernel(kfn, 227 * 1024);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "configure maxima_cluster_kernel");
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(beams * C2, 1, 1);
@@ -789,7 +951,8 @@ spx_status launch_maxima_cluster(spx_ctx* ctx, const float2* d_spec, uint32_t C1
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, maxima_cluster_kernel, a);
+  void* args[] = {(void*)&a};
+  e = cudaLaunchKernelExC(&cfg, kfn, args);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "launch maxima_cluster_kernel");
   return SPX_OK;
 }
@@ -812,6 +975,7 @@ spx_status launch_fft_peaks(spx_ctx* ctx, const FftPlan& plan, const float2* d_i
   a.win = d_win;
   a.tw_local = plan.d_tw_local;
   a.tw_cross = plan.d_tw_cross;
+  a.tw_pair = plan.d_tw_pair;
   a.out = reinterpret_cast<MaxValueDev*>(d_out);
   a.counts = d_counts;
   a.err = ctx->d_error;
@@ -836,6 +1000,21 @@ spx_status launch_fft_peaks(spx_ctx* ctx, const FftPlan& plan, const float2* d_i
     e = cudaLaunchKernel(kfn, dim3(beams), dim3(g.T), args, smem, ctx->stream);
     return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch fft_peaks_kernel");
   }
+  // power-of-two sizes at the default local size.  256 beams of 65536 points in
+  // 131072 bins, 6 sigma: 0.275 ms with the beam groups (FFT 0.192, search of
+  // their rows 0.080) -> 0.205 (columns 0.068, rows 0.066, search 0.066)
+  if (plan.d_tw_rows) {  // spectrum rows over the exchange scratch, then the maxima kernel
+    const size_t row_bytes = (size_t)beams * g.nfft * sizeof(float2);
+    void* p = nullptr;
+    spx_status st = get_scratch(ctx, kSlotExchange, row_bytes + (size_t)beams * kMxMaxC2 * sizeof(uint32_t), &p);
+    if (st != SPX_OK) return st;
+    float2* rows = static_cast<float2*>(p);
+    st = launch_fft_mid_rows(ctx, plan, d_in, beams, n_point, d_win, start - 1, std::min(end + 1, g.nfft), rows);
+    if (st != SPX_OK) return st;
+    return launch_maxima_cluster(ctx, rows, 16 * g.C, g.nfft / (16 * g.C), beams, g.nfft, start, end, cap_or_k, fs,
+                                 refine, factor, reinterpret_cast<uint32_t*>(static_cast<char*>(p) + row_bytes),
+                                 d_out, d_counts);
+  }
   // C > 1: scratch = exchange slots | per-CTA maxima counts | group-barrier arrivals
   const size_t xch_bytes = ((size_t)beams * g.nfft * sizeof(float2) + 255) & ~(size_t)255;
   const size_t cnt_bytes = ((size_t)beams * kMxMaxC2 * sizeof(uint32_t) + 255) & ~(size_t)255;
@@ -848,13 +1027,12 @@ spx_status launch_fft_peaks(spx_ctx* ctx, const FftPlan& plan, const float2* d_i
   if (group_geometry(g)) {
     e = cudaMemsetAsync(a.arrive, 0, (size_t)beams * sizeof(uint32_t), ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMemsetAsync(group barriers)");
-    const void* kfn = g.M == 16384 ? (const void*)fft_group_kernel<16384>
-                      : g.M == 8192 ? (const void*)fft_group_kernel<8192>
-                                    : (const void*)fft_group_kernel<4096>;
+    const void* kfn = g.M == 8192 ? (const void*)fft_group_kernel<8192> : (const void*)fft_group_kernel<4096>;
     e = configure_kernel(kfn, 227 * 1024);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "configure fft_group_kernel");
     // as many groups as can be resident at once (cooperative launch), at most one per beam
-    uint32_t groups = resident_ctas(kfn, g.T, smem, 1) / g.C;
+    const uint32_t T = g.M / 32;
+    uint32_t groups = resident_ctas(kfn, T, smem, 1) / g.C;
     if (groups > beams) groups = beams;
     if (groups == 0) return fail(ctx, SPX_ERR_CUDA, "fft_group_kernel: a group of CTAs does not fit the device");
     // prefetch distance: one round of the groups (also for samples in host
@@ -863,7 +1041,7 @@ spx_status launch_fft_peaks(spx_ctx* ctx, const FftPlan& plan, const float2* d_i
     void* args[] = {(void*)&g, (void*)&a, (void*)&groups};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(groups * g.C, 1, 1);
-    cfg.blockDim = dim3(g.T, 1, 1);
+    cfg.blockDim = dim3(T, 1, 1);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = ctx->stream;
     cudaLaunchAttribute attr[1];

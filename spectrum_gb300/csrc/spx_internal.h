@@ -20,6 +20,7 @@ struct FftPlan {
   FftGeom g{};
   float2* d_tw_local = nullptr;  // M - 1 entries (>= 1 allocated)
   float4* d_tw_pair = nullptr;   // the same twiddles in pairs (fft_pair.cuh; sizes of pair_size, else null)
+  float4* d_tw_rows = nullptr;   // row twiddles of the two-launch transforms (fft_mid.cu), else null
   float2* d_tw_cross = nullptr;  // W_N^{n2}, M entries (big plans: W_N^{n2 k1} as [k1][n2], then W_Cb^e)
   bool big = false;              // three-launch transform (2^19, 2^20, 2^21 points)
   // Sizes without a direct plan: Bluestein's chirp-z transform through a
@@ -120,6 +121,18 @@ spx_status launch_fft_big(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
                           uint32_t n_point, const float* d_win, uint32_t out_mode, float scale,
                           void* d_out);
 
+// Two-launch transforms of 32768 .. 262144 = C x 16384 points (fft_mid.cu).
+// The rows form leaves the spectrum in d_rows [beams][16 C][1024]: bin
+// rho + 16 C q is element q of row rho, defined for bins [klo, khi).
+bool mid_geometry(const FftGeom& g);
+cudaError_t upload_mid_twiddles(FftPlan* plan, const float2* twl);
+spx_status launch_fft_mid(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams,
+                          uint32_t n_point, const float* d_win, uint32_t out_mode, float scale,
+                          void* d_out);
+spx_status launch_fft_mid_rows(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams,
+                               uint32_t n_point, const float* d_win, uint32_t klo, uint32_t khi,
+                               float2* d_rows);
+
 // Transforms of more than 2^21 points: N1 x N2, both 2^a 3^b <= 16384 (fft_huge.cu).
 bool huge_size(uint32_t nfft);
 spx_status build_huge_plan(spx_ctx* ctx, uint32_t nfft, FftPlan* plan);
@@ -151,8 +164,8 @@ void mlp_device_params(const spx_mlp* mlp, const void** pb, const float** p, int
 // exchange-slot layout) to bin order in any output mode (fft_kernels.cu).
 spx_status launch_rows_transpose(spx_ctx* ctx, const FftGeom& g, const float2* rows, uint32_t beams,
                                  void* d_out, uint32_t out_mode, float scale);
-// Geometries the persistent beam-group kernels take (power-of-two local size
-// M in {4096, 8192, 16384} with M/16 threads, C in {2, 4, 8, 16}).
+// Geometries the persistent beam-group kernels take (local size M in {4096,
+// 8192}, C in {2, 4, 8, 16}).
 bool group_geometry(const FftGeom& g);
 // Self-test of the group barrier's bounded wait (one CTA, two arrivals expected).
 spx_status launch_group_timeout_probe(spx_ctx* ctx, uint32_t* d_count);

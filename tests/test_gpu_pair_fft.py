@@ -61,3 +61,25 @@ def test_inverse_and_unaligned_output_equal_the_scalar_kernels(spx, scalar, nfft
     half, full = (spx.fft_r2c(x.real.contiguous(), nfft, spx.WINDOW_HANN, f) for f in (False, True))
     assert _same(half, spx.fft_r2c(x.real.contiguous(), nfft, spx.WINDOW_HANN, False, ctx=scalar))
     assert _same(full, spx.fft_r2c(x.real.contiguous(), nfft, spx.WINDOW_HANN, True, ctx=scalar))
+
+
+@pytest.mark.parametrize("nfft", [32768, 65536, 131072, 262144])
+def test_maxima_of_row_spectra_equal_the_composed_search(spx, nfft):
+    """All maxima from the row layout of the two-launch transforms against the
+    transform in bin order and the search on it: windows that start and end
+    inside a column, cover one column, the whole spectrum or nothing."""
+    import torch
+    cb = nfft // 1024  # bins per column
+    x = _samples(3, nfft // 2 + 3, 0, nfft)
+    spec = spx.fft(x, nfft, spx.WINDOW_HANN)
+    for start, end in ((0, 0), (1, nfft), (cb - 1, cb + 1), (cb, 2 * cb), (5 * cb + 3, nfft // 2 + cb // 2 + 1),
+                       (nfft - 3, nfft), (cb + 1, cb + 2), (7, 7)):
+        for sigma in (0.0, 3.0):
+            kw = dict(search_start=start, search_end=end, max_per_beam=2000, refine=spx.REFINE_PARABOLIC,
+                      thresh_sigma=sigma, sample_rate=1e6)
+            out, counts = spx.fft_peaks(x, nfft, spx.WINDOW_HANN, spx.PEAK_ALL, **kw)
+            ref, rc = spx.all_maxima(spec, **kw)
+            assert torch.equal(counts, rc), (start, end, sigma)
+            for b in range(3):
+                n = min(int(rc[b]), ref.shape[1])
+                assert torch.equal(out[b, :n], ref[b, :n]), (start, end, sigma, b)
