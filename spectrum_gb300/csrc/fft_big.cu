@@ -3,9 +3,8 @@
 // repeat_count 2), beyond what one cluster holds on chip.
 //
 // nfft = Cb * M, n = M*n1 + n2, k = k1 + Cb*k2:
-//   launch 1 (big_cols_kernel; big_cols_pipe_kernel for 2^19): for each n2,
-//     the Cb-point DFT over n1 of the windowed, zero-padded samples, times
-//     W_N^{n2 k1}, written to scratch[beam][k1][n2] (device memory);
+//   launch 1 (big_cols_kernel): for each n2, the Cb-point DFT over n1 of the
+//     windowed, zero-padded samples, times W_N^{n2 k1}, written to scratch[beam][k1][n2] (device memory);
 //   2^19 and 2^20 (M = 4096, Cb = 128 or 256): launch 2 (big_rows4_kernel)
 //     transforms four rows k1 = 4r .. 4r+3 per CTA and writes bins
 //     4r .. 4r+3 + Cb*k2 of the output in the requested mode: runs of four
@@ -16,20 +15,24 @@
 //     requested mode in contiguous runs (a 16384-point row per CTA leaves no
 //     room for four rows, and stride-Cb stores straight from the row kernel
 //     kept its SMs waiting on the store queue: 0.63 ms for 64 x 2^20 points).
+// Both kernels run in packed arithmetic (fft_pair.cuh).  Measured, complex
+// output: 64 x 2^20 0.581 -> 0.512 ms (columns 0.317 -> 0.263, bound by the
+// latency of their loads at 15 warps per SM; rows 0.259 -> 0.25, one CTA per
+// SM whose phases do not overlap), 64 x 2^19 0.257 -> 0.247, 16 x 2^21 0.393 ->
+// 0.358.  Not kept: 32-byte stores per thread in the row kernel (32 x 2^20
+// 0.269 -> 0.294), five column CTAs per SM (96 registers, spills: 0.305).
 // All twiddles are FP64-generated and stored in FP32, which is what the
 // 120 dB dynamic range of the precision workload needs: W_N^{n2 k1}, k1 =
 // a + 16 b, as the product of two factor tables [a][n2] = W_N^{n2 a} and
-// [b][n2] = W_N^{16 n2 b} (a warp's 32 columns read 256 contiguous bytes of
-// each; a CTA's slice of the second, 4 KB, is read by all its warps from L1,
-// where the full [k1][n2] table of nfft entries came from L2: 64 x 2^20
-// 0.591 -> 0.580 ms, 128 x 2^19 0.479 -> 0.460 ms, max error vs FP64
-// 2.3e-7 -> 2.2e-7 of the peak); W_M from the local plan.  Replaces hipFFT's internal
+// [b][n2] = W_N^{16 n2 b} (a CTA's slice of the second is read by all its warps from L1,
+// where the full [k1][n2] table of nfft entries came from L2); W_M from the local plan.  Replaces hipFFT's internal
 // multi-pass plan for large sizes (src/fft_func/src/fft_processor_rocm.cpp:176-193).
 #include <algorithm>
 #include <cmath>
 #include <vector>
 
 #include "fft_core.cuh"
+#include "fft_pair.cuh"
 #include "spx_internal.h"
 
 namespace spx {
@@ -37,189 +40,105 @@ namespace spx {
 constexpr uint32_t kBigM = 16384;     // row length of the 2^21-point transform
 constexpr uint32_t kBigM4 = 4096;     // row length of the 2^19 / 2^20-point transforms
 constexpr uint32_t kRows4 = 4;        // rows per CTA of big_rows4_kernel
+constexpr int kCols256 = 16;          // columns per CTA of the 256-point column DFTs (32 KB tiles, four per SM)
 
 // Row length M of a big transform of nfft points.
 static uint32_t big_rows(uint32_t nfft) { return nfft <= (1u << 20) ? kBigM4 : kBigM; }
 
-// One CTA = 32 consecutive n2 columns x Cb rows (n1); lane = column, warp
-// t < G = row group (every warp access is 32 consecutive columns of one row:
-// 256-byte global runs, conflict-free shared rows); rows of M points.
+// One CTA = W consecutive n2 columns x Cb rows (n1); thread (p, t): column pair
+// p < W / 2 (packed arithmetic, fft_pair.cuh), row group t < G; rows of M points.
 // Cb = G x J: stage 1 is the J-point DFT over rows t + G j, on samples loaded
-// straight into registers (J loads in flight per thread); the shared tile
-// [Cb][32] only carries stage 1's outputs to stage 2, the G-point DFT over t.
-template <int CB, int G>
-__global__ void __launch_bounds__(32 * G)
+// straight into registers (J 16-byte loads in flight per thread); the shared
+// tile [Cb][W / 2] of 16-byte slots only carries stage 1's outputs to stage 2,
+// the G-point DFT over t.
+template <int CB, int G, int W>
+__global__ void __launch_bounds__(W / 2 * G, 512 / (W / 2 * G))
 big_cols_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __restrict__ win,
                 const float2* __restrict__ twN, uint32_t nfft, float2* __restrict__ scratch,
                 uint32_t ahead, uint32_t M) {
-  extern __shared__ float2 tile_raw[];
-  float2(*tile)[32] = reinterpret_cast<float2(*)[32]>(tile_raw);  // [CB][32]
-  const uint32_t tid = threadIdx.x;
-  const uint32_t beam = blockIdx.y, n2_0 = blockIdx.x * 32;
-  const float2* x = in + (size_t)beam * n_point;
-  {  // L2 prefetch of the 32-column tile of the CTA `ahead` places later
+  extern __shared__ float4 s4[];
+  constexpr uint32_t HP = W / 2, T = HP * G;
+  const uint32_t tid = threadIdx.x, p = tid % HP, t = tid / HP;
+  const uint32_t beam = blockIdx.y, c0 = blockIdx.x * W;
+  {  // L2 prefetch of the tile of the CTA `ahead` places later
     const uint64_t f = (uint64_t)blockIdx.y * gridDim.x + blockIdx.x + ahead;
-    if (ahead && f < (uint64_t)gridDim.x * gridDim.y && tid < CB) {
-      const uint32_t fb = (uint32_t)(f / gridDim.x), fc = (uint32_t)(f % gridDim.x) * 32;
-      const uint32_t lo = tid * M + fc, hi = min(lo + 32, n_point);
-      if (lo < hi) prefetch_l2(in + (size_t)fb * n_point + lo, (size_t)(hi - lo) * sizeof(float2), 0, 1);
+    if (ahead && f < (uint64_t)gridDim.x * gridDim.y) {
+      const uint32_t fb = (uint32_t)(f / gridDim.x), fc = (uint32_t)(f % gridDim.x) * W;
+      for (uint32_t r = tid; r < CB; r += T) {
+        const uint32_t lo = r * M + fc, hi = min(lo + W, n_point);
+        if (lo < hi) prefetch_l2(in + (size_t)fb * n_point + lo, (size_t)(hi - lo) * sizeof(float2), 0, 1);
+      }
     }
   }
-  const uint32_t col = tid & 31, t = tid >> 5;
   constexpr int J = CB / G;  // stage-1 radix
   static_assert(J == 16, "the W_N factor tables are built for k1 = a + 16 b");
+  const uint32_t n2 = c0 + 2 * p;
   // stage 1: thread t transforms rows t + G j (j < J), twiddles W_CB^{t a}
-  float2 v[J];
+  C2 v[J];
+  SamplePairs(in + (size_t)beam * n_point, n_point, win).load(v, t * M + n2, G * M);
+  PDft<J>::run(v);
 #pragma unroll
-  for (int j = 0; j < J; ++j) v[j] = load_sample(x, (t + G * j) * M + n2_0 + col, n_point, win);
-  Dft<J>::run(v);
-#pragma unroll
-  for (int a = 1; a < J; ++a) {
-    const uint32_t e = (t * a) % CB;
-    v[a] = cmul(v[a], __ldg(twN + (size_t)(J + G) * M + e));  // W_CB^e, after the two factor tables
+  for (int a = 0; a < J; ++a) {
+    if (a > 0) {
+      const float2 w = __ldg(twN + (size_t)(J + G) * M + (t * a) % CB);  // W_CB^e, after the two factor tables
+      v[a] = c2mul(v[a], C2{pk(w.x), pk(w.y)});
+    }
+    s4[(t + G * a) * HP + p] = make_float4(v[a].x.x, v[a].x.y, v[a].y.x, v[a].y.y);
   }
-#pragma unroll
-  for (int a = 0; a < J; ++a) tile[t + G * a][col] = v[a];
   __syncthreads();
   // stage 2: for a = t, t + G, ... (< J), the G-point DFT over t' of rows t' + G a -> k1 = a + J b
-#pragma unroll
-  for (uint32_t a = t; a < (uint32_t)J; a += G) {
-    float2 w[G];
-#pragma unroll
-    for (int tp = 0; tp < G; ++tp) w[tp] = tile[tp + G * a][col];
-    Dft<G>::run(w);
-    const uint32_t n2 = n2_0 + col;
-    float2* o = scratch + (size_t)beam * nfft + n2;
-    const float2 ta = __ldg(twN + (size_t)a * M + n2);  // W_N^{n2 a}
-#pragma unroll
-    for (int b = 0; b < G; ++b) {
-      const uint32_t k1 = a + J * b;  // W_N^{n2 k1} = W_N^{n2 a} W_N^{n2 J b}
-      o[(size_t)k1 * M] = cmul(w[b], cmul(ta, __ldg(twN + (size_t)(J + b) * M + n2)));
-    }
-  }
-}
-
-// 8-byte asynchronous copy global -> shared (zero-filled when src_bytes is 0).
-SPX_DEV void cp_async8(void* dst, const void* src, uint32_t src_bytes) {
-  const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(d), "l"(src), "r"(src_bytes) : "memory");
-}
-SPX_DEV void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-SPX_DEV void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-
-// The column DFTs of big_cols_kernel in a persistent loop over the tiles
-// f = blockIdx.x, blockIdx.x + gridDim.x, ... (beam f / tpb, columns
-// 32 (f mod tpb) ..): while a CTA transforms tile f, the samples of its next
-// tile stream into shared memory by asynchronous copies.  Each thread copies
-// exactly the elements it reads itself (rows t + G j of its column), so the
-// landing buffer needs no barrier; stage 1's outputs alternate between two
-// exchange tiles, so one CTA barrier per tile orders every access.  The
-// arithmetic is big_cols_kernel's: the same bits.
-template <int CB, int G>
-__global__ void __launch_bounds__(32 * G, 2)
-big_cols_pipe_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __restrict__ win,
-                     const float2* __restrict__ twN, uint32_t nfft, float2* __restrict__ scratch, uint32_t M,
-                     uint32_t tpb, uint32_t total) {
-  extern __shared__ float2 tile_raw[];
-  float2(*land)[32] = reinterpret_cast<float2(*)[32]>(tile_raw);                 // [CB][32]
-  float2(*xch0)[32] = reinterpret_cast<float2(*)[32]>(tile_raw + CB * 32);       // [CB][32]
-  float2(*xch1)[32] = reinterpret_cast<float2(*)[32]>(tile_raw + 2 * CB * 32);   // [CB][32]
-  constexpr int J = CB / G;  // stage-1 radix
-  static_assert(J == 16, "the W_N factor tables are built for k1 = a + 16 b");
-  const uint32_t tid = threadIdx.x, col = tid & 31, t = tid >> 5;
-  auto issue = [&](uint32_t f) {  // this thread's samples of tile f into its landing slots
-    const uint32_t beam = f / tpb, n2_0 = (f - beam * tpb) * 32;
-    const float2* x = in + (size_t)beam * n_point;
-#pragma unroll
-    for (int j = 0; j < J; ++j) {
-      const uint32_t n = (t + G * j) * M + n2_0 + col;
-      const bool ok = n < n_point;
-      cp_async8(&land[t + G * j][col], ok ? x + n : x, ok ? 8u : 0u);
-    }
-    cp_async_commit();
+  auto pair_tw = [&](uint32_t row) {  // W_N factor of columns n2, n2 + 1
+    const float4 w = __ldg(reinterpret_cast<const float4*>(twN + (size_t)row * M + n2));
+    return C2{make_float2(w.x, w.z), make_float2(w.y, w.w)};
   };
-  uint32_t f = blockIdx.x;
-  if (f < total) issue(f);
-  for (uint32_t it = 0; f < total; ++it, f += gridDim.x) {
-    const uint32_t beam = f / tpb, n2_0 = (f - beam * tpb) * 32;
-    cp_async_wait_all();  // this thread's copies of tile f have landed
-    float2 v[J];
+  float2* o = scratch + (size_t)beam * nfft + n2;
+#pragma unroll 1
+  for (uint32_t a = t; a < (uint32_t)J; a += G) {
+    C2 w[G];
 #pragma unroll
-    for (int j = 0; j < J; ++j) v[j] = land[t + G * j][col];
-    if (win) {  // window of the samples inside the beam (load_sample's arithmetic)
-#pragma unroll
-      for (int j = 0; j < J; ++j) {
-        const uint32_t n = (t + G * j) * M + n2_0 + col;
-        if (n < n_point) {
-          const float w = __ldg(win + n);
-          v[j].x = __fmul_rn(v[j].x, w);
-          v[j].y = __fmul_rn(v[j].y, w);
-        }
-      }
+    for (int tp = 0; tp < G; ++tp) {
+      const float4 z = s4[(tp + G * a) * HP + p];
+      w[tp] = C2{make_float2(z.x, z.y), make_float2(z.z, z.w)};
     }
-    Dft<J>::run(v);
+    PDft<G>::run(w);
+    const C2 ta = pair_tw(a);  // W_N^{n2 a}
 #pragma unroll
-    for (int a = 1; a < J; ++a) {
-      const uint32_t e = (t * a) % CB;
-      v[a] = cmul(v[a], __ldg(twN + (size_t)(J + G) * M + e));  // W_CB^e
-    }
-    float2(*xch)[32] = (it & 1u) ? xch1 : xch0;
-#pragma unroll
-    for (int a = 0; a < J; ++a) xch[t + G * a][col] = v[a];
-    // the stores above depend on every landed value, so this thread's reads
-    // of its landing slots are complete before the slots are refilled
-    if (f + gridDim.x < total) issue(f + gridDim.x);
-    __syncthreads();
-    const uint32_t n2 = n2_0 + col;
-    float2* o = scratch + (size_t)beam * nfft + n2;
-#pragma unroll
-    for (uint32_t a = t; a < (uint32_t)J; a += G) {
-      float2 w[G];
-#pragma unroll
-      for (int tp = 0; tp < G; ++tp) w[tp] = xch[tp + G * a][col];
-      Dft<G>::run(w);
-      const float2 ta = __ldg(twN + (size_t)a * M + n2);  // W_N^{n2 a}
-#pragma unroll
-      for (int b = 0; b < G; ++b) {
-        const uint32_t k1 = a + J * b;  // W_N^{n2 k1} = W_N^{n2 a} W_N^{n2 J b}
-        o[(size_t)k1 * M] = cmul(w[b], cmul(ta, __ldg(twN + (size_t)(J + b) * M + n2)));
-      }
+    for (int b = 0; b < G; ++b) {  // k1 = a + J b: W_N^{n2 k1} = W_N^{n2 a} W_N^{n2 J b}
+      const C2 z = c2mul(w[b], c2mul(ta, pair_tw(J + b)));
+      __stcg(reinterpret_cast<float4*>(o + (size_t)(a + J * b) * M), make_float4(z.x.x, z.y.x, z.x.y, z.y.y));
     }
   }
 }
 
-template <int EPT>
-__global__ void __launch_bounds__(kMaxLocal / EPT, 1)
-big_rows_kernel(FftGeom g, const float2* __restrict__ tw_local, float2* __restrict__ scratch) {
-  extern __shared__ float2 s[];
-  const uint32_t tid = threadIdx.x, T = blockDim.x;
-  const uint32_t beam = blockIdx.x / g.C, k1 = blockIdx.x % g.C;
-  float2* row = scratch + (size_t)beam * g.nfft + (size_t)k1 * g.M;
+// Rows of 16384 points (2^21), each written back over itself.
+__global__ void __launch_bounds__(512, 1)
+big_rows_kernel(FftGeom g, const float4* __restrict__ tw_pair, float2* __restrict__ scratch) {
+  extern __shared__ float4 s4[];
+  const uint32_t tid = threadIdx.x;
+  float2* row = scratch + (size_t)blockIdx.x * g.M;
   if (g.ahead && blockIdx.x + g.ahead < gridDim.x)  // the row the CTA one wave later reads
-    prefetch_l2(row + (size_t)g.ahead * g.M, (size_t)g.M * sizeof(float2), tid, T);
-  // the row was read by this CTA alone (first pass, before its barrier)
-  if constexpr (EPT == 16) {
-    if (g.M == 16384 && T == 1024) {  // the last pass writes the row from its registers
-      ct_local_fft_out<16384>(s, SampleLoader{row, g.M, nullptr}, tw_local, tid, RowOutStream{row});
-      return;
-    }
-  }
-  local_fft<EPT>(s, g, SampleLoader{row, g.M, nullptr}, tw_local, tid, T);
-  for (uint32_t i = tid; i < g.M; i += T) __stcs(row + i, s[sw(i)]);
+    prefetch_l2(row + (size_t)g.ahead * g.M, (size_t)g.M * sizeof(float2), tid, 512);
+  // the row is read by this CTA alone (first pass, before its barrier)
+  pair_local_fft_out<(int)kBigM>(s4, ExchangePairs{row}, tw_pair, tid, RowOutPairs{row});
 }
 
-// Four rows k1 = r0 .. r0+3 of 4096 points per CTA (four groups of 256
-// threads, one row each, in shared memory rows kRowPad4 elements apart), then
-// the bins r0 + q + Cb*k2 (q < 4) in the requested mode: each run of four
-// bins is one 32-byte sector of the output.  The row pitch puts the four rows
-// of one k2 on different bank pairs for a half-warp's reads.
-constexpr uint32_t kRowPad4 = sw_len(kBigM4) + 4;
+// Four rows k1 = r0 .. r0+3 of 4096 points per CTA in packed arithmetic
+// (fft_pair.cuh).  The first two passes run one row per group of 128 threads
+// behind the group's own barriers; in the last one the rows are interleaved
+// over the lanes (thread (q, t): row r0 + q, butterflies 2t, 2t + 1), so its
+// registers hold one element of neighbouring rows in neighbouring lanes and go
+// out in the requested mode as runs of four bins, 32-byte sectors.  Row pitch
+// in slots: the four lanes of one element and two neighbouring slots of each
+// hit eight different 16-byte banks.
+constexpr uint32_t kRowPitch4 = ps_len(kBigM4) + 2;
+constexpr int kBigComplex = 0, kBigMag = 1, kBigMagPhase = 2, kBigOther = 3;
 
-__global__ void __launch_bounds__(kRows4 * 256, 1)
-big_rows4_kernel(FftGeom g, const float2* __restrict__ tw_local, const float2* __restrict__ scratch,
+template <int MODE>
+__global__ void __launch_bounds__(kRows4 * 128, 1)
+big_rows4_kernel(FftGeom g, const float4* __restrict__ tw_pair, const float2* __restrict__ scratch,
                  void* __restrict__ out, uint32_t out_mode, float scale) {
-  extern __shared__ float2 s[];
-  constexpr uint32_t TG = 256;
+  extern __shared__ float4 s4[];
+  constexpr int TG = 128, M = (int)kBigM4;
   const uint32_t tid = threadIdx.x, grp = tid / TG;
   const uint32_t per_beam = g.C / kRows4;
   const uint32_t beam = blockIdx.x / per_beam, r0 = (blockIdx.x - beam * per_beam) * kRows4;
@@ -229,12 +148,43 @@ big_rows4_kernel(FftGeom g, const float2* __restrict__ tw_local, const float2* _
   if (g.ahead && blockIdx.x + g.ahead < gridDim.x)
     prefetch_l2(scratch + (size_t)(blockIdx.x + g.ahead) * (kRows4 * kBigM4), kRows4 * kBigM4 * sizeof(float2), tid,
                 kRows4 * TG);
-  // every group runs the same passes, so the plan's CTA barriers hold for all four
-  ct_local_fft<(int)kBigM4, (int)TG>(s + (size_t)grp * kRowPad4, SampleLoader{row, kBigM4, nullptr}, tw_local,
-                                     tid - grp * TG);
-  for (uint32_t e = tid; e < kRows4 * kBigM4; e += kRows4 * TG) {
-    const uint32_t k2 = e / kRows4, q = e - k2 * kRows4;
-    store_bin(out, out_mode, scale, g, beam, r0 + q + g.C * k2, s[(size_t)q * kRowPad4 + sw(k2)]);
+  float4* s = s4 + grp * kRowPitch4;
+  pair_first<M, TG, GroupSync<TG>>(s, ExchangePairs{row}, tid - grp * TG);
+  pair_passes_until_last<M, 1, TG, GroupSync<TG>>(s, tw_pair, tid - grp * TG);
+  __syncthreads();
+  const uint32_t q = tid % kRows4, k1 = r0 + q;
+  float4* sq = s4 + q * kRowPitch4;
+  if constexpr (MODE == kBigOther || MODE == kBigMagPhase) {
+    // through shared memory: the last pass's registers leave no room for the
+    // long output functions
+    pair_last<M, TG>(sq, tw_pair, tid / kRows4, SlotOut{sq});
+    __syncthreads();
+#pragma unroll 4
+    for (uint32_t p = tid / kRows4; p < kBigM4 / 2; p += TG) {
+      const float4 z = sq[ps(p)];
+      if constexpr (MODE == kBigMagPhase) {
+        float2* o = reinterpret_cast<float2*>(out) + (size_t)beam * g.nfft + k1 + (size_t)g.C * (2 * p);
+        o[0] = make_float2(mag_rn(make_float2(z.x, z.z)), atan2f(z.z, z.x));
+        o[g.C] = make_float2(mag_rn(make_float2(z.y, z.w)), atan2f(z.w, z.y));
+        continue;
+      }
+      store_bin(out, out_mode, scale, g, beam, k1 + g.C * (2 * p), make_float2(z.x, z.z));
+      store_bin(out, out_mode, scale, g, beam, k1 + g.C * (2 * p + 1), make_float2(z.y, z.w));
+    }
+  } else {
+    pair_last<M, TG>(sq, tw_pair, tid / kRows4, [&](uint32_t e, C2 z) {
+      const size_t at = (size_t)beam * g.nfft + k1 + (size_t)g.C * e;
+      const float2 a = first_of(z), b = second_of(z);
+      if constexpr (MODE == kBigComplex) {
+        reinterpret_cast<float2*>(out)[at] = a;
+        reinterpret_cast<float2*>(out)[at + g.C] = b;
+      } else {
+        float* o = reinterpret_cast<float*>(out);
+        const float a2 = mag2_rn(a), b2 = mag2_rn(b);
+        o[at] = __fmul_rn(out_mode == SPX_OUT_MAG2 ? a2 : __fsqrt_rn(a2), scale);
+        o[at + g.C] = __fmul_rn(out_mode == SPX_OUT_MAG2 ? b2 : __fsqrt_rn(b2), scale);
+      }
+    });
   }
 }
 
@@ -269,6 +219,7 @@ spx_status build_big_plan(spx_ctx* ctx, uint32_t nfft, FftPlan* plan) {
   for (uint32_t e = 0; e < cb; ++e) twn[(size_t)(J + G) * M + e] = w_n((uint64_t)e * M);
   cudaError_t e = cudaMalloc(&plan->d_tw_local, twl.size() * sizeof(float2));
   if (e == cudaSuccess) e = cudaMemcpy(plan->d_tw_local, twl.data(), twl.size() * sizeof(float2), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = upload_pair_twiddles(plan, twl.data());
   if (e == cudaSuccess) e = cudaMalloc(&plan->d_tw_cross, twn.size() * sizeof(float2));
   if (e == cudaSuccess) e = cudaMemcpy(plan->d_tw_cross, twn.data(), twn.size() * sizeof(float2), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "big plan tables");
@@ -286,63 +237,43 @@ spx_status launch_fft_big(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
   float2* scratch = static_cast<float2*>(scr);
   const uint32_t M = g.M;
   // Cb = 128 (2^19 as 128 x 4096, 2^21 as 128 x 16384: 8 x 16) or 256 (2^20
-  // as 256 x 4096: 16 x 16, 512 threads, two 16-point stages)
-  const uint32_t cthreads = g.C == 256 ? 512u : 256u;
-  cudaError_t e = cudaSuccess;
-  if (g.C == 128 && M == kBigM4 && !ctx->input_on_host) {
-    // 2^19, samples in device memory: the pipelined column kernel (96 KiB,
-    // two 256-thread CTAs per SM).
-    // Measured against big_cols_kernel (back-to-back calls, same bits):
-    // 128 x 2^19 0.505 -> 0.480 ms; for 2^20 (192 KiB, one 512-thread CTA per
-    // SM) 0.591 -> 0.615 ms and for 2^21 0.692 -> 0.696 ms, so those keep
-    // big_cols_kernel.
-    const void* kfn = (const void*)big_cols_pipe_kernel<128, 8>;
-    const size_t smem = 3 * (size_t)g.C * 32 * sizeof(float2);  // landing tile + two exchange tiles
-    e = configure_kernel(kfn, smem);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "configure big_cols_pipe_kernel");
-    const uint32_t tpb = M / 32, total = tpb * beams;
-    const uint32_t resident = resident_ctas(kfn, cthreads, smem, 1);
-    if (resident == 0) return fail(ctx, SPX_ERR_CUDA, "big_cols_pipe_kernel: no resident CTA");
-    const uint32_t ctas = std::min(total, resident);
-    void* args[] = {(void*)&d_in,    (void*)&n_point, (void*)&d_win, (void*)&plan.d_tw_cross, (void*)&g.nfft,
-                    (void*)&scratch, (void*)&M,       (void*)&tpb,   (void*)&total};
-    e = cudaLaunchKernel(kfn, dim3(ctas), dim3(cthreads), args, smem, ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "launch big_cols_pipe_kernel");
-  } else {
-    const void* kcols =
-        g.C == 256 ? (const void*)big_cols_kernel<256, 16> : (const void*)big_cols_kernel<128, 8>;
-    const size_t csmem = (size_t)g.C * 32 * sizeof(float2);
-    e = configure_kernel(kcols, csmem);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "configure big_cols_kernel");
-    const uint32_t ahead_cols = ctx->input_on_host ? 0u : resident_ctas(kcols, cthreads, csmem, 1);
-    void* cargs[] = {(void*)&d_in, (void*)&n_point, (void*)&d_win, (void*)&plan.d_tw_cross, (void*)&g.nfft,
-                     (void*)&scratch, (void*)&ahead_cols, (void*)&M};
-    e = cudaLaunchKernel(kcols, dim3(M / 32, beams), dim3(cthreads), cargs, csmem, ctx->stream);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "launch big_cols_kernel");
-  }
-  if (M == kBigM4) {  // four rows per CTA, bin order written directly
-    const void* kfn = (const void*)big_rows4_kernel;
-    const size_t smem = (size_t)kRows4 * kRowPad4 * sizeof(float2);
-    e = configure_kernel(kfn, smem);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "configure big_rows4_kernel");
-    FftGeom gg = g;
-    gg.beams = beams;
-    gg.ahead = ctx->input_on_host ? 0u : resident_ctas(kfn, kRows4 * 256, smem, 1);
-    const float2* twl = plan.d_tw_local;
-    const float2* scr_c = scratch;
-    void* args[] = {(void*)&gg, (void*)&twl, (void*)&scr_c, (void*)&d_out, (void*)&out_mode, (void*)&scale};
-    e = cudaLaunchKernel(kfn, dim3(beams * (g.C / kRows4)), dim3(kRows4 * 256), args, smem, ctx->stream);
-    return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch big_rows4_kernel");
-  }
-  const void* kfn = (const void*)big_rows_kernel<kEPTDefault>;
-  e = configure_kernel(kfn, kMaxFftSmem);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "configure big_rows_kernel");
+  // as 256 x 4096: 16 x 16)
+  const uint32_t W = g.C == 256 ? kCols256 : 32u, cthreads = W / 2 * (g.C / 16);
+  const void* kcols = g.C == 256 ? (const void*)big_cols_kernel<256, 16, kCols256>
+                                 : (const void*)big_cols_kernel<128, 8, 32>;
+  const size_t csmem = (size_t)g.C * W * sizeof(float2);
+  cudaError_t e = configure_kernel(kcols, csmem);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "configure big_cols_kernel");
+  const uint32_t ahead_cols = ctx->input_on_host ? 0u : resident_ctas(kcols, cthreads, csmem, 1);
+  void* cargs[] = {(void*)&d_in, (void*)&n_point, (void*)&d_win, (void*)&plan.d_tw_cross, (void*)&g.nfft,
+                   (void*)&scratch, (void*)&ahead_cols, (void*)&M};
+  e = cudaLaunchKernel(kcols, dim3(M / W, beams), dim3(cthreads), cargs, csmem, ctx->stream);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "launch big_cols_kernel");
+  const float4* twp = plan.d_tw_pair;
   FftGeom gg = g;
   gg.beams = beams;
-  gg.ahead = resident_ctas(kfn, g.T, (size_t)g.Mpad * sizeof(float2), 1);
-  const float2* twl = plan.d_tw_local;
-  void* args[] = {(void*)&gg, (void*)&twl, (void*)&scratch};
-  e = cudaLaunchKernel(kfn, dim3(beams * g.C), dim3(g.T), args, (size_t)g.Mpad * sizeof(float2), ctx->stream);
+  if (M == kBigM4) {  // four rows per CTA, bin order written directly
+    const void* kfn = out_mode == SPX_OUT_COMPLEX ? (const void*)big_rows4_kernel<kBigComplex>
+                      : out_mode == SPX_OUT_MAG || out_mode == SPX_OUT_MAG2
+                          ? (const void*)big_rows4_kernel<kBigMag>
+                      : out_mode == SPX_OUT_MAGPHASE ? (const void*)big_rows4_kernel<kBigMagPhase>
+                                                     : (const void*)big_rows4_kernel<kBigOther>;
+    const size_t smem = (size_t)kRows4 * kRowPitch4 * sizeof(float4);
+    e = configure_kernel(kfn, smem);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "configure big_rows4_kernel");
+    gg.ahead = ctx->input_on_host ? 0u : resident_ctas(kfn, kRows4 * 128, smem, 1);
+    const float2* scr_c = scratch;
+    void* args[] = {(void*)&gg, (void*)&twp, (void*)&scr_c, (void*)&d_out, (void*)&out_mode, (void*)&scale};
+    e = cudaLaunchKernel(kfn, dim3(beams * (g.C / kRows4)), dim3(kRows4 * 128), args, smem, ctx->stream);
+    return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch big_rows4_kernel");
+  }
+  const void* kfn = (const void*)big_rows_kernel;
+  const size_t smem = ps_len(kBigM) * sizeof(float4);
+  e = configure_kernel(kfn, smem);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "configure big_rows_kernel");
+  gg.ahead = resident_ctas(kfn, 512, smem, 1);
+  void* args[] = {(void*)&gg, (void*)&twp, (void*)&scratch};
+  e = cudaLaunchKernel(kfn, dim3(beams * g.C), dim3(512), args, smem, ctx->stream);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "launch big_rows_kernel");
   return launch_rows_transpose(ctx, g, scratch, beams, d_out, out_mode, scale);
 }

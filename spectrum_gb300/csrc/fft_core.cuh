@@ -457,8 +457,19 @@ struct CtPlan {
   static_assert(M == (1 << a) * ct_pow3(b) && M <= 16384, "M must be 2^a 3^b <= 16384");
 };
 
+// Barriers of a local FFT: the whole CTA's, or one group of N consecutive
+// threads' (N a multiple of 32; groups of one CTA use different hardware
+// barriers, 1 + their number).
+struct CtaSync {
+  static SPX_DEV void wait() { __syncthreads(); }
+};
+template <int N>
+struct GroupSync {
+  static SPX_DEV void wait() { asm volatile("bar.sync %0, %1;" ::"r"(1 + threadIdx.x / N), "n"(N) : "memory"); }
+};
+
 // First pass (Ns = 1) from `load`, results into shared memory.
-template <int M, int T = CtPlan<M>::T, typename Load>
+template <int M, int T = CtPlan<M>::T, typename Sync = CtaSync, typename Load>
 SPX_DEV void ct_first(float2* s, const Load& load, uint32_t tid) {
   using P = CtPlan<M>;
   constexpr int R = P::radix(0), B = M / R, Q = (B + T - 1) / T;
@@ -481,13 +492,13 @@ SPX_DEV void ct_first(float2* s, const Load& load, uint32_t tid) {
       }
     }
   }
-  __syncthreads();
+  Sync::wait();
 }
 
 // Pass P >= 1 in shared memory.  The last pass (Ns = M / R = B) writes each
 // butterfly's outputs to the elements it read (base = j), so it needs no
 // barrier between its loads and its stores.
-template <int M, int P, int T>
+template <int M, int P, int T, typename Sync = CtaSync>
 SPX_DEV void ct_pass(float2* s, const float2* __restrict__ tw, uint32_t tid) {
   using PL = CtPlan<M>;
   constexpr int R = PL::radix(P), Ns = PL::ns(P), B = M / R, Q = (B + T - 1) / T;
@@ -501,7 +512,7 @@ SPX_DEV void ct_pass(float2* s, const float2* __restrict__ tw, uint32_t tid) {
       for (int r = 0; r < R; ++r) v[q][r] = s[(B % 16 == 0) ? sj + sw(r * B) : sw(j + r * B)];
     }
   }
-  if constexpr (P + 1 < PL::npass) __syncthreads();
+  if constexpr (P + 1 < PL::npass) Sync::wait();
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const uint32_t j = tid + q * T;
@@ -522,14 +533,14 @@ SPX_DEV void ct_pass(float2* s, const float2* __restrict__ tw, uint32_t tid) {
       for (int r = 0; r < R; ++r) s[(Ns % 16 == 0) ? sb + sw(r * Ns) : sw(base + r * Ns)] = v[q][r];
     }
   }
-  __syncthreads();
+  Sync::wait();
 }
 
-template <int M, int P, int T>
+template <int M, int P, int T, typename Sync = CtaSync>
 SPX_DEV void ct_passes_from(float2* s, const float2* __restrict__ tw, uint32_t tid) {
   if constexpr (P < CtPlan<M>::npass) {
-    ct_pass<M, P, T>(s, tw, tid);
-    ct_passes_from<M, P + 1, T>(s, tw, tid);
+    ct_pass<M, P, T, Sync>(s, tw, tid);
+    ct_passes_from<M, P + 1, T, Sync>(s, tw, tid);
   }
 }
 
@@ -580,12 +591,12 @@ SPX_DEV void ct_passes_until_last(float2* s, const float2* __restrict__ tw, uint
   }
 }
 
-// Whole local FFT of M points (first pass from `load`) by a CTA of T
-// threads, ending with a barrier.
-template <int M, int T = CtPlan<M>::T, typename Load>
+// Whole local FFT of M points (first pass from `load`) by T threads (a CTA,
+// or a group of one with its own barrier), ending with a barrier.
+template <int M, int T = CtPlan<M>::T, typename Sync = CtaSync, typename Load>
 SPX_DEV void ct_local_fft(float2* s, const Load& load, const float2* __restrict__ tw, uint32_t tid) {
-  ct_first<M, T>(s, load, tid);
-  ct_passes_from<M, 1, T>(s, tw, tid);
+  ct_first<M, T, Sync>(s, load, tid);
+  ct_passes_from<M, 1, T, Sync>(s, tw, tid);
 }
 
 // The local FFT of ct_local_fft with the last pass's outputs handed to

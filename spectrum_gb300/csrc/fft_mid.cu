@@ -122,9 +122,6 @@ struct MidRowsArgs {
 constexpr int kMidComplex = 0, kMidMag = 1, kMidOther = 2;
 constexpr uint32_t kMidRows = 4;  // rows per CTA
 
-struct CtaSync {
-  static SPX_DEV void wait() { __syncthreads(); }
-};
 struct WarpSync {
   static SPX_DEV void wait() { __syncwarp(); }
 };

@@ -255,7 +255,7 @@ struct ExchangePairs {
 };
 
 // ---- passes ------------------------------------------------------------------------
-template <int M, int T, typename Load>
+template <int M, int T, typename Sync = CtaSync, typename Load>
 SPX_DEV void pair_first(float4* s, const Load& load, uint32_t tid) {
   constexpr int R = CtPlan<M>::radix(0), B = M / R, Q = B / 2 / T;
   static_assert(R % 2 == 0 && Q * 2 * T == B, "whole pairs");
@@ -275,7 +275,7 @@ SPX_DEV void pair_first(float4* s, const Load& load, uint32_t tid) {
       d[R / 2 + r / 2] = make_float4(v[r].x.y, v[r + 1].x.y, v[r].y.y, v[r + 1].y.y);
     }
   }
-  __syncthreads();
+  Sync::wait();
 }
 
 SPX_DEV C2 ld_tw(const float4* __restrict__ t) {
@@ -318,13 +318,13 @@ SPX_DEV void pair_butterfly(C2* v, const float4* __restrict__ tw, uint32_t m) {
 }
 
 // Pass P (not the first, not the last) in shared memory.
-template <int M, int P, int T>
+template <int M, int P, int T, typename Sync = CtaSync>
 SPX_DEV void pair_pass(float4* s, const float4* __restrict__ tw, uint32_t tid) {
   constexpr int R = CtPlan<M>::radix(P), Ns = CtPlan<M>::ns(P), Q = M / R / 2 / T, H = Ns / 2;
   static_assert(Q == 1, "one pair of butterflies per thread");
   C2 v[R];
   pair_load<M, P>(s, v, tid);
-  __syncthreads();
+  Sync::wait();
   pair_butterfly<M, P>(v, tw, tid);
   // slot of output r: ((j - k) R + k) / 2 + r H with j = 2m; H divides 16 or is a multiple of it
   const uint32_t kk = tid & (H - 1);
@@ -332,13 +332,13 @@ SPX_DEV void pair_pass(float4* s, const float4* __restrict__ tw, uint32_t tid) {
 #pragma unroll
   for (int r = 0; r < R; ++r)
     d[r * H + ((r * H) >> 4)] = make_float4(v[r].x.x, v[r].x.y, v[r].y.x, v[r].y.y);
-  __syncthreads();
+  Sync::wait();
 }
-template <int M, int P, int T>
+template <int M, int P, int T, typename Sync = CtaSync>
 SPX_DEV void pair_passes_until_last(float4* s, const float4* __restrict__ tw, uint32_t tid) {
   if constexpr (P + 1 < CtPlan<M>::npass) {
-    pair_pass<M, P, T>(s, tw, tid);
-    pair_passes_until_last<M, P + 1, T>(s, tw, tid);
+    pair_pass<M, P, T, Sync>(s, tw, tid);
+    pair_passes_until_last<M, P + 1, T, Sync>(s, tw, tid);
   }
 }
 
@@ -485,6 +485,13 @@ SPX_DEV void pair_cross_stage(float2* __restrict__ slot, uint32_t c, const Sampl
 #pragma unroll
     for (int k1 = 1; k1 < CR; ++k1) put(k1, c2mul(v[k1], w[k1]));
   }
+}
+
+// Four complex values, one 32-byte store (p on a 32-byte boundary).
+SPX_DEV void st256(float2* p, float2 a, float2 b, float2 c, float2 d) {
+  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(b.x),
+               "f"(b.y), "f"(c.x), "f"(c.y), "f"(d.x), "f"(d.y)
+               : "memory");
 }
 
 // Elements i, i + 1 into a 16-byte aligned row of device memory.

@@ -63,6 +63,24 @@ def test_inverse_and_unaligned_output_equal_the_scalar_kernels(spx, scalar, nfft
     assert _same(full, spx.fft_r2c(x.real.contiguous(), nfft, spx.WINDOW_HANN, True, ctx=scalar))
 
 
+@pytest.mark.parametrize("nfft", [1 << 19, 1 << 20, 1 << 21])
+def test_big_transform_modes_agree(spx, nfft):
+    """The output modes of the 2^19 .. 2^21-point transforms (different ways out
+    of the row kernel) hold the same spectrum bit for bit, and it is the
+    library FFT's within FP32 rounding; odd lengths take 8-byte loads."""
+    import torch
+    for n, offset in ((nfft, 0), (nfft // 2 + 1, 1)):
+        x = _samples(2, n, offset, nfft + n)
+        z = spx.fft(x, nfft, spx.WINDOW_HANN)
+        w = torch.sin(torch.pi * torch.arange(n, device="cuda", dtype=torch.float64) / (n - 1)) ** 2
+        ref = torch.fft.fft(x.to(torch.complex128) * w, n=nfft)
+        assert ((z - ref).abs().max() / ref.abs().max()).item() < 1e-6  # ~ log2(N) roundings of 6e-8
+        m2 = spx.magnitude(z, 1.0, squared=True)
+        assert _same(spx.fft(x, nfft, spx.WINDOW_HANN, "mag2"), m2)
+        assert _same(spx.fft(x, nfft, spx.WINDOW_HANN, "mag"), spx.magnitude(z))
+        assert _same(spx.fft(x, nfft, spx.WINDOW_HANN, "magphase"), spx.mag_phase(z))
+
+
 @pytest.mark.parametrize("nfft", [32768, 65536, 131072, 262144])
 def test_maxima_of_row_spectra_equal_the_composed_search(spx, nfft):
     """All maxima from the row layout of the two-launch transforms against the
