@@ -399,8 +399,8 @@ spx_status spx_batch_load_plans(spx_ctx* ctx, spx_batch* batch, const char* path
  *                       leaves the bin; d_amplitude [beams x K] (may be NULL)
  *                       receives |X[k]| exp(y1); d_used_mlp (may be NULL)
  *                       1 where the network was used.
- * Training-data generation and training allocate; forward/refine allocate
- * activations only when a larger row count is first seen. */
+ * Training-data generation allocates; gradients and training allocate their
+ * partial sums (at most 6 MB) when a larger row count is first seen. */
 typedef struct spx_mlp spx_mlp;
 uint32_t spx_mlp_param_count(void);
 spx_status spx_mlp_create(spx_ctx* ctx, uint64_t seed, spx_mlp** out);

@@ -40,124 +40,275 @@ SPX_DEV float gelu_grad(float z) {
          z * 0.39894228040143268f * expf(-0.5f * z * z);
 }
 
-// ---- training layers (one thread per output element) ---------------------------
-// Z[b][o] = sum_i X[b][i] W[o][i] + bias[o];  H = GELU(Z) when act, else Z.
-__global__ void mlp_fwd_kernel(const float* __restrict__ X, const __nv_bfloat16* __restrict__ W,
-                               const float* __restrict__ bias, uint32_t B, int in, int out,
-                               float* __restrict__ Z, float* __restrict__ H, int act) {
-  const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (uint64_t)B * out) return;
-  const uint32_t b = idx / out, o = idx % out;
-  const float* x = X + (size_t)b * in;
-  const __nv_bfloat16* w = W + (size_t)o * in;
-  float acc = bias[o];
-  for (int i = 0; i < in; ++i) acc = fmaf(x[i], __bfloat162float(w[i]), acc);
-  Z[idx] = acc;
-  if (H) H[idx] = act ? gelu(acc) : acc;
+// ---- training: forward, backward and the weight gradients of a tile in one CTA ----
+// A CTA takes tiles of kTile rows and keeps everything between the layers in
+// shared memory: activations as [unit][row] (pitch kTp: consecutive units or
+// four-row quads of consecutive lanes hit different banks), the weights as FP32.
+// Every product is a register tile fed by 128-bit shared loads.  The weight
+// gradients stay in registers over the CTA's tiles and leave as one partial sum
+// per CTA, added by mlp_reduce_kernel in CTA order: tiles are dealt to a number
+// of CTAs that depends on the rows alone, so the gradient is the same bits on
+// every run (no atomics).
+// Bound: 28 kFLOP a row are a few microseconds of the FP32 pipe; the tile's
+// chain of layers (seven barriers) and two launches are what is left.  One
+// thread per output and layer took twelve launches with chains of 512 rows in as
+// few as 16 CTAs: loss and gradients of 4096 rows 263 -> 29 us,
+// error against FP64 1.6e-7 -> 4.8e-8.
+constexpr int kTile = 32, kTp = kTile + 4;  // rows per tile; row pitch of [unit][row] arrays
+constexpr int kWp = kH + 4;                 // row pitch of W2
+constexpr int kW1p = 12;                    // row pitch of W1
+constexpr uint32_t kMaxTileCtas = 304;      // two per SM
+constexpr uint32_t kPart = kNParams + 2;    // floats of a partial sum: gradients, loss, padding
+
+struct TileSmem {
+  float w2[kH * kWp], w1[kH * kW1p], w3[kOut * kH], b1[kH], b2[kH], b3[kOut + 2];
+  float x[kIn * kTp], h1[kH * kTp], h2[kH * kTp];
+  float g1[kH * kTp], g2[kH * kTp];  // GELU' of layers 1, 2, then their dZ
+  float dy[kOut * kTp];
+};
+
+struct TileArgs {
+  const __nv_bfloat16* pb;
+  const float* p;
+  const float *x, *t;
+  const uint32_t* mask;  // may be null
+  uint32_t rows;
+  // row j of the pass is row (pa (first + j) + pc) mod n of x, t and mask (an
+  // affine permutation of [0, n), n a power of two), or row j when n = 0
+  uint32_t n, first, pa, pc;
+  float* y;     // forward: [rows][2]
+  float* part;  // gradients: [CTAs][kPart]
+};
+
+SPX_DEV float dot4(float4 a, float4 b, float acc) {
+  return fmaf(a.w, b.w, fmaf(a.z, b.z, fmaf(a.y, b.y, fmaf(a.x, b.x, acc))));
+}
+SPX_DEV void fma4(float (&acc)[4], float w, float4 v) {
+  acc[0] = fmaf(v.x, w, acc[0]);
+  acc[1] = fmaf(v.y, w, acc[1]);
+  acc[2] = fmaf(v.z, w, acc[2]);
+  acc[3] = fmaf(v.w, w, acc[3]);
 }
 
-// Mean squared error over the rows with mask != 0 (mask may be null):
-// dY = (Y - T) * 2 / (B * kOut) on those rows, 0 elsewhere; loss += MSE.
-__global__ void mlp_out_grad_kernel(const float* __restrict__ Y, const float* __restrict__ Tg,
-                                    const uint32_t* __restrict__ mask, uint32_t B,
-                                    float* __restrict__ dY, float* __restrict__ loss) {
-  const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
-  float l = 0.f;
-  if (idx < B * kOut) {
-    const bool on = !mask || mask[idx / kOut] != 0;
-    const float d = on ? Y[idx] - Tg[idx] : 0.f;
-    dY[idx] = d * (2.0f / (float)(B * kOut));
-    l = d * d / (float)(B * kOut);
+template <bool GRAD>
+__global__ void __launch_bounds__(256)
+mlp_tile_kernel(TileArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TileSmem& s = *reinterpret_cast<TileSmem*>(smem_raw);
+  const uint32_t tid = threadIdx.x;
+  for (uint32_t i = tid; i < kH * kH; i += 256) s.w2[(i / kH) * kWp + i % kH] = __bfloat162float(a.pb[kOffW2 + i]);
+  for (uint32_t i = tid; i < kH * kIn; i += 256) s.w1[(i / kIn) * kW1p + i % kIn] = __bfloat162float(a.pb[kOffW1 + i]);
+  if (tid < kOut * kH) s.w3[tid] = __bfloat162float(a.pb[kOffW3 + tid]);
+  if (tid < kH) {
+    s.b1[tid] = a.p[kOffB1 + tid];
+    s.b2[tid] = a.p[kOffB2 + tid];
   }
-  for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
-  if (loss && (threadIdx.x & 31) == 0) atomicAdd(loss, l);
-}
-
-// dX[b][i] = (sum_o dZ[b][o] W[o][i]) * GELU'(Zprev[b][i])
-__global__ void mlp_bwd_data_kernel(const float* __restrict__ dZ, const __nv_bfloat16* __restrict__ W,
-                                    const float* __restrict__ Zprev, uint32_t B, int in, int out,
-                                    float* __restrict__ dX) {
-  const uint64_t idx = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= (uint64_t)B * in) return;
-  const uint32_t b = idx / in, i = idx % in;
-  const float* dz = dZ + (size_t)b * out;
-  float acc = 0.f;
-  for (int o = 0; o < out; ++o) acc = fmaf(dz[o], __bfloat162float(W[(size_t)o * in + i]), acc);
-  dX[idx] = acc * gelu_grad(Zprev[idx]);
-}
-
-// Partial weight gradients of one chunk of kBwdChunk rows (blockIdx.y):
-// part[chunk][o*in + i] = sum_b dZ[b][o] X[b][i] and part[chunk][out*in + o]
-// = sum_b dZ[b][o] over the chunk's rows b, in row order.  mlp_sum_chunks
-// then adds the chunks in chunk order: the gradient is the same bits on every
-// run (no atomics), so training is reproducible.
-constexpr uint32_t kBwdChunk = 512;
-constexpr uint32_t kMaxLayerParams = kH * (kH + 1);  // largest out * (in + 1)
-__global__ void mlp_bwd_weight_kernel(const float* __restrict__ dZ, const float* __restrict__ X,
-                                      uint32_t B, int in, int out, float* __restrict__ part) {
-  const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t n = (uint32_t)(out * (in + 1));
-  if (idx >= n) return;
-  const uint32_t o = idx / (in + 1), i = idx % (in + 1);
-  const uint32_t b0 = blockIdx.y * kBwdChunk, b1 = min(B, b0 + kBwdChunk);
-  float acc = 0.f;
-  float* dst = part + (size_t)blockIdx.y * n;
-  if (i < (uint32_t)in) {
-    for (uint32_t b = b0; b < b1; ++b) acc = fmaf(dZ[(size_t)b * out + o], X[(size_t)b * in + i], acc);
-    dst[o * in + i] = acc;
-  } else {
-    for (uint32_t b = b0; b < b1; ++b) acc += dZ[(size_t)b * out + o];
-    dst[out * in + o] = acc;
+  if (tid < kOut) s.b3[tid] = a.p[kOffB3 + tid];
+  auto source = [&](uint32_t j) { return a.n ? (a.pa * (a.first + j) + a.pc) & (a.n - 1) : j; };
+  auto f4 = [](const float* p) { return *reinterpret_cast<const float4*>(p); };
+  const uint32_t r4 = 4 * (tid & 7), up = tid >> 3;  // four rows, two units of the layers
+  const uint32_t to = tid & 15, ti = tid >> 4;       // W2 gradient: units to + 16 j, inputs ti + 16 k
+  float gw2[4][4] = {}, gw1[3] = {}, gw3 = 0.f, loss = 0.f;
+  const uint32_t tiles = (a.rows + kTile - 1) / kTile;
+#pragma unroll 1
+  for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+    const uint32_t j0 = tile * kTile;
+    for (uint32_t i = tid; i < kTile * kIn; i += 256) {
+      const uint32_t r = i / kIn, c = i - r * kIn;
+      s.x[c * kTp + r] = j0 + r < a.rows ? a.x[(size_t)source(j0 + r) * kIn + c] : 0.f;
+    }
+    __syncthreads();
+    // layer 1, units up and up + 32
+#pragma unroll
+    for (uint32_t u = up; u < kH; u += 32) {
+      float z[4] = {s.b1[u], s.b1[u], s.b1[u], s.b1[u]};
+#pragma unroll
+      for (uint32_t i = 0; i < kIn; ++i) fma4(z, s.w1[u * kW1p + i], f4(s.x + i * kTp + r4));
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        s.h1[u * kTp + r4 + q] = gelu(z[q]);
+        if (GRAD) s.g1[u * kTp + r4 + q] = gelu_grad(z[q]);
+      }
+    }
+    __syncthreads();
+    // layer 2
+    {
+      float z[2][4];
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) z[e][q] = s.b2[up + 32 * e];
+#pragma unroll 4
+      for (uint32_t i = 0; i < kH; i += 4) {
+        const float4 w0 = f4(s.w2 + up * kWp + i), w1 = f4(s.w2 + (up + 32) * kWp + i);
+        const float4 h0 = f4(s.h1 + i * kTp + r4), h1 = f4(s.h1 + (i + 1) * kTp + r4),
+                     h2 = f4(s.h1 + (i + 2) * kTp + r4), h3 = f4(s.h1 + (i + 3) * kTp + r4);
+        fma4(z[0], w0.x, h0); fma4(z[0], w0.y, h1); fma4(z[0], w0.z, h2); fma4(z[0], w0.w, h3);
+        fma4(z[1], w1.x, h0); fma4(z[1], w1.y, h1); fma4(z[1], w1.z, h2); fma4(z[1], w1.w, h3);
+      }
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t at = (up + 32 * e) * kTp + r4 + q;
+          s.h2[at] = gelu(z[e][q]);
+          if (GRAD) s.g2[at] = gelu_grad(z[e][q]);
+        }
+    }
+    __syncthreads();
+    // layer 3: thread (row, output); masked mean squared error and its gradient
+    if (tid < kTile * kOut) {
+      const uint32_t r = tid & (kTile - 1), o = tid / kTile, j = j0 + r;
+      float y = s.b3[o];
+#pragma unroll 16
+      for (uint32_t i = 0; i < kH; ++i) y = fmaf(s.h2[i * kTp + r], s.w3[o * kH + i], y);
+      if constexpr (GRAD) {
+        float d = 0.f;
+        if (j < a.rows) {
+          const uint32_t src = source(j);
+          if (!a.mask || a.mask[src] != 0) d = y - a.t[(size_t)src * kOut + o];
+        }
+        const float n = (float)((uint64_t)a.rows * kOut);
+        s.dy[o * kTp + r] = d * (2.0f / n);
+        loss += d * d / n;
+      } else if (j < a.rows) {
+        a.y[(size_t)j * kOut + o] = y;
+      }
+    }
+    if constexpr (GRAD) {
+      __syncthreads();
+      // dZ2 = (dY W3) GELU'(Z2), over g2
+#pragma unroll
+      for (uint32_t u = up; u < kH; u += 32) {
+        float d[4] = {0.f, 0.f, 0.f, 0.f};
+        fma4(d, s.w3[u], f4(s.dy + r4));
+        fma4(d, s.w3[kH + u], f4(s.dy + kTp + r4));
+#pragma unroll
+        for (int q = 0; q < 4; ++q) s.g2[u * kTp + r4 + q] *= d[q];
+      }
+      __syncthreads();
+      // W3 and the biases of layers 2 and 3
+      if (tid < kOut * kH) {
+        const uint32_t o = tid / kH, i = tid % kH;
+#pragma unroll
+        for (int r = 0; r < kTile; r += 4) gw3 = dot4(f4(s.dy + o * kTp + r), f4(s.h2 + i * kTp + r), gw3);
+      } else if (tid < kOut * kH + kH + kOut) {
+        const uint32_t u = tid - kOut * kH;
+        const float* d = u < kH ? s.g2 + u * kTp : s.dy + (u - kH) * kTp;
+#pragma unroll
+        for (int r = 0; r < kTile; r += 4) gw3 = dot4(f4(d + r), make_float4(1.f, 1.f, 1.f, 1.f), gw3);
+      }
+      // dZ1 = (dZ2 W2) GELU'(Z1), inputs 2 up and 2 up + 1, over g1
+      {
+        float d[2][4] = {};
+#pragma unroll 8
+        for (uint32_t o = 0; o < kH; ++o) {
+          const float2 w = *reinterpret_cast<const float2*>(s.w2 + o * kWp + 2 * up);
+          const float4 z = f4(s.g2 + o * kTp + r4);
+          fma4(d[0], w.x, z);
+          fma4(d[1], w.y, z);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) s.g1[(2 * up + e) * kTp + r4 + q] *= d[e][q];
+      }
+      // W2
+#pragma unroll 2
+      for (int r = 0; r < kTile; r += 4) {
+        float4 z[4], h[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          z[k] = f4(s.g2 + (to + 16 * k) * kTp + r);
+          h[k] = f4(s.h1 + (ti + 16 * k) * kTp + r);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) gw2[j][k] = dot4(z[j], h[k], gw2[j][k]);
+      }
+      __syncthreads();
+      // W1 and its bias (input kIn)
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        const uint32_t i = (tid + 256 * e) / kH, o = tid % kH;
+        if (i > (uint32_t)kIn) break;
+#pragma unroll
+        for (int r = 0; r < kTile; r += 4)
+          gw1[e] = dot4(f4(s.g1 + o * kTp + r), i < (uint32_t)kIn ? f4(s.x + i * kTp + r) : make_float4(1.f, 1.f, 1.f, 1.f),
+                        gw1[e]);
+      }
+    }
+    __syncthreads();  // the tile's arrays are rewritten by the next one
+  }
+  if constexpr (GRAD) {
+    float* g = a.part + (size_t)blockIdx.x * kPart;
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) g[kOffW2 + (to + 16 * j) * kH + ti + 16 * k] = gw2[j][k];
+#pragma unroll
+    for (int e = 0; e < 3; ++e) {
+      const uint32_t i = (tid + 256 * e) / kH, o = tid % kH;
+      if (i < (uint32_t)kIn) g[kOffW1 + o * kIn + i] = gw1[e];
+      if (i == (uint32_t)kIn) g[kOffB1 + o] = gw1[e];
+    }
+    if (tid < kOut * kH) g[kOffW3 + tid] = gw3;
+    else if (tid < kOut * kH + kH) g[kOffB2 + tid - kOut * kH] = gw3;
+    else if (tid < kOut * kH + kH + kOut) g[kOffB3 + tid - kOut * kH - kH] = gw3;
+    if (tid < kTile * kOut) {  // two warps
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
+      if ((tid & 31) == 0) s.dy[tid >> 5] = loss;
+    }
+    __syncthreads();
+    if (tid == 0) g[kNParams] = s.dy[0] + s.dy[1];
   }
 }
 
-// g[idx] = sum over chunks c = 0, 1, ... of part[c][idx] (a layer's W then b,
-// contiguous in the parameter layout).
-__global__ void mlp_sum_chunks_kernel(const float* __restrict__ part, uint32_t chunks, uint32_t n,
-                                      float* __restrict__ g) {
-  const uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= n) return;
+// The partial sums of `parts` CTAs added in a fixed order: 32 parameters per
+// CTA, eight threads each.  The last "parameter" is the loss (added to *loss).
+// grad != null takes the gradient; else one Adam step of the FP32 masters
+// (bias-corrected) and the BF16 copy.
+struct AdamArgs {
+  float *p, *m, *v;
+  __nv_bfloat16* pb;
+  float lr, b1, b2, eps, c1, c2;
+};
+__global__ void __launch_bounds__(256)
+mlp_reduce_kernel(const float* __restrict__ part, uint32_t parts, float* __restrict__ grad, float* __restrict__ loss,
+                  AdamArgs ad) {
+  __shared__ float sum[8][32];
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
   float acc = 0.f;
-  for (uint32_t c = 0; c < chunks; ++c) acc += part[(size_t)c * n + idx];
-  g[idx] = acc;
-}
-
-// Adam on the FP32 masters (bias-corrected), then the BF16 copy.
-__global__ void mlp_adam_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
-                                const float* __restrict__ g, __nv_bfloat16* __restrict__ pb,
-                                uint32_t n, float lr, float b1, float b2, float eps, float c1,
-                                float c2) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-  p[i] = pi;
-  pb[i] = __float2bfloat16_rn(pi);
+  if (i <= (uint32_t)kNParams)
+    for (uint32_t c = w; c < parts; c += 8) acc += part[(size_t)c * kPart + i];
+  sum[w][lane] = acc;
+  __syncthreads();
+  if (w != 0 || i > (uint32_t)kNParams) return;
+  float g = sum[0][lane];
+#pragma unroll
+  for (int k = 1; k < 8; ++k) g += sum[k][lane];
+  if (i == (uint32_t)kNParams) {
+    if (loss) *loss += g;
+    return;
+  }
+  if (grad) {
+    grad[i] = g;
+    return;
+  }
+  const float mi = ad.b1 * ad.m[i] + (1.f - ad.b1) * g;
+  const float vi = ad.b2 * ad.v[i] + (1.f - ad.b2) * g * g;
+  ad.m[i] = mi;
+  ad.v[i] = vi;
+  const float pi = ad.p[i] - ad.lr * (mi / ad.c1) / (sqrtf(vi / ad.c2) + ad.eps);
+  ad.p[i] = pi;
+  ad.pb[i] = __float2bfloat16_rn(pi);
 }
 
 __global__ void to_bf16_kernel(const float* __restrict__ p, __nv_bfloat16* __restrict__ pb, uint32_t n) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) pb[i] = __float2bfloat16_rn(p[i]);
-}
-
-// Row gather for one minibatch: row j of the batch is training row
-// (a * (first + j) + c) mod n — an affine permutation of [0, n) (a odd, n a
-// power of two) that changes every epoch.
-__global__ void mlp_gather_kernel(const float* __restrict__ feat, const float* __restrict__ tgt,
-                                  const uint32_t* __restrict__ valid, uint32_t n, uint32_t first,
-                                  uint32_t B, uint32_t a, uint32_t c, float* __restrict__ bx,
-                                  float* __restrict__ bt, uint32_t* __restrict__ bm) {
-  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-  if (j >= B) return;
-  const uint32_t r = (a * (first + j) + c) & (n - 1);
-  for (int i = 0; i < kIn; ++i) bx[(size_t)j * kIn + i] = feat[(size_t)r * kIn + i];
-  bt[(size_t)j * 2] = tgt[(size_t)r * 2];
-  bt[(size_t)j * 2 + 1] = tgt[(size_t)r * 2 + 1];
-  bm[j] = valid ? valid[r] : 1u;
 }
 
 // ---- features -------------------------------------------------------------------
@@ -337,9 +488,8 @@ struct spx_mlp {
   float* d_p = nullptr;           // FP32 masters
   float* d_m = nullptr;           // Adam first moment
   float* d_v = nullptr;           // Adam second moment
-  float* d_g = nullptr;           // gradients
   __nv_bfloat16* d_pb = nullptr;  // BF16 copy read by every product
-  float* d_work = nullptr;        // activations and minibatch rows
+  float* d_work = nullptr;        // partial sums of the gradients
   size_t work_floats = 0;
   uint64_t step = 0;              // Adam step count
 };
@@ -356,19 +506,12 @@ namespace {
 
 unsigned nblocks(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
-// Per row: Z1 H1 Z2 H2 (4 x 64), Y (2), dZ2 dZ1 (2 x 64), dY (2), then the
-// minibatch slot: x (10), t (2), mask (1 word).
-constexpr size_t kWorkPerRow = 4 * kH + kOut + 2 * kH + kOut + kIn + 2 + 1;
+// CTAs of a pass over `rows` rows (a number that depends on the rows alone).
+uint32_t tile_ctas(uint32_t rows) { return std::min<uint32_t>((rows + kTile - 1) / kTile, kMaxTileCtas); }
 
-struct Acts {
-  float *Z1, *H1, *Z2, *H2, *Y, *dZ2, *dZ1, *dY, *bx, *bt;
-  uint32_t* bm;
-  float* part;  // per-chunk partial weight gradients, ceil(B / kBwdChunk) x kMaxLayerParams
-};
-
-spx_status ensure_work(spx_ctx* ctx, spx_mlp* m, uint32_t B, Acts* a) {
-  const size_t chunks = (B + kBwdChunk - 1) / kBwdChunk;
-  const size_t need = (size_t)B * kWorkPerRow + chunks * kMaxLayerParams;
+// Room for the partial sums of a pass.
+spx_status ensure_work(spx_ctx* ctx, spx_mlp* m, uint32_t rows) {
+  const size_t need = (size_t)tile_ctas(rows) * kPart;
   if (m->work_floats < need) {
     cudaError_t e = cudaSuccess;
     if (m->d_work) e = cudaStreamSynchronize(ctx->stream);
@@ -376,66 +519,39 @@ spx_status ensure_work(spx_ctx* ctx, spx_mlp* m, uint32_t B, Acts* a) {
     m->d_work = nullptr;
     m->work_floats = 0;
     if (e == cudaSuccess) e = cudaMalloc(&m->d_work, need * sizeof(float));
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(mlp activations)");
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(mlp partial sums)");
     m->work_floats = need;
   }
-  float* w = m->d_work;
-  a->Z1 = w;
-  a->H1 = a->Z1 + (size_t)B * kH;
-  a->Z2 = a->H1 + (size_t)B * kH;
-  a->H2 = a->Z2 + (size_t)B * kH;
-  a->Y = a->H2 + (size_t)B * kH;
-  a->dZ2 = a->Y + (size_t)B * kOut;
-  a->dZ1 = a->dZ2 + (size_t)B * kH;
-  a->dY = a->dZ1 + (size_t)B * kH;
-  a->bx = a->dY + (size_t)B * kOut;
-  a->bt = a->bx + (size_t)B * kIn;
-  a->bm = reinterpret_cast<uint32_t*>(a->bt + (size_t)B * 2);
-  a->part = w + (size_t)B * kWorkPerRow;
   return SPX_OK;
 }
 
-void forward(spx_ctx* ctx, spx_mlp* m, const float* X, uint32_t B, const Acts& a) {
-  const float* p = m->d_p;
-  const __nv_bfloat16* pb = m->d_pb;
-  cudaStream_t s = ctx->stream;
-  mlp_fwd_kernel<<<nblocks((uint64_t)B * kH, 256), 256, 0, s>>>(X, pb + kOffW1, p + kOffB1, B, kIn, kH, a.Z1, a.H1, 1);
-  mlp_fwd_kernel<<<nblocks((uint64_t)B * kH, 256), 256, 0, s>>>(a.H1, pb + kOffW2, p + kOffB2, B, kH, kH, a.Z2, a.H2, 1);
-  mlp_fwd_kernel<<<nblocks((uint64_t)B * kOut, 256), 256, 0, s>>>(a.H2, pb + kOffW3, p + kOffB3, B, kH, kOut, a.Y, nullptr, 0);
+template <bool GRAD>
+spx_status launch_tiles(spx_ctx* ctx, const spx_mlp* m, TileArgs a) {
+  a.pb = m->d_pb;
+  a.p = m->d_p;
+  a.part = m->d_work;
+  const void* kfn = (const void*)mlp_tile_kernel<GRAD>;
+  cudaError_t e = configure_kernel(kfn, sizeof(TileSmem));
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "configure mlp_tile_kernel");
+  mlp_tile_kernel<GRAD><<<tile_ctas(a.rows), 256, sizeof(TileSmem), ctx->stream>>>(a);
+  e = cudaGetLastError();
+  return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch mlp_tile_kernel");
 }
 
-// Weight and bias gradients of one layer (in -> out) into g (W then b),
-// through per-chunk partial sums added in a fixed order.
-void layer_weight_grad(cudaStream_t s, const float* dZ, const float* X, uint32_t B, int in, int out,
-                       const Acts& a, float* g) {
-  const unsigned ch = (B + kBwdChunk - 1) / kBwdChunk;
-  const uint32_t n = (uint32_t)(out * (in + 1));
-  mlp_bwd_weight_kernel<<<dim3(nblocks(n, 128), ch), 128, 0, s>>>(dZ, X, B, in, out, a.part);
-  mlp_sum_chunks_kernel<<<nblocks(n, 128), 128, 0, s>>>(a.part, ch, n, g);
-}
-
-// Gradient of the masked MSE into m->d_g (every entry written, the same bits
-// on every run); loss accumulated into d_loss.
-void backward(spx_ctx* ctx, spx_mlp* m, const float* X, const float* Tg, const uint32_t* mask,
-              uint32_t B, const Acts& a, float* d_loss) {
-  cudaStream_t s = ctx->stream;
-  const __nv_bfloat16* pb = m->d_pb;
-  float* g = m->d_g;
-  mlp_out_grad_kernel<<<nblocks((uint64_t)B * kOut, 256), 256, 0, s>>>(a.Y, Tg, mask, B, a.dY, d_loss);
-  layer_weight_grad(s, a.dY, a.H2, B, kH, kOut, a, g + kOffW3);
-  mlp_bwd_data_kernel<<<nblocks((uint64_t)B * kH, 256), 256, 0, s>>>(a.dY, pb + kOffW3, a.Z2, B, kH, kOut, a.dZ2);
-  layer_weight_grad(s, a.dZ2, a.H1, B, kH, kH, a, g + kOffW2);
-  mlp_bwd_data_kernel<<<nblocks((uint64_t)B * kH, 256), 256, 0, s>>>(a.dZ2, pb + kOffW2, a.Z1, B, kH, kH, a.dZ1);
-  layer_weight_grad(s, a.dZ1, X, B, kIn, kH, a, g + kOffW1);
-}
-
-void adam(spx_ctx* ctx, spx_mlp* m, float lr) {
-  m->step += 1;
-  const float b1 = 0.9f, b2 = 0.999f;
-  const float c1 = 1.f - (float)std::pow(0.9, (double)m->step);
-  const float c2 = 1.f - (float)std::pow(0.999, (double)m->step);
-  mlp_adam_kernel<<<nblocks(kNParams, 256), 256, 0, ctx->stream>>>(m->d_p, m->d_m, m->d_v, m->d_g, m->d_pb,
-                                                                   kNParams, lr, b1, b2, 1e-8f, c1, c2);
+// Loss and gradient of a pass; the gradient into d_grad, or (null) one Adam step.
+spx_status backward(spx_ctx* ctx, spx_mlp* m, const TileArgs& a, float* d_loss, float* d_grad, float lr) {
+  spx_status st = ensure_work(ctx, m, a.rows);
+  if (st == SPX_OK) st = launch_tiles<true>(ctx, m, a);
+  if (st != SPX_OK) return st;
+  AdamArgs ad{};
+  if (!d_grad) {
+    m->step += 1;
+    ad = AdamArgs{m->d_p, m->d_m, m->d_v, m->d_pb, lr, 0.9f, 0.999f, 1e-8f,
+                  1.f - (float)std::pow(0.9, (double)m->step), 1.f - (float)std::pow(0.999, (double)m->step)};
+  }
+  mlp_reduce_kernel<<<nblocks(kNParams + 1, 32), 256, 0, ctx->stream>>>(m->d_work, tile_ctas(a.rows), d_grad, d_loss, ad);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch mlp_reduce_kernel");
 }
 
 spx_status launch_status(spx_ctx* ctx, const char* what) {
@@ -457,7 +573,7 @@ spx_status spx_mlp_create(spx_ctx* ctx, uint64_t seed, spx_mlp** out) {
   if (!m) return fail(ctx, SPX_ERR_OUT_OF_MEMORY, "spx_mlp_create: host allocation failed");
   m->device = ctx->device;
   cudaError_t e = cudaSuccess;
-  float** bufs[] = {&m->d_p, &m->d_m, &m->d_v, &m->d_g};
+  float** bufs[] = {&m->d_p, &m->d_m, &m->d_v};
   for (float** b : bufs)
     if (e == cudaSuccess) e = cudaMalloc(b, kNParams * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&m->d_pb, kNParams * sizeof(__nv_bfloat16));
@@ -490,7 +606,6 @@ spx_status spx_mlp_destroy(spx_mlp* m) {
   cudaFree(m->d_p);
   cudaFree(m->d_m);
   cudaFree(m->d_v);
-  cudaFree(m->d_g);
   cudaFree(m->d_pb);
   cudaFree(m->d_work);
   delete m;
@@ -524,11 +639,21 @@ spx_status spx_mlp_forward(spx_ctx* ctx, spx_mlp* m, const float* d_x, uint32_t 
   if (rows == 0) return SPX_OK;
   if (!d_x || !d_y) return fail(ctx, SPX_ERR_INVALID_ARG, "spx_mlp_forward: null pointer");
   DeviceGuard guard(ctx->device);
-  Acts a;
-  spx_status st = ensure_work(ctx, m, rows, &a);
+  TileArgs a{};
+  a.x = d_x;
+  a.rows = rows;
+  a.y = d_y;
+  // an output over the input: through scratch (a CTA would write rows another still reads)
+  const size_t y_bytes = (size_t)rows * kOut * sizeof(float);
+  const uintptr_t x0 = reinterpret_cast<uintptr_t>(d_x), y0 = reinterpret_cast<uintptr_t>(d_y);
+  if (y0 >= x0 + (size_t)rows * kIn * sizeof(float) || x0 >= y0 + y_bytes) return launch_tiles<false>(ctx, m, a);
+  void* tmp = nullptr;
+  spx_status st = get_scratch(ctx, kSlotWork, y_bytes, &tmp);
   if (st != SPX_OK) return st;
-  forward(ctx, m, d_x, rows, a);
-  cudaMemcpyAsync(d_y, a.Y, (size_t)rows * kOut * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream);
+  a.y = static_cast<float*>(tmp);
+  st = launch_tiles<false>(ctx, m, a);
+  if (st != SPX_OK) return st;
+  cudaMemcpyAsync(d_y, tmp, y_bytes, cudaMemcpyDeviceToDevice, ctx->stream);
   return launch_status(ctx, "spx_mlp_forward");
 }
 
@@ -538,13 +663,12 @@ spx_status spx_mlp_gradients(spx_ctx* ctx, spx_mlp* m, const float* d_x, const f
   if (!d_x || !d_t || !d_grad || rows == 0)
     return fail(ctx, SPX_ERR_INVALID_ARG, "spx_mlp_gradients: null pointer or no rows");
   DeviceGuard guard(ctx->device);
-  Acts a;
-  spx_status st = ensure_work(ctx, m, rows, &a);
-  if (st != SPX_OK) return st;
-  forward(ctx, m, d_x, rows, a);
-  backward(ctx, m, d_x, d_t, d_mask, rows, a, d_loss);
-  cudaMemcpyAsync(d_grad, m->d_g, kNParams * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream);
-  return launch_status(ctx, "spx_mlp_gradients");
+  TileArgs a{};
+  a.x = d_x;
+  a.t = d_t;
+  a.mask = d_mask;
+  a.rows = rows;
+  return backward(ctx, m, a, d_loss, d_grad, 0.f);
 }
 
 spx_status spx_mlp_train_step(spx_ctx* ctx, spx_mlp* m, const float* d_x, const float* d_t,
@@ -554,13 +678,12 @@ spx_status spx_mlp_train_step(spx_ctx* ctx, spx_mlp* m, const float* d_x, const 
     return fail(ctx, SPX_ERR_INVALID_ARG, "spx_mlp_train_step: null pointer or no rows");
   if (!(lr > 0.f) || !std::isfinite(lr)) return fail(ctx, SPX_ERR_INVALID_ARG, "spx_mlp_train_step: lr must be > 0");
   DeviceGuard guard(ctx->device);
-  Acts a;
-  spx_status st = ensure_work(ctx, m, rows, &a);
-  if (st != SPX_OK) return st;
-  forward(ctx, m, d_x, rows, a);
-  backward(ctx, m, d_x, d_t, d_mask, rows, a, d_loss);
-  adam(ctx, m, lr);
-  return launch_status(ctx, "spx_mlp_train_step");
+  TileArgs a{};
+  a.x = d_x;
+  a.t = d_t;
+  a.mask = d_mask;
+  a.rows = rows;
+  return backward(ctx, m, a, d_loss, nullptr, lr);
 }
 
 spx_status spx_mlp_train(spx_ctx* ctx, spx_mlp* m, const float* d_feat, const float* d_target,
@@ -573,9 +696,7 @@ spx_status spx_mlp_train(spx_ctx* ctx, spx_mlp* m, const float* d_feat, const fl
   if (!(lr_max > 0.f) || !(lr_min > 0.f) || lr_min > lr_max || !std::isfinite(lr_max))
     return fail(ctx, SPX_ERR_INVALID_ARG, "spx_mlp_train: need 0 < lr_min <= lr_max");
   DeviceGuard guard(ctx->device);
-  Acts a;
-  spx_status st = ensure_work(ctx, m, batch, &a);
-  if (st != SPX_OK) return st;
+  spx_status st = SPX_OK;
   if (d_epoch_loss) cudaMemsetAsync(d_epoch_loss, 0, (size_t)epochs * sizeof(float), ctx->stream);
   const uint32_t steps_per_epoch = rows / batch;
   const double total = (double)steps_per_epoch * epochs;
@@ -591,14 +712,18 @@ spx_status spx_mlp_train(spx_ctx* ctx, spx_mlp* m, const float* d_feat, const fl
       // cosine decay from lr_max to lr_min over the whole run
       const double cosv = 0.5 * (1.0 + std::cos(3.14159265358979323846 * (double)step / total));
       const float lr = (float)(lr_min + (lr_max - lr_min) * cosv);
-      mlp_gather_kernel<<<nblocks(batch, 256), 256, 0, ctx->stream>>>(d_feat, d_target, d_valid, rows,
-                                                                      s * batch, batch, pa, pc, a.bx, a.bt, a.bm);
-      forward(ctx, m, a.bx, batch, a);
-      backward(ctx, m, a.bx, a.bt, a.bm, batch, a, d_epoch_loss ? d_epoch_loss + ep : nullptr);
-      adam(ctx, m, lr);
+      TileArgs t{};
+      t.x = d_feat;
+      t.t = d_target;
+      t.mask = d_valid;
+      t.rows = batch;
+      t.n = rows;
+      t.first = s * batch;
+      t.pa = pa;
+      t.pc = pc;
+      st = backward(ctx, m, t, d_epoch_loss ? d_epoch_loss + ep : nullptr, nullptr, lr);
+      if (st != SPX_OK) return st;
     }
-    st = launch_status(ctx, "spx_mlp_train");
-    if (st != SPX_OK) return st;
   }
   // per-epoch loss: mean over the epoch's steps
   if (d_epoch_loss) {
