@@ -10,17 +10,20 @@
 //   X[k] = w[k] * sum_n (x[n] w[n]) conj(w[k - n])
 //        = w[k] * IFFT_m( FFT_m(a) * FFT_m(b) )[k],
 //   a[n] = x[n] w[n] (n < N, 0 up to m), b[j] = conj(w[j]) at j and m - j.
-// Four launches per call: the pre-multiplied, zero-padded sequence, the
+// The steps: the pre-multiplied, zero-padded sequence, the
 // m-point transform (the library's own plan), the product with FFT_m(b) (made
 // once per plan on the device), the m-point inverse transform (the forward
 // plan with the reversing 1/m epilogue of spx_ifft), and the post-multiply
-// with the output epilogue of spx_fft (any output mode).  w is FP64-generated
+// with the output epilogue of spx_fft (any output mode): one launch up to m =
+// 16384, four up to 262144, one per step (a few more inside the transforms)
+// beyond.  w is FP64-generated
 // (n^2 reduced mod 2N exactly in integers) and stored FP32.  Error: a few
 // FP32 transforms of m points, ~1e-6 of the peak.
 #include <cmath>
 #include <vector>
 
 #include "fft_core.cuh"
+#include "fft_pair.cuh"
 #include "spx_internal.h"
 
 namespace spx {
@@ -65,6 +68,61 @@ __global__ void chirp_post_kernel(const float2* __restrict__ c, const float2* __
   }
 }
 
+// The whole chirp-z transform of a beam in one CTA, m = M points: the samples
+// times the chirp, FFT_M in shared memory, its last pass times FFT_M(b), FFT_M
+// again from shared memory, the last pass times the chirp into the output.  The
+// operations are those of the five launches above, so the bits are too; the
+// padded sequence never leaves the SM, where the launches moved it through
+// device memory five times.  tw and tw2 are the same table: with one pointer
+// the compiler carries the first transform's twiddles over to the second in
+// registers and spills 600 bytes a thread.
+template <int M>
+__global__ void __launch_bounds__(M / 32, M >= 16384 ? 1 : M == 8192 ? 2 : M == 4096 ? 4 : 8)
+chirp_pair_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __restrict__ win, FftGeom g,
+                  const float4* __restrict__ tw, const float4* tw2, const float2* __restrict__ w,
+                  const float2* __restrict__ bfft,
+                  void* __restrict__ out, uint32_t out_mode, float scale) {
+  extern __shared__ float4 s4[];
+  const uint32_t tid = threadIdx.x, beam = blockIdx.x;
+  if (g.ahead && beam + g.ahead < g.beams)
+    prefetch_l2(in + (size_t)(beam + g.ahead) * n_point, (size_t)n_point * sizeof(float2), tid, M / 32);
+  pair_local_fft_out<M>(s4, ChirpPairs{SamplePairs(in + (size_t)beam * n_point, n_point, win), w}, tw, tid,
+                        [=](uint32_t i, C2 z) {
+                          const float4 b = __ldg(reinterpret_cast<const float4*>(bfft + i));
+                          SlotOut{s4}(i, c2mul(z, C2{make_float2(b.x, b.z), make_float2(b.y, b.w)}));
+                        });
+  __syncthreads();
+  constexpr int T = M / 32;
+  pair_first_slots<M, T>(s4, tid);
+  pair_passes_until_last<M, 1, T>(s4, tw2, tid);
+  pair_last<M, T>(s4, tw2, tid, SlotOut{s4});
+  __syncthreads();
+  // bin k is element (M - k) mod M of the convolution
+  const float inv = 1.0f / (float)M;
+#pragma unroll 4
+  for (uint32_t k = tid; k < g.nfft; k += T) {
+    const float2 c = pair_elem(s4, (M - k) & (M - 1));
+    store_bin(out, out_mode, scale, g, beam, k,
+              cmul(make_float2(__fmul_rn(c.x, inv), __fmul_rn(c.y, inv)), __ldg(w + k)));
+  }
+}
+
+template <int M>
+static cudaError_t launch_chirp_pair(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams,
+                                     uint32_t n_point, const float* d_win, uint32_t out_mode, float scale, void* d_out) {
+  const void* kfn = (const void*)chirp_pair_kernel<M>;
+  const size_t smem = ps_len(M) * sizeof(float4);
+  cudaError_t e = configure_kernel(kfn, smem);
+  if (e != cudaSuccess) return e;
+  FftGeom g = plan.g;
+  g.beams = beams;
+  g.ahead = ctx->input_on_host ? 0u : resident_ctas(kfn, M / 32, smem, 1);
+  const float4* tw = plan.sub->d_tw_pair;
+  void* args[] = {(void*)&d_in,         (void*)&n_point, (void*)&d_win, (void*)&g, (void*)&tw, (void*)&tw,
+                  (void*)&plan.d_chirp, (void*)&plan.d_bfft, (void*)&d_out,   (void*)&out_mode, (void*)&scale};
+  return cudaLaunchKernel(kfn, dim3(beams), dim3(M / 32), args, smem, ctx->stream);
+}
+
 static unsigned grid_for(uint64_t total, int sms) {
   const uint64_t want = (total + 255) / 256;
   return (unsigned)std::min<uint64_t>(want, (uint64_t)sms * 8);
@@ -90,7 +148,7 @@ spx_status build_bluestein_plan(spx_ctx* ctx, uint32_t nfft, FftPlan* plan) {
     b[n] = cw;
     if (n > 0) b[m - n] = cw;
   }
-  cudaError_t e = cudaMalloc(&plan->d_chirp, (size_t)nfft * sizeof(float2));
+  cudaError_t e = cudaMalloc(&plan->d_chirp, ((size_t)nfft + 1) * sizeof(float2));  // read in pairs
   if (e == cudaSuccess) e = cudaMalloc(&plan->d_bfft, (size_t)m * sizeof(float2));
   if (e == cudaSuccess)
     e = cudaMemcpy(plan->d_chirp, w.data(), (size_t)nfft * sizeof(float2), cudaMemcpyHostToDevice);
@@ -108,6 +166,24 @@ spx_status launch_fft_bluestein(spx_ctx* ctx, const FftPlan& plan, const float2*
                                 void* d_out) {
   if (beams == 0) return SPX_OK;
   const uint32_t m = plan.bm, N = plan.g.nfft;
+  // m at its default plan, 1024 .. 16384 points: one launch; 32768 .. 262144:
+  // the two launches of each m-point transform with the chirp products inside;
+  // against the five launches (pre, transform, product, transform, post), 2^25
+  // bins: N = 500 1.16 -> 0.36 ms, 1000 1.14 -> 0.38, 5000 1.88 -> 0.84, 10007
+  // 2.64 -> 1.53, 100003 2.26 -> 1.30.  Beyond, and at tuned plans, the launches.
+  if (plan.sub->d_tw_pair && plan.sub->g.C == 1 && plan.sub->g.ept == 16) {
+    cudaError_t e;
+    switch (m) {
+      case 1024: e = launch_chirp_pair<1024>(ctx, plan, d_in, beams, n_point, d_win, out_mode, scale, d_out); break;
+      case 2048: e = launch_chirp_pair<2048>(ctx, plan, d_in, beams, n_point, d_win, out_mode, scale, d_out); break;
+      case 4096: e = launch_chirp_pair<4096>(ctx, plan, d_in, beams, n_point, d_win, out_mode, scale, d_out); break;
+      case 8192: e = launch_chirp_pair<8192>(ctx, plan, d_in, beams, n_point, d_win, out_mode, scale, d_out); break;
+      default: e = launch_chirp_pair<16384>(ctx, plan, d_in, beams, n_point, d_win, out_mode, scale, d_out); break;
+    }
+    return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch chirp_pair_kernel");
+  }
+  if (plan.sub->d_tw_rows)
+    return launch_fft_mid_chirp(ctx, plan, d_in, beams, n_point, d_win, out_mode, scale, d_out);
   void* buf = nullptr;
   spx_status st = get_scratch(ctx, kSlotChirp, (size_t)beams * m * sizeof(float2), &buf);
   if (st != SPX_OK) return st;

@@ -59,10 +59,12 @@ constexpr int kMidCols = C == 16 ? 32 : 256 / C;
 // the C-point DFT over n1 and its twiddles; stage 2: k1 = g, the 16-point DFT
 // over r.  All 16 loads of a thread (16 bytes each) are issued before its first
 // DFT.  Slots of the tile are [k1][r][p]: every access of a warp is contiguous.
-template <int C>
-__global__ void __launch_bounds__(kMidCols<C> / 2 * C, C == 16 ? 2 : C == 2 ? 4 : 5)
+// CHIRP: the samples of a chirp-z transform, times its chirp.
+template <int C, bool CHIRP>
+__global__ void __launch_bounds__(kMidCols<C> / 2 * C, C == 16 ? 2 : C == 2 || CHIRP ? 4 : 5)
 mid_cols_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __restrict__ win,
-                const float2* __restrict__ twc, float2* __restrict__ scratch, uint32_t ahead) {
+                const float2* __restrict__ twc, float2* __restrict__ scratch, uint32_t ahead,
+                const float2* __restrict__ chirp) {
   extern __shared__ float4 s4[];
   constexpr uint32_t W = kMidCols<C>, HP = W / 2, U = 16 / C, nfft = C * kMidLocal;
   const uint32_t tid = threadIdx.x, p = tid % HP, g = tid / HP;
@@ -78,7 +80,12 @@ mid_cols_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __
   const uint32_t j = c0 + 2 * p;
   C2 v[U][C];
 #pragma unroll
-  for (uint32_t u = 0; u < U; ++u) ld.load(v[u], kMidRow * (g + C * u) + j, kMidLocal);
+  for (uint32_t u = 0; u < U; ++u) {
+    if constexpr (CHIRP)
+      ChirpPairs{ld, chirp}.load(v[u], kMidRow * (g + C * u) + j, kMidLocal);
+    else
+      ld.load(v[u], kMidRow * (g + C * u) + j, kMidLocal);
+  }
 #pragma unroll
   for (uint32_t u = 0; u < U; ++u) {
     const uint32_t r = g + C * u;
@@ -118,8 +125,13 @@ struct MidRowsArgs {
   uint32_t out_mode;
   float scale;
   uint32_t qlo, qhi;      // window form: elements [qlo, qhi) of each row are written
+  const float2* chirp;    // chirp-z forms: FFT_m(b), or the chirp
+  FftGeom og;             // kMidChirpPost: geometry of the output (its nfft bins)
 };
 constexpr int kMidComplex = 0, kMidMag = 1, kMidOther = 2;
+// Chirp-z forms: times FFT_m(b); bin k is element (m - k) mod m of the
+// convolution, scaled by 1/m, times the chirp into the output
+constexpr int kMidChirpMul = 3, kMidChirpPost = 4;
 constexpr uint32_t kMidRows = 4;  // rows per CTA
 
 struct WarpSync {
@@ -237,6 +249,14 @@ mid_rows_kernel(MidRowsArgs a) {
       const size_t at = (size_t)beam * a.g.nfft + k;
       if constexpr (MODE == kMidComplex) {
         reinterpret_cast<float2*>(a.out)[at] = z;
+      } else if constexpr (MODE == kMidChirpMul) {
+        reinterpret_cast<float2*>(a.out)[at] = cmul(z, __ldg(a.chirp + k));
+      } else if constexpr (MODE == kMidChirpPost) {
+        const float inv = 1.0f / (float)a.g.nfft;
+        const uint32_t b = (a.g.nfft - k) & (a.g.nfft - 1);
+        if (b < a.og.nfft)
+          store_bin(a.out, a.out_mode, a.scale, a.og, beam, b,
+                    cmul(make_float2(__fmul_rn(z.x, inv), __fmul_rn(z.y, inv)), __ldg(a.chirp + b)));
       } else if constexpr (MODE == kMidMag) {
         const float m2 = mag2_rn(z);
         reinterpret_cast<float*>(a.out)[at] = __fmul_rn(a.out_mode == SPX_OUT_MAG2 ? m2 : __fsqrt_rn(m2), a.scale);
@@ -277,26 +297,29 @@ cudaError_t upload_mid_twiddles(FftPlan* plan, const float2* twl) {
 
 template <int C>
 static cudaError_t launch_cols(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams,
-                               uint32_t n_point, const float* d_win, float2* scratch) {
-  const void* kfn = (const void*)mid_cols_kernel<C>;
+                               uint32_t n_point, const float* d_win, float2* scratch, const float2* chirp) {
+  const void* kfn = chirp ? (const void*)mid_cols_kernel<C, true> : (const void*)mid_cols_kernel<C, false>;
   constexpr uint32_t threads = kMidCols<C> / 2 * C;
   const size_t smem = (size_t)16 * C * kMidCols<C> * sizeof(float2);
   cudaError_t e = configure_kernel(kfn, smem);
   if (e != cudaSuccess) return e;
   uint32_t ahead = ctx->input_on_host ? 0u : resident_ctas(kfn, threads, smem, 1);
-  void* args[] = {(void*)&d_in, (void*)&n_point, (void*)&d_win, (void*)&plan.d_tw_cross, (void*)&scratch, (void*)&ahead};
+  void* args[] = {(void*)&d_in, (void*)&n_point, (void*)&d_win, (void*)&plan.d_tw_cross, (void*)&scratch, (void*)&ahead,
+                  (void*)&chirp};
   return cudaLaunchKernel(kfn, dim3(beams * (kMidRow / kMidCols<C>)), dim3(threads), args, smem, ctx->stream);
 }
 
-// Launch 1 into the exchange scratch, then launch 2 (kernel kfn).
+// Launch 1 into the exchange scratch (with the samples times `chirp` when not
+// null), then launch 2 (kernel kfn).
 static spx_status launch_mid(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams, uint32_t n_point,
-                             const float* d_win, float2* scratch, const void* kfn, size_t smem, MidRowsArgs a) {
+                             const float* d_win, float2* scratch, const void* kfn, size_t smem, MidRowsArgs a,
+                             const float2* chirp = nullptr) {
   cudaError_t e;
   switch (plan.g.C) {
-    case 2: e = launch_cols<2>(ctx, plan, d_in, beams, n_point, d_win, scratch); break;
-    case 4: e = launch_cols<4>(ctx, plan, d_in, beams, n_point, d_win, scratch); break;
-    case 8: e = launch_cols<8>(ctx, plan, d_in, beams, n_point, d_win, scratch); break;
-    default: e = launch_cols<16>(ctx, plan, d_in, beams, n_point, d_win, scratch); break;
+    case 2: e = launch_cols<2>(ctx, plan, d_in, beams, n_point, d_win, scratch, chirp); break;
+    case 4: e = launch_cols<4>(ctx, plan, d_in, beams, n_point, d_win, scratch, chirp); break;
+    case 8: e = launch_cols<8>(ctx, plan, d_in, beams, n_point, d_win, scratch, chirp); break;
+    default: e = launch_cols<16>(ctx, plan, d_in, beams, n_point, d_win, scratch, chirp); break;
   }
   if (e != cudaSuccess) return cuda_fail(ctx, e, "launch mid_cols_kernel");
   e = configure_kernel(kfn, smem);
@@ -326,6 +349,34 @@ spx_status launch_fft_mid(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
                         : (const void*)mid_rows_kernel<kMidOther>;
   return launch_mid(ctx, plan, d_in, beams, n_point, d_win, static_cast<float2*>(scr), kfn,
                     kMidRows * kMidPitch * sizeof(float4), a);
+}
+
+spx_status launch_fft_mid_chirp(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams,
+                                uint32_t n_point, const float* d_win, uint32_t out_mode, float scale, void* d_out) {
+  const FftPlan& sub = *plan.sub;
+  const uint32_t m = plan.bm;
+  void *scr = nullptr, *conv = nullptr;
+  spx_status st = get_scratch(ctx, kSlotExchange, (size_t)beams * m * sizeof(float2), &scr);
+  if (st == SPX_OK) st = get_scratch(ctx, kSlotChirp, (size_t)beams * m * sizeof(float2), &conv);
+  if (st != SPX_OK) return st;
+  const size_t smem = kMidRows * kMidPitch * sizeof(float4);
+  MidRowsArgs a{};
+  a.out = conv;
+  a.chirp = plan.d_bfft;
+  st = launch_mid(ctx, sub, d_in, beams, n_point, d_win, static_cast<float2*>(scr),
+                  (const void*)mid_rows_kernel<kMidChirpMul>, smem, a, plan.d_chirp);
+  if (st != SPX_OK) return st;
+  a.out = d_out;
+  a.out_mode = out_mode;
+  a.scale = scale;
+  a.chirp = plan.d_chirp;
+  a.og = plan.g;
+  const bool on_host = ctx->input_on_host;
+  ctx->input_on_host = false;  // the convolution is in device memory
+  st = launch_mid(ctx, sub, static_cast<const float2*>(conv), beams, m, nullptr, static_cast<float2*>(scr),
+                  (const void*)mid_rows_kernel<kMidChirpPost>, smem, a);
+  ctx->input_on_host = on_host;
+  return st;
 }
 
 spx_status launch_fft_mid_rows(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams,

@@ -240,6 +240,27 @@ struct SamplePairs {
   }
 };
 
+// Samples of a chirp-z transform: SamplePairs times the chirp w[n], n < n_point
+// (chirp_pre_kernel's product), zero beyond.  w is readable up to an even count.
+struct ChirpPairs {
+  SamplePairs x;
+  const float2* __restrict__ w;
+  template <int R>
+  SPX_DEV void load(C2 (&v)[R], uint32_t n0, uint32_t step) const {
+    x.load(v, n0, step);
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+      const uint32_t n = n0 + r * step;
+      if (n < x.n_point) {
+        const float4 c = __ldg(reinterpret_cast<const float4*>(w + n));
+        const C2 z = c2mul(v[r], C2{make_float2(c.x, c.z), make_float2(c.y, c.w)});
+        const bool both = n + 1 < x.n_point;
+        v[r] = C2{make_float2(z.x.x, both ? z.x.y : 0.f), make_float2(z.y.x, both ? z.y.y : 0.f)};
+      }
+    }
+  }
+};
+
 // Elements n, n + 1 of a row written earlier by other CTAs (exchange slots):
 // L2-coherent 16-byte loads (rows start on 16-byte boundaries).
 struct ExchangePairs {
@@ -255,6 +276,20 @@ struct ExchangePairs {
 };
 
 // ---- passes ------------------------------------------------------------------------
+// Outputs of butterflies 2m, 2m + 1 of a first pass: slots m R + r/2 and
+// m R + R/2 + r/2 (r even); R = 16: ps(16 m + c) = 17 m + c (c < 16); R = 8:
+// 8 m + m/2 + c (c < 8).
+template <int R>
+SPX_DEV void pair_first_store(float4* s, uint32_t m, const C2* v) {
+  static_assert(R == 16 || R == 8, "first radix");
+  float4* d = s + (R == 16 ? 17 * m : 8 * m + (m >> 1));
+#pragma unroll
+  for (int r = 0; r < R; r += 2) {
+    d[r / 2] = make_float4(v[r].x.x, v[r + 1].x.x, v[r].y.x, v[r + 1].y.x);
+    d[R / 2 + r / 2] = make_float4(v[r].x.y, v[r + 1].x.y, v[r].y.y, v[r + 1].y.y);
+  }
+}
+
 template <int M, int T, typename Sync = CtaSync, typename Load>
 SPX_DEV void pair_first(float4* s, const Load& load, uint32_t tid) {
   constexpr int R = CtPlan<M>::radix(0), B = M / R, Q = B / 2 / T;
@@ -265,15 +300,7 @@ SPX_DEV void pair_first(float4* s, const Load& load, uint32_t tid) {
     C2 v[R];
     load.load(v, 2 * m, B);
     PDft<R>::run(v);
-    // butterflies 2m, 2m + 1: slots m R + r/2 and m R + R/2 + r/2 (r even);
-    // R = 16: ps(16 m + c) = 17 m + c (c < 16); R = 8: 8 m + m/2 + c (c < 8)
-    static_assert(R == 16 || R == 8, "first radix");
-    float4* d = s + (R == 16 ? 17 * m : 8 * m + (m >> 1));
-#pragma unroll
-    for (int r = 0; r < R; r += 2) {
-      d[r / 2] = make_float4(v[r].x.x, v[r + 1].x.x, v[r].y.x, v[r + 1].y.x);
-      d[R / 2 + r / 2] = make_float4(v[r].x.y, v[r + 1].x.y, v[r].y.y, v[r + 1].y.y);
-    }
+    pair_first_store<R>(s, m, v);
   }
   Sync::wait();
 }
@@ -315,6 +342,23 @@ SPX_DEV void pair_butterfly(C2* v, const float4* __restrict__ tw, uint32_t m) {
     for (int r = 1; r < R; ++r) v[r] = c2mul(v[r], ld_tw(t + (r - 1) * (Ns / 2) + kk));
   }
   PDft<R>::run(v);
+}
+
+// First pass from the slots themselves (the natural-order result of an earlier
+// transform, behind a barrier): every load before the first store.
+template <int M, int T>
+SPX_DEV void pair_first_slots(float4* s, uint32_t tid) {
+  constexpr int R = CtPlan<M>::radix(0), Q = M / R / 2 / T;
+  C2 v[Q][R];
+#pragma unroll
+  for (int q = 0; q < Q; ++q) pair_load<M, 0>(s, v[q], tid + q * T);
+  __syncthreads();
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    PDft<R>::run(v[q]);
+    pair_first_store<R>(s, tid + q * T, v[q]);
+  }
+  __syncthreads();
 }
 
 // Pass P (not the first, not the last) in shared memory.

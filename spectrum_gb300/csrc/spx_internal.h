@@ -132,6 +132,10 @@ spx_status launch_fft_mid(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
 spx_status launch_fft_mid_rows(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams,
                                uint32_t n_point, const float* d_win, uint32_t klo, uint32_t khi,
                                float2* d_rows);
+// A chirp-z transform (plan.bluestein) whose m-point transforms are of this kind.
+spx_status launch_fft_mid_chirp(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams,
+                                uint32_t n_point, const float* d_win, uint32_t out_mode, float scale,
+                                void* d_out);
 
 // Transforms of more than 2^21 points: N1 x N2, both 2^a 3^b <= 16384 (fft_huge.cu).
 bool huge_size(uint32_t nfft);

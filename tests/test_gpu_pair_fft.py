@@ -101,3 +101,31 @@ def test_maxima_of_row_spectra_equal_the_composed_search(spx, nfft):
             for b in range(3):
                 n = min(int(rc[b]), ref.shape[1])
                 assert torch.equal(out[b, :n], ref[b, :n]), (start, end, sigma, b)
+
+
+@pytest.mark.parametrize("nfft", [5, 500, 1000, 2000, 3001, 5000, 10007, 20011, 50021, 100003])
+def test_chirp_z_in_one_launch_equals_the_launches(spx, nfft):
+    """Lengths with other prime factors: the one-launch chirp-z transform (m up
+    to 16384) and the one with its products inside the m-point transforms (m up
+    to 262144) against the five launches over the scalar kernels, which a
+    context tuned for the m-point transform still runs."""
+    import torch
+    from spectrum_gb300._capi import lib
+    general = spx.Context(0)
+    m = spx.next_pow2(2 * nfft - 1)
+    if m >= 1024:
+        general.check(lib.spx_set_fft_tuning(general.h, m, 32, 0))
+    for n, offset, window in ((nfft, 0, spx.WINDOW_NONE), (nfft - 1, 1, spx.WINDOW_HANN),
+                              (nfft // 2 + 1, 0, spx.WINDOW_BLACKMAN), (1, 0, spx.WINDOW_NONE)):
+        x = _samples(3, n, offset, nfft + n)
+        for out in MODES:
+            assert _same(spx.fft(x, nfft, window, out, 0.5), spx.fft(x, nfft, window, out, 0.5, ctx=general)), (n, out)
+    x = _samples(3, nfft, 1, nfft)
+    ref = spx.ifft(x, ctx=general)
+    y = x.clone()
+    spx.ifft(y, out=y)
+    assert _same(y, ref)
+    r = x.real.contiguous()
+    for full in (False, True):
+        assert _same(spx.fft_r2c(r, nfft, spx.WINDOW_HANN, full),
+                     spx.fft_r2c(r, nfft, spx.WINDOW_HANN, full, ctx=general))
