@@ -552,10 +552,11 @@ spx_status launch_fft_out(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
     if (e != cudaSuccess) return cuda_fail(ctx, e, "launch fft_out_kernel");
     return SPX_OK;
   }
-  // power-of-two sizes at the default local size: two launches of small CTAs
-  // against the beam groups and the transpose, 2^25 points in all:
-  // 32768 0.323 -> 0.247 ms, 65536 0.324 -> 0.230, 131072 0.326 -> 0.233,
-  // 262144 0.354 -> 0.250
+  // C x 16384 points at the default plan: two launches of small CTAs against
+  // the beam groups (C a power of two) or clusters and the transpose, 2^25
+  // points in all: 32768 0.323 -> 0.247 ms, 65536 0.324 -> 0.230, 131072 0.326 ->
+  // 0.233, 262144 0.354 -> 0.250; 49152 0.402 -> 0.229, 98304 0.407 -> 0.224, 147456
+  // 0.423 -> 0.212, 196608 0.579 -> 0.231
   if (plan.d_tw_rows) return launch_fft_mid(ctx, plan, d_in, beams, n_point, d_win, out_mode, scale, d_out);
   const size_t xch_bytes = ((size_t)beams * g.nfft * sizeof(float2) + 255) & ~(size_t)255;
   void* xch = nullptr;

@@ -1,5 +1,5 @@
-// fft_mid.cu — power-of-two transforms of 32768 .. 262144 points in two
-// launches of small CTAs.
+// fft_mid.cu — transforms of C x 16384 points (32768, 49152, 65536 .. 262144)
+// in two launches of small CTAs.
 //
 // The plan is that of the beam groups (fft_core.cuh): nfft = C x 16384 with a
 // C-point cross stage, then a 16384-point local FFT of radices 16, 16, 16, 4;
@@ -50,28 +50,32 @@ constexpr uint32_t kMidRow = 1024;     // row length of launch 2
 constexpr uint32_t kMidTw = 208;
 
 // ---- launch 1 ----------------------------------------------------------------------
-// Columns per CTA: 4096 points (8192 for C = 16, whose 256 rows of 32 columns
+// Thread groups per column pair: C, rounded up to a power of two.
+template <int C>
+constexpr int kMidGroups = C <= 2 ? 2 : C <= 4 ? 4 : C <= 8 ? 8 : 16;
+// Columns per CTA: 128 threads (256 for 16 groups, whose rows of 32 columns
 // keep 256-byte runs).
 template <int C>
-constexpr int kMidCols = C == 16 ? 32 : 256 / C;
+constexpr int kMidCols = kMidGroups<C> == 16 ? 32 : 256 / kMidGroups<C>;
 
-// Thread (p, g): column pair p, g < C.  Stage 1: rows r = g + C u (u < 16 / C),
-// the C-point DFT over n1 and its twiddles; stage 2: k1 = g, the 16-point DFT
-// over r.  All 16 loads of a thread (16 bytes each) are issued before its first
-// DFT.  Slots of the tile are [k1][r][p]: every access of a warp is contiguous.
+// Thread (p, g): column pair p, group g < G.  Stage 1: rows r = g + G u
+// (u < 16 / G), the C-point DFT over n1 and its twiddles; stage 2: k1 = g < C,
+// the 16-point DFT over r.  All loads of a thread (16 bytes each) are issued
+// before its first DFT.  Slots of the tile are [k1][r][p]: every access of a
+// warp is contiguous.
 // CHIRP: the samples of a chirp-z transform, times its chirp.
 template <int C, bool CHIRP>
-__global__ void __launch_bounds__(kMidCols<C> / 2 * C, C == 16 ? 2 : C == 2 || CHIRP ? 4 : 5)
+__global__ void __launch_bounds__(kMidCols<C> / 2 * kMidGroups<C>, kMidGroups<C> == 16 ? 2 : C == 2 || CHIRP ? 4 : 5)
 mid_cols_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __restrict__ win,
                 const float2* __restrict__ twc, float2* __restrict__ scratch, uint32_t ahead,
                 const float2* __restrict__ chirp) {
   extern __shared__ float4 s4[];
-  constexpr uint32_t W = kMidCols<C>, HP = W / 2, U = 16 / C, nfft = C * kMidLocal;
+  constexpr uint32_t W = kMidCols<C>, HP = W / 2, G = kMidGroups<C>, U = 16 / G, nfft = C * kMidLocal;
   const uint32_t tid = threadIdx.x, p = tid % HP, g = tid / HP;
   const uint32_t beam = blockIdx.x / (kMidRow / W), c0 = (blockIdx.x - beam * (kMidRow / W)) * W;
   if (ahead && blockIdx.x + ahead < gridDim.x) {  // L2 prefetch of the tile one residency wave later
     const uint32_t f = blockIdx.x + ahead, fb = f / (kMidRow / W), fc = (f - fb * (kMidRow / W)) * W;
-    for (uint32_t r = tid; r < 16 * C; r += HP * C) {
+    for (uint32_t r = tid; r < 16 * C; r += HP * G) {
       const uint32_t lo = r * kMidRow + fc, hi = min(lo + W, n_point);
       if (lo < hi) prefetch_l2(in + (size_t)fb * n_point + lo, (size_t)(hi - lo) * sizeof(float2), 0, 1);
     }
@@ -82,13 +86,13 @@ mid_cols_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __
 #pragma unroll
   for (uint32_t u = 0; u < U; ++u) {
     if constexpr (CHIRP)
-      ChirpPairs{ld, chirp}.load(v[u], kMidRow * (g + C * u) + j, kMidLocal);
+      ChirpPairs{ld, chirp}.load(v[u], kMidRow * (g + G * u) + j, kMidLocal);
     else
-      ld.load(v[u], kMidRow * (g + C * u) + j, kMidLocal);
+      ld.load(v[u], kMidRow * (g + G * u) + j, kMidLocal);
   }
 #pragma unroll
   for (uint32_t u = 0; u < U; ++u) {
-    const uint32_t r = g + C * u;
+    const uint32_t r = g + G * u;
     const float4 t = __ldg(reinterpret_cast<const float4*>(twc + kMidRow * r + j));
     PDft<C>::run(v[u]);
     C2 w[C];
@@ -102,6 +106,7 @@ mid_cols_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __
     }
   }
   __syncthreads();
+  if (C < (int)G && g >= (uint32_t)C) return;
   C2 b[16];
 #pragma unroll
   for (int r = 0; r < 16; ++r) {
@@ -131,7 +136,7 @@ struct MidRowsArgs {
 constexpr int kMidComplex = 0, kMidMag = 1, kMidOther = 2;
 // Chirp-z forms: times FFT_m(b); bin k is element (m - k) mod m of the
 // convolution, scaled by 1/m, times the chirp into the output
-constexpr int kMidChirpMul = 3, kMidChirpPost = 4;
+constexpr int kMidChirpMul = 3, kMidChirpPost = 4, kMidMagPhase = 5;
 constexpr uint32_t kMidRows = 4;  // rows per CTA
 
 struct WarpSync {
@@ -249,6 +254,8 @@ mid_rows_kernel(MidRowsArgs a) {
       const size_t at = (size_t)beam * a.g.nfft + k;
       if constexpr (MODE == kMidComplex) {
         reinterpret_cast<float2*>(a.out)[at] = z;
+      } else if constexpr (MODE == kMidMagPhase) {
+        reinterpret_cast<float2*>(a.out)[at] = make_float2(mag_rn(z), atan2f(z.y, z.x));
       } else if constexpr (MODE == kMidChirpMul) {
         reinterpret_cast<float2*>(a.out)[at] = cmul(z, __ldg(a.chirp + k));
       } else if constexpr (MODE == kMidChirpPost) {
@@ -269,7 +276,7 @@ mid_rows_kernel(MidRowsArgs a) {
 
 // ---- host --------------------------------------------------------------------------
 bool mid_geometry(const FftGeom& g) {
-  return g.M == kMidLocal && g.ept == 16 && (g.C == 2 || g.C == 4 || g.C == 8 || g.C == 16);
+  return g.M == kMidLocal && g.ept == 16 && g.C > 1;
 }
 
 cudaError_t upload_mid_twiddles(FftPlan* plan, const float2* twl) {
@@ -298,8 +305,10 @@ cudaError_t upload_mid_twiddles(FftPlan* plan, const float2* twl) {
 template <int C>
 static cudaError_t launch_cols(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams,
                                uint32_t n_point, const float* d_win, float2* scratch, const float2* chirp) {
-  const void* kfn = chirp ? (const void*)mid_cols_kernel<C, true> : (const void*)mid_cols_kernel<C, false>;
-  constexpr uint32_t threads = kMidCols<C> / 2 * C;
+  const void* kfn = (const void*)mid_cols_kernel<C, false>;
+  if constexpr ((C & (C - 1)) == 0)  // chirp-z transforms take powers of two
+    if (chirp) kfn = (const void*)mid_cols_kernel<C, true>;
+  constexpr uint32_t threads = kMidCols<C> / 2 * kMidGroups<C>;
   const size_t smem = (size_t)16 * C * kMidCols<C> * sizeof(float2);
   cudaError_t e = configure_kernel(kfn, smem);
   if (e != cudaSuccess) return e;
@@ -317,6 +326,10 @@ static spx_status launch_mid(spx_ctx* ctx, const FftPlan& plan, const float2* d_
   cudaError_t e;
   switch (plan.g.C) {
     case 2: e = launch_cols<2>(ctx, plan, d_in, beams, n_point, d_win, scratch, chirp); break;
+    case 3: e = launch_cols<3>(ctx, plan, d_in, beams, n_point, d_win, scratch, chirp); break;
+    case 6: e = launch_cols<6>(ctx, plan, d_in, beams, n_point, d_win, scratch, chirp); break;
+    case 9: e = launch_cols<9>(ctx, plan, d_in, beams, n_point, d_win, scratch, chirp); break;
+    case 12: e = launch_cols<12>(ctx, plan, d_in, beams, n_point, d_win, scratch, chirp); break;
     case 4: e = launch_cols<4>(ctx, plan, d_in, beams, n_point, d_win, scratch, chirp); break;
     case 8: e = launch_cols<8>(ctx, plan, d_in, beams, n_point, d_win, scratch, chirp); break;
     default: e = launch_cols<16>(ctx, plan, d_in, beams, n_point, d_win, scratch, chirp); break;
@@ -346,7 +359,8 @@ spx_status launch_fft_mid(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
   const void* kfn = out_mode == SPX_OUT_COMPLEX ? (const void*)mid_rows_kernel<kMidComplex>
                     : out_mode == SPX_OUT_MAG || out_mode == SPX_OUT_MAG2
                         ? (const void*)mid_rows_kernel<kMidMag>
-                        : (const void*)mid_rows_kernel<kMidOther>;
+                    : out_mode == SPX_OUT_MAGPHASE ? (const void*)mid_rows_kernel<kMidMagPhase>
+                                                   : (const void*)mid_rows_kernel<kMidOther>;
   return launch_mid(ctx, plan, d_in, beams, n_point, d_win, static_cast<float2*>(scr), kfn,
                     kMidRows * kMidPitch * sizeof(float4), a);
 }

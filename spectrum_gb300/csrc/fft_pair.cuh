@@ -82,6 +82,85 @@ template <>
 struct PDft<4> {
   static SPX_DEV void run(C2* v) { pdft4(v[0], v[1], v[2], v[3]); }
 };
+SPX_DEV void pdft3(C2& a0, C2& a1, C2& a2) {
+  const C2 t = c2add(a1, a2), u = c2sub(a1, a2);
+  const C2 m{pfma(pk(-0.5f), t.x, a0.x), pfma(pk(-0.5f), t.y, a0.y)};
+  const float2 k = pk(kS3), nk = pk(-kS3);
+  a0 = c2add(a0, t);
+  a1 = C2{pfma(u.y, k, m.x), pfma(u.x, nk, m.y)};  // m - i k u
+  a2 = C2{pfma(u.y, nk, m.x), pfma(u.x, k, m.y)};  // m + i k u
+}
+template <>
+struct PDft<3> {
+  static SPX_DEV void run(C2* v) { pdft3(v[0], v[1], v[2]); }
+};
+template <>
+struct PDft<6> {
+  static SPX_DEV void run(C2* v) {
+    C2 e0 = v[0], e1 = v[2], e2 = v[4], o0 = v[1], o1 = v[3], o2 = v[5];
+    pdft3(e0, e1, e2);
+    pdft3(o0, o1, o2);
+    o1 = c2mulc(o1, 0.5f, -kS3);
+    o2 = c2mulc(o2, -0.5f, -kS3);
+    v[0] = c2add(e0, o0);
+    v[3] = c2sub(e0, o0);
+    v[1] = c2add(e1, o1);
+    v[4] = c2sub(e1, o1);
+    v[2] = c2add(e2, o2);
+    v[5] = c2sub(e2, o2);
+  }
+};
+template <>
+struct PDft<9> {
+  static SPX_DEV void run(C2* v) {
+    // columns n2: v[n2], v[n2 + 3], v[n2 + 6] -> b[n2][k1] in place
+#pragma unroll
+    for (int n2 = 0; n2 < 3; ++n2) pdft3(v[n2], v[3 + n2], v[6 + n2]);
+    auto b = [&](int n2, int k1) -> C2& { return v[3 * k1 + n2]; };
+    b(1, 1) = c2mulc(b(1, 1), kC9a, -kS9a);
+    b(1, 2) = c2mulc(b(1, 2), kC9b, -kS9b);
+    b(2, 1) = c2mulc(b(2, 1), kC9b, -kS9b);
+    b(2, 2) = c2mulc(b(2, 2), -kC9c, -kS9c);
+    C2 o[9];
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) {
+      C2 a0 = b(0, k1), a1 = b(1, k1), a2 = b(2, k1);
+      pdft3(a0, a1, a2);
+      o[k1] = a0;
+      o[k1 + 3] = a1;
+      o[k1 + 6] = a2;
+    }
+#pragma unroll
+    for (int i = 0; i < 9; ++i) v[i] = o[i];
+  }
+};
+template <>
+struct PDft<12> {
+  static SPX_DEV void run(C2* v) {
+    // columns n2: v[n2], v[n2 + 4], v[n2 + 8] -> b[n2][k1] in place
+#pragma unroll
+    for (int n2 = 0; n2 < 4; ++n2) pdft3(v[n2], v[4 + n2], v[8 + n2]);
+    auto b = [&](int n2, int k1) -> C2& { return v[4 * k1 + n2]; };
+    b(1, 1) = c2mulc(b(1, 1), kS3, -0.5f);
+    b(1, 2) = c2mulc(b(1, 2), 0.5f, -kS3);
+    b(2, 1) = c2mulc(b(2, 1), 0.5f, -kS3);
+    b(2, 2) = c2mulc(b(2, 2), -0.5f, -kS3);
+    b(3, 1) = C2{b(3, 1).y, pneg(b(3, 1).x)};
+    b(3, 2) = C2{pneg(b(3, 2).x), pneg(b(3, 2).y)};
+    C2 o[12];
+#pragma unroll
+    for (int k1 = 0; k1 < 3; ++k1) {
+      C2 a0 = b(0, k1), a1 = b(1, k1), a2 = b(2, k1), a3 = b(3, k1);
+      pdft4(a0, a1, a2, a3);
+      o[k1] = a0;
+      o[k1 + 3] = a1;
+      o[k1 + 6] = a2;
+      o[k1 + 9] = a3;
+    }
+#pragma unroll
+    for (int i = 0; i < 12; ++i) v[i] = o[i];
+  }
+};
 template <>
 struct PDft<8> {
   static SPX_DEV void run(C2* v) {

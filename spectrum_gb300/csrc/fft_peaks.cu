@@ -1003,6 +1003,19 @@ spx_status launch_fft_peaks(spx_ctx* ctx, const FftPlan& plan, const float2* d_i
   // power-of-two sizes at the default local size.  256 beams of 65536 points in
   // 131072 bins, 6 sigma: 0.275 ms with the beam groups (FFT 0.192, search of
   // their rows 0.080) -> 0.205 (columns 0.068, rows 0.066, search 0.066)
+  // C = 3, 6, 9, 12: the spectrum in bin order (rows of 48 .. 192 columns are not
+  // what the column-by-column search takes).  All maxima of 2^25 points against
+  // the cluster transform: 49152 0.305 -> 0.262 ms, 98304 0.314 -> 0.250, 147456
+  // 0.351 -> 0.267, 196608 0.481 -> 0.274
+  if (plan.d_tw_rows && !mx_rows(16 * g.C)) {
+    void *spec = nullptr, *cnt = nullptr;
+    spx_status st = get_scratch(ctx, kSlotSpectrum, (size_t)beams * g.nfft * sizeof(float2), &spec);
+    if (st == SPX_OK) st = get_scratch(ctx, kSlotWork, (size_t)beams * kMxMaxC2 * sizeof(uint32_t), &cnt);
+    if (st == SPX_OK) st = launch_fft_mid(ctx, plan, d_in, beams, n_point, d_win, SPX_OUT_COMPLEX, 1.0f, spec);
+    if (st != SPX_OK) return st;
+    return launch_maxima_cluster(ctx, static_cast<float2*>(spec), 1, g.nfft, beams, g.nfft, start, end, cap_or_k, fs,
+                                 refine, factor, static_cast<uint32_t*>(cnt), d_out, d_counts);
+  }
   if (plan.d_tw_rows) {  // spectrum rows over the exchange scratch, then the maxima kernel
     const size_t row_bytes = (size_t)beams * g.nfft * sizeof(float2);
     void* p = nullptr;

@@ -10,7 +10,7 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-SIZES = [1024, 2048, 4096, 8192, 16384, 32768, 131072, 262144]
+SIZES = [1024, 2048, 4096, 8192, 16384, 32768, 49152, 98304, 131072, 147456, 196608, 262144]
 MODES = ("complex", "mag", "mag2", "magphase")
 
 
@@ -81,7 +81,7 @@ def test_big_transform_modes_agree(spx, nfft):
         assert _same(spx.fft(x, nfft, spx.WINDOW_HANN, "magphase"), spx.mag_phase(z))
 
 
-@pytest.mark.parametrize("nfft", [32768, 65536, 131072, 262144])
+@pytest.mark.parametrize("nfft", [32768, 49152, 65536, 131072, 262144])
 def test_maxima_of_row_spectra_equal_the_composed_search(spx, nfft):
     """All maxima from the row layout of the two-launch transforms against the
     transform in bin order and the search on it: windows that start and end
