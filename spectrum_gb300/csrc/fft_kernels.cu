@@ -45,19 +45,28 @@ fft_out_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __r
 // thread in packed arithmetic (fft_pair.cuh), M / 32 threads of up to 128
 // registers (64 of them the butterflies), 16 warps per SM at every size.
 // Measured against fft_out_kernel<16> (same bits): 8192 x 4096 |X|^2 0.133 ->
-// 0.089 ms (4.5 TB/s of input and output), 2048 x 16384 inverse 0.191 -> 0.153 ms.
+// 0.089 ms, 2048 x 16384 inverse 0.191 -> 0.153 ms; with the window loaded beside
+// the samples 8192 x 4096 0.080 ms (5.0 TB/s of input and output); 4096 x 8192
+// complex 0.163 -> 0.114, inverse 0.167 -> 0.104 with the two-exchange plan
+// (0.136 before it and the window loads).  16384 points: one CTA per SM, whose
+// load, exchange and store phases do not overlap (33 % of the issue slots, 50 %
+// of the L1's data path).
 template <int M>
 constexpr int kPairMinBlocks = M >= 16384 ? 1 : M == 8192 ? 2 : M == 4096 ? 4 : M == 2048 ? 8 : 16;
 
 template <int M, int MODE>
 __global__ void __launch_bounds__(M / 32, kPairMinBlocks<M>)
 fft_pair_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __restrict__ win, FftGeom g,
-                const float4* __restrict__ tw, void* __restrict__ out, uint32_t out_mode, float scale) {
+                const float2* __restrict__ tw, const float4* __restrict__ tw_pair, void* __restrict__ out,
+                uint32_t out_mode, float scale) {
   extern __shared__ float4 s4[];
   const uint32_t tid = threadIdx.x, beam = blockIdx.x;
   prefetch_future_beam(g, in, n_point, beam, 0, tid, M / 32);
-  pair_local_fft_out<M>(s4, SamplePairs(in + (size_t)beam * n_point, n_point, win), tw, tid,
-                        BinOutPairs<M, MODE>(out, out_mode, scale, g, beam));
+  const SamplePairs ld(in + (size_t)beam * n_point, n_point, win);
+  if constexpr (M == 8192)
+    pair8k_fft_out(s4, ld, tw, tid, BinOut8k<MODE>{out, out_mode, beam, scale, g});
+  else
+    pair_local_fft_out<M>(s4, ld, tw_pair, tid, BinOutPairs<M, MODE>(out, out_mode, scale, g, beam));
 }
 
 // ---------------------------------------------------------------------------
@@ -487,7 +496,7 @@ static cudaError_t launch_beams(K kernel, FftGeom& g, uint32_t beams, size_t sme
 // fft_pair_kernel of the plan's size; 16-byte stores (8-byte for magnitudes)
 // need that alignment of d_out, other outputs take the general form.
 template <int M>
-static cudaError_t launch_pair_m(FftGeom g, const float4* tw, const float2* d_in, uint32_t beams, uint32_t n_point,
+static cudaError_t launch_pair_m(FftGeom g, const float2* tw, const float4* twp, const float2* d_in, uint32_t beams, uint32_t n_point,
                                  const float* d_win, uint32_t out_mode, float scale, void* d_out,
                                  cudaStream_t stream, bool prefetch) {
   const uintptr_t mis = reinterpret_cast<uintptr_t>(d_out);
@@ -503,7 +512,7 @@ static cudaError_t launch_pair_m(FftGeom g, const float4* tw, const float2* d_in
   g.beams = beams;
   g.ahead = prefetch ? resident_ctas(kfn, M / 32, smem, 1) : 0u;
   void* args[] = {(void*)&d_in, (void*)&n_point, (void*)&d_win, (void*)&g,
-                  (void*)&tw,   (void*)&d_out,   (void*)&out_mode, (void*)&scale};
+                  (void*)&tw,   (void*)&twp,     (void*)&d_out, (void*)&out_mode, (void*)&scale};
   return cudaLaunchKernel(kfn, dim3(beams), dim3(M / 32), args, smem, stream);
 }
 
@@ -511,7 +520,7 @@ static cudaError_t launch_pair(const FftPlan& plan, const float2* d_in, uint32_t
                                const float* d_win, uint32_t out_mode, float scale, void* d_out, cudaStream_t stream,
                                bool prefetch) {
   auto go = [&](auto m) {
-    return launch_pair_m<decltype(m)::value>(plan.g, plan.d_tw_pair, d_in, beams, n_point, d_win, out_mode, scale,
+    return launch_pair_m<decltype(m)::value>(plan.g, plan.d_tw_local, plan.d_tw_pair, d_in, beams, n_point, d_win, out_mode, scale,
                                              d_out, stream, prefetch);
   };
   switch (plan.g.M) {

@@ -46,6 +46,8 @@ SPX_DEV float2 pfma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); 
 struct C2 {
   float2 x, y;
 };
+SPX_DEV float2 first_of(C2 z) { return make_float2(z.x.x, z.y.x); }
+SPX_DEV float2 second_of(C2 z) { return make_float2(z.x.y, z.y.y); }
 SPX_DEV C2 c2add(C2 a, C2 b) { return C2{padd(a.x, b.x), padd(a.y, b.y)}; }
 SPX_DEV C2 c2sub(C2 a, C2 b) { return C2{psub(a.x, b.x), psub(a.y, b.y)}; }
 // a * w, the operations of cmul on both values
@@ -269,6 +271,13 @@ SPX_DEV float4 ld_stream4(const float2* p) {
   return v;
 }
 
+// Two table values (volatile: issued where it stands).
+SPX_DEV float2 ld_table2(const float* p) {
+  float2 v;
+  asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+
 // Samples n, n + 1 (n even) of a beam: window applied (load_sample's rounded
 // multiplies), zero beyond n_point.  16-byte loads when the beam starts on a
 // 16-byte boundary and n_point is even (no pair then straddles the end), else
@@ -284,21 +293,29 @@ struct SamplePairs {
   SPX_DEV void load(C2 (&v)[R], uint32_t n0, uint32_t step) const {
     float4 a[R];
     if (vec) {
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const uint32_t n = n0 + r * step;
-        a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (n < n_point) a[r] = ld_stream4(x + n);
-      }
-      if (win) {
+      if (win) {  // samples and window in flight together
+        float2 w[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const uint32_t n = n0 + r * step;
+          a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+          w[r] = make_float2(0.f, 0.f);
           if (n < n_point) {
-            const float2 w = __ldg(reinterpret_cast<const float2*>(win + n));
-            a[r] = make_float4(__fmul_rn(a[r].x, w.x), __fmul_rn(a[r].y, w.x), __fmul_rn(a[r].z, w.y),
-                               __fmul_rn(a[r].w, w.y));
+            a[r] = ld_stream4(x + n);
+            w[r] = ld_table2(win + n);
           }
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (n0 + r * step < n_point)
+            a[r] = make_float4(__fmul_rn(a[r].x, w[r].x), __fmul_rn(a[r].y, w[r].x), __fmul_rn(a[r].z, w[r].y),
+                               __fmul_rn(a[r].w, w[r].y));
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const uint32_t n = n0 + r * step;
+          a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (n < n_point) a[r] = ld_stream4(x + n);
         }
       }
     } else {
@@ -493,6 +510,79 @@ SPX_DEV void pair_local_fft_out(float4* s, const Load& load, const float4* __res
   pair_last<M, T>(s, tw, tid, out);
 }
 
+// ---- 8192 points -------------------------------------------------------------------
+// Radices 16, 16, 16, 2.  Here a pair is an element and its neighbour at the
+// distance of the NEXT stride: the butterflies j, j + Ns of a pass share their
+// twiddles (one 8-byte load for both) and leave their outputs r as elements e,
+// e + 16 Ns, the next pass's pairs, so the first pass stores its registers as
+// they are, and the third leaves elements e, e + 4096: the last pass's
+// butterflies, finished in registers.  Two exchanges instead of three.
+// (16384 points end in a radix-4 pass over two pairs, 4096 in a radix-16 pass
+// over eight: their last pass would be scalar, which costs more than the pairs
+// of neighbours do.)
+//   pass 0: butterflies 2m, 2m + 1      -> elements 32 m + r, + 16: slot 16 m + r
+//   pass 1: j = 32 a + k and j + 16     -> elements 512 a + 16 r + k, + 256: slot 256 a + 16 r + k
+//   pass 2: j = k and j + 256           -> elements k + 256 r, + 4096: slot 256 r + k
+// out(e, z0, z1) takes elements e and e + 4096.
+SPX_DEV C2 tw_both(const float2* __restrict__ t) {  // one twiddle for both values
+  const float2 w = __ldg(t);
+  return C2{pk(w.x), pk(w.y)};
+}
+template <typename Load, typename Out>
+SPX_DEV void pair8k_fft_out(float4* s, const Load& load, const float2* __restrict__ tw, uint32_t tid, const Out& out) {
+  using P = CtPlan<8192>;
+  static_assert(P::npass == 4 && P::radix(0) == 16 && P::radix(1) == 16 && P::radix(2) == 16 && P::radix(3) == 2, "plan");
+  constexpr uint32_t step = 256 + 16;  // slots between a pass's inputs
+  C2 v[16];
+  load.load(v, 2 * tid, 512);
+  PDft<16>::run(v);
+#pragma unroll
+  for (int r = 0; r < 16; ++r) s[17 * tid + r] = make_float4(v[r].x.x, v[r].x.y, v[r].y.x, v[r].y.y);
+  __syncthreads();
+  const float4* p = s + ps(tid);
+#pragma unroll
+  for (int q = 1; q <= 2; ++q) {
+    const uint32_t Ns = q == 1 ? 16 : 256, k = tid & (Ns - 1);
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+      const float4 a = p[r * step];
+      v[r] = C2{make_float2(a.x, a.y), make_float2(a.z, a.w)};
+    }
+    if (q == 1) __syncthreads();
+    const float2* t = tw + P::twoff(q) + k;
+#pragma unroll
+    for (int r = 1; r < 16; ++r) v[r] = c2mul(v[r], tw_both(t + (r - 1) * Ns));
+    PDft<16>::run(v);
+    if (q == 1) {
+      float4* d = s + ps(256 * (tid >> 4)) + k;
+#pragma unroll
+      for (int r = 0; r < 16; ++r) d[17 * r] = make_float4(v[r].x.x, v[r].x.y, v[r].y.x, v[r].y.y);
+      __syncthreads();
+    }
+  }
+  // (the last twiddles all in flight before the outputs, whose square roots
+  // would keep the compiler from issuing them early)
+  float2 w[16];
+#pragma unroll
+  for (int r = 0; r < 16; ++r) w[r] = ld_table2(reinterpret_cast<const float*>(tw + P::twoff(3) + tid + 256 * r));
+#pragma unroll
+  for (int r = 0; r < 16; ++r) {
+    const float2 a = first_of(v[r]), b = cmul(second_of(v[r]), w[r]);
+    out(tid + 256 * r, cadd(a, b), csub(a, b));
+  }
+}
+
+// Result back into the slots (element i at pair8k_elem(s, i)); only slots this
+// thread read.
+struct Slot8kOut {
+  float4* s;
+  SPX_DEV void operator()(uint32_t e, float2 a, float2 b) const { s[ps(e)] = make_float4(a.x, b.x, a.y, b.y); }
+};
+SPX_DEV float2 pair8k_elem(const float4* s, uint32_t i) {
+  const float* f = reinterpret_cast<const float*>(s + ps(i & 4095u)) + (i >> 12);
+  return make_float2(f[0], f[2]);
+}
+
 // Result back into the slots it was read from (element i at pair_elem(s, i)).
 struct SlotOut {
   float4* s;
@@ -505,8 +595,6 @@ SPX_DEV void pair_local_fft(float4* s, const Load& load, const float4* __restric
 }
 
 // ---- outputs -------------------------------------------------------------------------
-SPX_DEV float2 first_of(C2 z) { return make_float2(z.x.x, z.y.x); }
-SPX_DEV float2 second_of(C2 z) { return make_float2(z.x.y, z.y.y); }
 
 // Output of bins i, i + 1 of one beam's natural-order spectrum (the layouts
 // of store_bin); `out` is 16-byte aligned (8 bytes for magnitudes).
@@ -579,6 +667,36 @@ struct BinOutPairs<M, kPairOther> {  // any mode, any alignment
   SPX_DEV void operator()(uint32_t i, C2 z) const {
     store_bin(out, mode, scale, g, beam, i, first_of(z));
     store_bin(out, mode, scale, g, beam, i + 1, second_of(z));
+  }
+};
+
+// Output of elements e and e + 4096 of an 8192-point transform (8192-point
+// specialisations of the modes above; every store of a warp is contiguous).
+template <int MODE>
+struct BinOut8k {
+  void* out;
+  uint32_t mode, beam;
+  float scale;
+  const FftGeom& g;
+  SPX_DEV void one(uint32_t k, float2 z) const {
+    const size_t at = (size_t)beam * 8192 + k;
+    if constexpr (MODE == kPairComplex) {
+      reinterpret_cast<float2*>(out)[at] = z;
+    } else if constexpr (MODE == kPairMag) {
+      const float m2 = mag2_rn(z);
+      reinterpret_cast<float*>(out)[at] = __fmul_rn(mode == SPX_OUT_MAG2 ? m2 : __fsqrt_rn(m2), scale);
+    } else if constexpr (MODE == kPairMagPhase) {
+      reinterpret_cast<float2*>(out)[at] = make_float2(mag_rn(z), atan2f(z.y, z.x));
+    } else if constexpr (MODE == kPairReversed) {
+      reinterpret_cast<float2*>(out)[(size_t)beam * 8192 + ((8192 - k) & 8191)] =
+          make_float2(__fmul_rn(z.x, scale), __fmul_rn(z.y, scale));
+    } else {
+      store_bin(out, mode, scale, g, beam, k, z);
+    }
+  }
+  SPX_DEV void operator()(uint32_t e, float2 a, float2 b) const {
+    one(e, a);
+    one(e + 4096, b);
   }
 };
 
