@@ -33,9 +33,15 @@ MAXVALUE_DTYPE = np.dtype(
 _OUT_MODES = {"complex": OUT_COMPLEX, "mag": OUT_MAG, "mag2": OUT_MAG2, "magphase": OUT_MAGPHASE}
 
 
+_torch_module = None
+
+
 def _torch():
-    import torch
-    return torch
+    global _torch_module
+    if _torch_module is None:
+        import torch
+        _torch_module = torch
+    return _torch_module
 
 
 class Context:
@@ -60,9 +66,8 @@ class Context:
             pass
 
     def bind_stream(self, stream=None) -> None:
-        torch = _torch()
-        s = stream if stream is not None else torch.cuda.current_stream(self.device)
-        check(lib.spx_set_stream(self.h, C.c_void_p(s.cuda_stream)), self.h)
+        s = _raw_stream(self.device) if stream is None else stream.cuda_stream
+        check(lib.spx_set_stream(self.h, s), self.h)
 
     def synchronize(self) -> None:
         self.bind_stream()
@@ -70,6 +75,26 @@ class Context:
 
     def check(self, status: int) -> None:
         check(status, self.h)
+
+
+def _raw_stream(device: int) -> int:
+    """torch's current stream of a device as a cudaStream_t value."""
+    torch = _torch()
+    raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # no Stream object built per call
+    return raw(device) if raw else torch.cuda.current_stream(device).cuda_stream
+
+
+def _zeros(shape, dtype, device):
+    """torch.zeros of a CUDA device, cleared on its current stream."""
+    torch = _torch()
+    t = torch.empty(shape, dtype=dtype, device=device)
+    if t.device.index != torch.cuda.current_device():
+        return t.zero_()
+    if t.numel():
+        err = _capi.memset_async(t.data_ptr(), 0, t.numel() * t.element_size(), _raw_stream(t.device.index))
+        if err:
+            raise RuntimeError(f"cudaMemsetAsync: error {err}")
+    return t
 
 
 _contexts: dict[int, Context] = {}
@@ -90,12 +115,12 @@ def _ctx_for(t, ctx):
 
 
 def _ptr(t):
-    return C.c_void_p(t.data_ptr()) if t is not None else None
+    return t.data_ptr() if t is not None else None
 
 
 def _require_cuda(t, dtype, name):
     torch = _torch()
-    if not isinstance(t, torch.Tensor) or not t.is_cuda:
+    if not (isinstance(t, torch.Tensor) and t.is_cuda):
         raise ValueError(f"{name} must be a CUDA tensor")
     if t.dtype != dtype:
         raise ValueError(f"{name} must be {dtype}, got {t.dtype}")
@@ -219,7 +244,7 @@ def topk(spec, k: int, mag=None, sample_rate: float = 1000.0, search_start: int 
     beams, nfft = spec.reshape(-1, spec.shape[-1]).shape
     if mag is not None:
         _require_cuda(mag, torch.float32, "mag")
-    o = torch.zeros((beams, k, 8), dtype=torch.int32, device=spec.device)
+    o = _zeros((beams, k, 8), torch.int32, spec.device)
     counts = torch.empty(beams, dtype=torch.int32, device=spec.device)
     p = peak_params(PEAK_TOPK, search_start, search_end, 0, k, refine, sample_rate, thresh_sigma)
     c = _ctx_for(spec, ctx)
@@ -234,16 +259,17 @@ def fft_peaks(x, nfft: int, window: int = WINDOW_NONE, mode: int = PEAK_ALL,
     """Raw samples [beams, n_point] -> peaks in one call (layouts as the peak functions)."""
     torch = _torch()
     _require_cuda(x, torch.complex64, "x")
-    x2 = x.reshape(-1, x.shape[-1])
+    x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
     beams, n_point = x2.shape
+    # every row of ONE / TWO and every count of ALL / TOPK is written by the search
     if mode in (PEAK_ONE, PEAK_TWO):
-        per = 4 if mode == PEAK_ONE else 8
-    elif mode == PEAK_ALL:
-        per = _capi.all_maxima_capacity(nfft, search_start, search_end, max_per_beam)[2]
+        o = torch.empty((beams, 4 if mode == PEAK_ONE else 8, 8), dtype=torch.int32, device=x.device)
+        counts = _zeros((beams,), torch.int32, x.device)
     else:
-        per = max_per_beam
-    o = torch.zeros((beams, per, 8), dtype=torch.int32, device=x.device)
-    counts = torch.zeros(beams, dtype=torch.int32, device=x.device)
+        per = (_capi.all_maxima_capacity(nfft, search_start, search_end, max_per_beam)[2] if mode == PEAK_ALL
+               else max_per_beam)
+        o = _zeros((beams, per, 8), torch.int32, x.device)
+        counts = torch.empty((beams,), dtype=torch.int32, device=x.device)
     p = peak_params(mode, search_start, search_end, search_range, max_per_beam, refine,
                     sample_rate, thresh_sigma)
     c = _ctx_for(x, ctx)

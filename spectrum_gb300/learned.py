@@ -166,10 +166,11 @@ class MLPRefiner:
     def gradients(self, x, t, mask=None):
         """-> (gradient [N_PARAMS] CUDA tensor, loss CUDA scalar tensor)."""
         import torch
+        from . import _zeros
         _check_rows(x, N_IN, "x")
         _check_rows(t, N_OUT, "t")
         g = torch.empty(N_PARAMS, dtype=torch.float32, device=x.device)
-        loss = torch.zeros(1, dtype=torch.float32, device=x.device)
+        loss = _zeros((1,), torch.float32, x.device)
         self.ctx.bind_stream()
         self.ctx.check(lib.spx_mlp_gradients(self.ctx.h, self.h, _ptr(x), _ptr(t), _ptr(mask),
                                              x.shape[0], _ptr(g), _ptr(loss)))
@@ -177,9 +178,10 @@ class MLPRefiner:
 
     def train_step(self, x, t, lr: float, mask=None):
         import torch
+        from . import _zeros
         _check_rows(x, N_IN, "x")
         _check_rows(t, N_OUT, "t")
-        loss = torch.zeros(1, dtype=torch.float32, device=x.device)
+        loss = _zeros((1,), torch.float32, x.device)
         self.ctx.bind_stream()
         self.ctx.check(lib.spx_mlp_train_step(self.ctx.h, self.h, _ptr(x), _ptr(t), _ptr(mask),
                                               x.shape[0], float(lr), _ptr(loss)))
@@ -204,10 +206,11 @@ class MLPRefiner:
         spectrum spec [beams, nfft]; returns (amplitude [beams, K] float32,
         used [beams, K] int32: 1 where the network's estimate was kept)."""
         import torch
+        from . import _zeros
         beams, nfft = spec.reshape(-1, spec.shape[-1]).shape
         k = peaks.shape[1]
-        amp = torch.zeros((beams, k), dtype=torch.float32, device=spec.device)
-        used = torch.zeros((beams, k), dtype=torch.int32, device=spec.device)
+        amp = _zeros((beams, k), torch.float32, spec.device)
+        used = _zeros((beams, k), torch.int32, spec.device)
         self.ctx.bind_stream()
         self.ctx.check(lib.spx_mlp_refine(self.ctx.h, self.h, _ptr(spec), beams, int(n_point), nfft,
                                           float(sample_rate), k, _ptr(peaks), _ptr(counts),
@@ -222,14 +225,14 @@ class MLPRefiner:
         int32 MaxValue words, counts [beams], amplitude [beams, K], used
         [beams, K]), the bits of fft_peaks + refine."""
         import torch
-        from . import PEAK_TOPK, _require_cuda
+        from . import PEAK_TOPK, _require_cuda, _zeros
         _require_cuda(x, torch.complex64, "x")
         x2 = x.reshape(-1, x.shape[-1])
         beams, n_point = x2.shape
-        out = torch.zeros((beams, k, 8), dtype=torch.int32, device=x.device)
-        counts = torch.zeros(beams, dtype=torch.int32, device=x.device)
-        amp = torch.zeros((beams, k), dtype=torch.float32, device=x.device)
-        used = torch.zeros((beams, k), dtype=torch.int32, device=x.device)
+        out = _zeros((beams, k, 8), torch.int32, x.device)
+        counts = torch.empty((beams,), dtype=torch.int32, device=x.device)  # written by the search
+        amp = _zeros((beams, k), torch.float32, x.device)
+        used = _zeros((beams, k), torch.int32, x.device)
         p = _capi.peak_params(PEAK_TOPK, search_start, search_end, 0, k, refine, sample_rate, thresh_sigma)
         self.ctx.bind_stream()
         self.ctx.check(lib.spx_fft_peaks_mlp(self.ctx.h, self.h, _ptr(x2), beams, n_point, int(nfft), int(window),
