@@ -66,6 +66,7 @@ struct spx_ctx {
   void* d_scratch[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
   size_t scratch_bytes[6] = {0, 0, 0, 0, 0, 0};
   uint32_t* d_error = nullptr;         // device error word (kErr* bits)
+  uint32_t* h_error = nullptr;         // its page-locked copy, filled by spx_synchronize
   uint32_t epoch = 0;                  // lookback status epoch
   // Host-buffer pipeline (spx_fft_peaks_host): copy streams, staging, events.
   cudaStream_t copy_in = nullptr, copy_out = nullptr;
