@@ -317,9 +317,10 @@ spx_status spx_fft_peaks_host(spx_ctx* ctx, const void* h_in, uint32_t beams,
  * Device scratch is owned by the batch.  A batch's plan for an nfft (its
  * local size M, C = nfft / M) is the context's plan for that nfft: every
  * call on the context uses it.
- *  spx_batch_run           every beam's FFT in ONE launch (clusters of the
- *                          largest C), then one top-K launch
- *  spx_batch_run_per_size  the same kernel once per distinct nfft (the
+ *  spx_batch_run           every beam's FFT in one launch (clusters of the
+ *                          largest C; larger batches of beams above 16384
+ *                          points in two more), then one top-K launch
+ *  spx_batch_run_per_size  the same kernels once per distinct nfft (the
  *                          per-size baseline; bit-identical results)
  *  spx_batch_capture/replay  record spx_batch_run for fixed pointers as a
  *                          CUDA graph on the context's (non-default) stream

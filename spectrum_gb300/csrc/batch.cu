@@ -3,9 +3,9 @@
 // A batch holds, for B beams with their own n_point and nfft (2^a*3^b), the
 // per-size FFT plans, the packing of all beams into the clusters of a single
 // launch, the device scratch (exchange slots) and optionally a CUDA graph of
-// a run.  A run is two launches:
-//   1. fft_batch_kernel: every beam's windowed, zero-padded FFT in ONE
-//      launch.  Beam b with nfft = C x M takes C CTAs (ranks 0..C-1) of one
+// a run.  A run is up to four launches:
+//   1. fft_batch_kernel: the windowed, zero-padded FFT of every beam (of every
+//      beam but those of 1a, where there are many).  Beam b with nfft = C x M takes C CTAs (ranks 0..C-1) of one
 //      cluster; a cluster of Cl CTAs (Cl = the largest C, or more, chosen
 //      by spx_batch_set_cluster or the autotuner) hosts one or
 //      several beams on disjoint rank ranges (first-fit decreasing, largest
@@ -17,8 +17,14 @@
 //      plan otherwise), and leaves the row in the slot (row c: X[c + C*i]).
 //      It also prefetches into L2 the samples of the CTA one residency wave
 //      later.
+//   1a. batch_cols_kernel, beside it, and batch_rows_kernel (batch_rows.cuh):
+//      the beams of C x M points, C >= 2, with M one of the common local sizes
+//      (96 % of the points of lengths U[1000, 100000]), once they hold
+//      kBrMinPoints: 1024 such beams, Hann, top-8: 0.733 -> 0.564 ms
+//      (columns 0.27 ms, rows 0.20, top-K 0.09).
 //   2. topk_batch_kernel: the K largest strict local maxima of every beam,
-//      one CTA per beam, reading bin k from row k mod C of the beam's slot.
+//      one CTA per beam, reading bin k from row k mod C of the beam's slot (or
+//      from the rows of 1a).
 // The plans are the context's plans for those sizes and the window is
 // evaluated by window_at (the function that fills spx_fft's tables): every
 // beam's list is the bits of spx_fft_peaks on that beam alone.
@@ -47,6 +53,7 @@
 #include <sstream>
 #include <vector>
 
+#include "batch_rows.cuh"
 #include "fft_core.cuh"
 #include "spx_internal.h"
 
@@ -66,6 +73,10 @@ struct BatchGeom {
   FftGeom g;
   const float2* twl;
   const float2* twc;
+  // beams of batch_rows.cuh: row pairs' twiddles (null: the cluster kernel), R0,
+  // L = M / R0, NP = ceil(R0 / 2)
+  const float4* twr;
+  uint32_t R0, L, NP, pairs;  // pairs per CTA of the second launch
 };
 
 constexpr uint32_t kBpThreads = 1024;  // threads of a batch CTA (16 points each at M = 16384)
@@ -221,6 +232,67 @@ SPX_DEV uint64_t bt_scan(const Bins& bins, uint32_t start, uint32_t end, uint32_
   return mine;
 }
 
+// The same for a beam of batch_rows.cuh: element q of row (k1, r0), at
+// (k1 2 NP + r0) L + q, is bin rho + C R0 q, rho = k1 + C r0.  A lane owns column
+// q and walks its C R0 consecutive bins, R0 loads (256 bytes a warp) at a time;
+// the bins before and after the column come from the neighbouring columns.
+template <uint32_t R0>
+SPX_DEV uint64_t br_scan(const float2* rows, uint32_t C, uint32_t L, uint32_t start, uint32_t end, uint32_t K,
+                         uint32_t lane, uint32_t warp) {
+  constexpr uint32_t NP2 = 2 * ((R0 + 1) / 2), U = R0 == 9 ? 9 : 8;
+  const uint32_t CB = C * R0, q_lo = start / CB, q_hi = (end - 1) / CB;
+  uint64_t mine = 0;
+  // |X|^2 below which no bin's rounded square root reaches the list's K-th entry
+  // (0: the list is not full).  The test of a bin is on |X|^2: sqrt_rn never
+  // turns a smaller value into a larger one, so it lets every maximum of |X|
+  // through, and the few bins that pass it are tested on |X| itself.
+  float least2 = 0.f;
+  for (uint32_t q0 = q_lo + warp * 32; q0 <= q_hi; q0 += kBtThreads) {
+    const uint32_t q = q0 + lane;
+    const bool in = q <= q_hi;
+    const float2* col = rows + q;
+    float l = 0.f, c = 0.f;  // |X|^2 of bins k - 1 and k
+    if (in && q * CB >= start) l = mag2_rn(__ldg(rows + (size_t)((C - 1) * NP2 + R0 - 1) * L + q - 1));
+    if (in) c = mag2_rn(__ldg(col));
+    // bins of the column in the window: [klo, khi), none for lanes past the end
+    const uint32_t klo = max(start, q * CB), khi = in ? min(end, (q + 1) * CB) : 0u;
+    uint32_t k = q * CB, k1 = 0, r0 = 0;
+    for (uint32_t b = 0; b < CB; b += U) {
+      float2 z[U];  // bins k + 1 .. k + U
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u) {
+        if (++k1 == C) {
+          k1 = 0;
+          ++r0;
+        }
+        z[u] = make_float2(0.f, 0.f);
+        if (in && k + u < end) z[u] = r0 < R0 ? __ldg(col + (k1 * NP2 + r0) * L) : __ldg(col + 1);
+      }
+#pragma unroll
+      for (uint32_t u = 0; u < U; ++u, ++k) {
+        const float r = mag2_rn(z[u]);
+        uint32_t want = __ballot_sync(0xffffffffu, c > l && c > r && c >= least2 && k >= klo && k < khi);
+        if (want) {
+          const float cm = __fsqrt_rn(c);
+          const uint64_t key = ((uint64_t)__float_as_uint(cm) << 32) | (uint32_t)(~k);
+          const uint64_t kth = __shfl_sync(0xffffffffu, mine, K - 1);
+          want &= __ballot_sync(0xffffffffu, cm > __fsqrt_rn(l) && cm > __fsqrt_rn(r) && key > kth);
+          while (want) {
+            const int src = __ffs(want) - 1;
+            want &= want - 1;
+            mine = warp_list_insert(mine, __shfl_sync(0xffffffffu, key, src), lane);
+          }
+          const float least = __uint_as_float((uint32_t)(__shfl_sync(0xffffffffu, mine, K - 1) >> 32));
+          least2 = 0.999999f * (least * least);
+        }
+        l = c;
+        c = r;
+      }
+    }
+  }
+  return mine;
+}
+
 // The K largest strict local maxima of every beam's spectrum (one CTA per
 // beam; beam_list orders the CTAs, largest spectra first): per-warp lists
 // merged by warp 0, which writes the MaxValues with the rules and arithmetic
@@ -239,14 +311,19 @@ topk_batch_kernel(const float2* __restrict__ xch, const BatchBeam* __restrict__ 
   if (end >= nfft) end = nfft - 1;
   const uint32_t C = geoms[bm.geom].g.C, M = geoms[bm.geom].g.M;
   const RowBins bins{xch + bm.spec_off, M};
+  const bool br = geoms[bm.geom].twr != nullptr;
+  const uint32_t R0 = geoms[bm.geom].R0, L = geoms[bm.geom].L, NP = geoms[bm.geom].NP;
   const uint32_t cmagic = 0xFFFFFFFFu / C + 1u;  // k div C = umulhi(k, cmagic) (k * C < 2^32)
   auto bin = [&](uint32_t k) -> float2 {
-    const uint32_t q = C == 1 ? k : __umulhi(k, cmagic);
-    return bins(k - q * C, q);
+    const uint32_t q = C == 1 ? k : __umulhi(k, cmagic), k1 = k - q * C;
+    return br ? __ldg(xch + bm.spec_off + (size_t)(k1 * 2 * NP + q % R0) * L + q / R0) : bins(k1, q);
   };
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint64_t mine = 0;
-  if (start < end) {
+  if (start < end && br) {  // (the same for the whole CTA)
+    const float2* rows = xch + bm.spec_off;
+    mine = R0 == 9 ? br_scan<9>(rows, C, L, start, end, a.K, lane, warp) : br_scan<16>(rows, C, L, start, end, a.K, lane, warp);
+  } else if (start < end) {
     switch (C) {  // the same for the whole CTA
       case 1: mine = bt_scan<1, kBtThreads>(bins, start, end, a.K, lane, warp); break;
       case 2: mine = bt_scan<2, kBtThreads>(bins, start, end, a.K, lane, warp); break;
@@ -287,6 +364,8 @@ topk_batch_kernel(const float2* __restrict__ xch, const BatchBeam* __restrict__ 
 __global__ void __launch_bounds__(kBpThreads, 1) fft_batch_kernel(BatchArgs a) {
   extern __shared__ float2 s[];
   cg::cluster_group cl = cg::this_cluster();
+  // the column kernel of the larger beams need not wait for this one
+  asm volatile("griddepcontrol.launch_dependents;");
   // L2 prefetch of the samples the CTA one residency wave later reads first
   if (a.ahead && blockIdx.x + a.ahead < gridDim.x) {
     const BatchCta f = a.ctas[blockIdx.x + a.ahead];
@@ -316,6 +395,98 @@ __global__ void __launch_bounds__(kBpThreads, 1) fft_batch_kernel(BatchArgs a) {
   }
 }
 
+// The two launches of batch_rows.cuh; a CTA takes item d.c of beam d.beam.
+// (largest transforms first; the samples of the tile one residency wave later
+// are prefetched into L2)
+__global__ void __launch_bounds__(kBrThreads, 4) batch_cols_kernel(BatchArgs a, const BatchCta* __restrict__ items) {
+  extern __shared__ float4 s4[];
+  if (a.ahead && blockIdx.x + a.ahead < gridDim.x) {
+    const BatchCta f = items[blockIdx.x + a.ahead];
+    const BatchBeam fb = a.beams[f.beam];
+    const BatchGeom* fg = a.geoms + fb.geom;
+    const uint32_t W = 2 * (uint32_t)br_hw((int)fg->g.C, (int)fg->R0), rows = fg->g.C * fg->R0;
+    for (uint32_t r = threadIdx.x; r < rows; r += kBrThreads) {
+      const uint32_t lo = r * fg->L + f.c * W, hi = min(min(lo + W, (r + 1) * fg->L), fb.n_point);
+      if (lo < hi) prefetch_l2(a.in + fb.in_off + lo, (size_t)(hi - lo) * sizeof(float2), 0, 1);
+    }
+  }
+  const BatchCta d = items[blockIdx.x];
+  const BatchBeam bm = a.beams[d.beam];
+  const BatchGeom* bg = a.geoms + bm.geom;
+  const BatchSamples ld{a.in + bm.in_off, bm.n_point, make_window_gen(a.window, bm.n_point)};
+  const uint32_t M = bg->g.M, L = bg->L;
+  const float2* twc = bg->twc;
+  float4* slot = reinterpret_cast<float4*>(a.xch + bm.spec_off);
+  auto go = [&](auto c, auto r) {
+    constexpr int C = decltype(c)::value, R = decltype(r)::value;
+    br_cols<C, R>(s4, ld, M, L, d.c * 2 * br_hw(C, R), twc, slot);
+  };
+  // (launched beside fft_batch_kernel, whose beams it does not touch; the wait
+  // below makes this launch's end the end of both)
+  auto with_c = [&](auto r) {
+    switch (bg->g.C) {
+      case 2: go(std::integral_constant<int, 2>(), r); break;
+      case 3: go(std::integral_constant<int, 3>(), r); break;
+      case 4: go(std::integral_constant<int, 4>(), r); break;
+      case 6: go(std::integral_constant<int, 6>(), r); break;
+      case 8: go(std::integral_constant<int, 8>(), r); break;
+      default: go(std::integral_constant<int, 9>(), r); break;
+    }
+  };
+  if (bg->R0 == 16)
+    with_c(std::integral_constant<int, 16>());
+  else
+    with_c(std::integral_constant<int, 9>());
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(kBrThreads, 4)
+batch_rows_kernel(BatchArgs a, const BatchCta* __restrict__ items, uint32_t start, uint32_t end) {
+  extern __shared__ float4 s4[];
+  const BatchCta d = items[blockIdx.x];
+  const BatchBeam bm = a.beams[d.beam];
+  const BatchGeom* bg = a.geoms + bm.geom;
+  // elements that hold bins [start - 1, end + 1) of the search window
+  if (start == 0) start = 1;
+  if (end == 0) end = bm.nfft / 2;
+  if (end >= bm.nfft) end = bm.nfft - 1;
+  const uint32_t CB = bg->g.C * bg->R0, qlo = (start - 1) / CB, qhi = end < start ? 0u : (end + CB) / CB;
+  if (a.ahead && blockIdx.x + a.ahead < gridDim.x && threadIdx.x < 2) {  // L2 prefetch of the pairs one residency wave later
+    const BatchCta f = items[blockIdx.x + a.ahead];
+    const BatchBeam fb = a.beams[f.beam];
+    const uint32_t fl = a.geoms[fb.geom].L, n = (uint32_t)a.geoms[fb.geom].pairs * fl;  // elements x 2 of an item
+    prefetch_l2(a.xch + fb.spec_off + (size_t)f.c * n * 2 + threadIdx.x * n, (size_t)n * sizeof(float2), 0, 1);
+  }
+  br_switch(bg->g.M, [&](auto m) {
+    br_rows<decltype(m)::value>(s4, d.c, a.xch + bm.spec_off, bg->twr, qlo, qhi);
+  });
+}
+
+// Twiddles of the row pairs of local size g.M (its scalar tables at twl), as
+// br_pass reads them: per pair i and pass, [r - 1][q] = W^{r (R0 q + 2 i)} and
+// W^{r (R0 q + 2 i + 1)}; a split radix-4 table's products as tw4 forms them.
+std::vector<float4> br_tables(const FftGeom& g, const float2* twl) {
+  const uint32_t R0 = g.radix[0], NP = (R0 + 1) / 2;
+  std::vector<float4> t;
+  for (uint32_t i = 0; i < NP; ++i)
+    for (uint32_t p = 1; p < g.npass; ++p) {
+      const uint32_t R = g.radix[p], Ns = g.ns[p];
+      const float2* w = twl + g.twoff[p];
+      auto value = [&](uint32_t r, uint32_t k) {
+        if (!tw_split(R, Ns)) return w[(r - 1) * Ns + k];
+        const float2 a = w[64 + (k >> 6)], b = w[k & 63u];
+        return make_float2(std::fmaf(a.x, b.x, -a.y * b.y), std::fmaf(a.x, b.y, a.y * b.x));
+      };
+      for (uint32_t r = 1; r <= tw_rows(R); ++r)
+        for (uint32_t q = 0; q < Ns / R0; ++q) {
+          const uint32_t k = R0 * q + 2 * i;
+          const float2 a = value(r, k), b = value(r, 2 * i + 1 < R0 ? k + 1 : k);
+          t.push_back(make_float4(a.x, b.x, a.y, b.y));
+        }
+    }
+  return t;
+}
+
 }  // namespace spx
 
 // ---------------------------------------------------------------------------
@@ -328,6 +499,8 @@ struct LaunchSet {  // one FFT launch (packed CTA table, cluster size) and its t
   BatchCta* d_ctas = nullptr;
   uint32_t* d_beam_list = nullptr;  // the top-K launch's beams, largest spectra first
   uint32_t n_ctas = 0, cluster = 1, beams = 0;
+  BatchCta *d_cols = nullptr, *d_rows = nullptr;  // items of batch_rows.cuh
+  uint32_t n_cols = 0, n_rows = 0;
 };
 
 struct spx_batch {
@@ -353,6 +526,11 @@ struct spx_batch {
 };
 
 namespace {
+
+// Fewest points in beams of batch_rows.cuh that take its launches: 64 beams of
+// 1000 .. 100000 samples (3.1 M points) run as long either way (0.107 ms), 300 of
+// up to 50000 (7.4 M) 0.134 -> 0.117 ms.
+constexpr uint64_t kBrMinPoints = 1ull << 22;
 
 constexpr uint32_t kClusterSizes[] = {1, 2, 3, 4, 6, 8, 9, 12, 16};
 
@@ -439,6 +617,10 @@ spx_status build(spx_ctx* ctx, spx_batch* b) {
   b->tables.clear();
   b->d_beams = nullptr;
   b->d_geoms = nullptr;
+  // beams for batch_rows.cuh: a launch more, which pays from kBrMinPoints on
+  auto by_items = [](uint32_t nfft, uint32_t M) { return nfft > M && nfft / M <= kBrMaxC && br_size(M); };
+  uint64_t item_points = 0;
+  for (uint32_t n : b->nfft) item_points += by_items(n, b->local[n]) ? n : 0u;
   std::map<uint32_t, uint32_t> geom_of;  // nfft -> geometry index
   std::vector<BatchGeom> geoms;
   for (auto& kv : b->local) {
@@ -446,7 +628,24 @@ spx_status build(spx_ctx* ctx, spx_batch* b) {
     spx_status st = plan_with_local(ctx, kv.first, kv.second, &plan);
     if (st != SPX_OK) return st;
     geom_of[kv.first] = (uint32_t)geoms.size();
-    geoms.push_back(BatchGeom{plan->g, plan->d_tw_local, plan->d_tw_cross});
+    BatchGeom bg{plan->g, plan->d_tw_local, plan->d_tw_cross, nullptr, 0, 0, 0, 0};
+    if (item_points >= kBrMinPoints && plan->g.ept == 16 && by_items(kv.first, plan->g.M)) {
+      float4*& table = ctx->batch_tables[plan->g.M];
+      if (!table) {
+        std::vector<float2> twl(plan->g.M);
+        fill_local_twiddles(plan->g, twl.data());
+        const std::vector<float4> t = br_tables(plan->g, twl.data());
+        cudaError_t e = cudaMalloc(&table, t.size() * sizeof(float4));
+        if (e == cudaSuccess) e = cudaMemcpy(table, t.data(), t.size() * sizeof(float4), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "batch row twiddles");
+      }
+      bg.twr = table;
+      bg.R0 = plan->g.radix[0];
+      bg.L = plan->g.M / bg.R0;
+      bg.NP = (bg.R0 + 1) / 2;
+      br_switch(bg.g.M, [&](auto m) { bg.pairs = kBrThreads / BrSize<decltype(m)::value>::T; });
+    }
+    geoms.push_back(bg);
   }
   std::vector<BatchBeam> beams(b->beams);
   std::vector<uint32_t> group(b->beams);
@@ -455,43 +654,87 @@ spx_status build(spx_ctx* ctx, spx_batch* b) {
     beams[i] = BatchBeam{in_off, spec_off, b->n_point[i], b->nfft[i], geom_of[b->nfft[i]], 0};
     group[i] = geoms[geom_of[b->nfft[i]]].g.C;
     in_off += b->n_point[i];
-    spec_off += (b->nfft[i] + 31u) & ~31u;  // 256-byte aligned spectra
+    const BatchGeom& bg = geoms[geom_of[b->nfft[i]]];
+    const uint32_t slot = bg.twr ? bg.g.C * 2 * bg.NP * bg.L : b->nfft[i];
+    spec_off += (slot + 31u) & ~31u;  // 256-byte aligned spectra
   }
   b->in_total = in_off;
   b->spec_total = spec_off;
   spx_status st = upload(ctx, b, beams, &b->d_beams);
   if (st == SPX_OK) st = upload(ctx, b, geoms, &b->d_geoms);
   if (st != SPX_OK) return st;
-  auto make_set = [&](const std::vector<uint32_t>& ids, uint32_t nfft, LaunchSet* ls) -> spx_status {
+  // the tables of every launch set, one after another (uploaded once: a set's
+  // pointers hold offsets until then)
+  std::vector<BatchCta> ctas, cols, rows;
+  std::vector<uint32_t> lists;
+  struct Offsets {
+    LaunchSet* ls;
+    size_t ctas, cols, rows, list;
+  };
+  std::vector<Offsets> offsets;
+  auto geom = [&](uint32_t id) -> const BatchGeom& { return geoms[beams[id].geom]; };
+  auto make_set = [&](const std::vector<uint32_t>& ids, uint32_t nfft, LaunchSet* ls) {
+    offsets.push_back(Offsets{ls, ctas.size(), cols.size(), rows.size(), lists.size()});
+    const Offsets& o = offsets.back();
     uint32_t cl = 1;
     for (uint32_t id : ids) cl = std::max(cl, group[id]);
     // the single launch may use larger clusters than its largest beam needs
     // (several beams per cluster): how many fit at once depends on how the
     // cluster size divides the GPU's SM groups
     if (nfft == 0 && b->cluster_pref > cl) cl = b->cluster_pref;
-    const std::vector<BatchCta> ctas = pack(ids, group, b->nfft, cl);
-    ls->nfft = nfft;
-    ls->n_ctas = (uint32_t)ctas.size();
-    ls->cluster = cl;
-    ls->beams = (uint32_t)ids.size();
     std::vector<uint32_t> by_size(ids);
     std::stable_sort(by_size.begin(), by_size.end(),
                      [&](uint32_t x, uint32_t y) { return b->nfft[x] > b->nfft[y]; });
-    spx_status s2 = upload(ctx, b, ctas, &ls->d_ctas);
-    if (s2 == SPX_OK) s2 = upload(ctx, b, by_size, &ls->d_beam_list);
-    return s2;
+    lists.insert(lists.end(), by_size.begin(), by_size.end());
+    // beams of batch_rows.cuh: the column tiles by transform size, largest first;
+    // the row items by local size and pair number (CTAs that run at the same time
+    // read the same 8 .. 12 KB of twiddles); the others packed into clusters
+    std::vector<uint32_t> others;
+    std::map<uint32_t, std::vector<uint32_t>, std::greater<uint32_t>> by_local;
+    for (uint32_t id : by_size) {
+      const BatchGeom& bg = geom(id);
+      if (!bg.twr) continue;
+      by_local[bg.g.M].push_back(id);
+      const uint32_t W = 2 * (uint32_t)br_hw((int)bg.g.C, (int)bg.R0), tiles = (bg.L + W - 1) / W;
+      for (uint32_t t = 0; t < tiles; ++t) cols.push_back(BatchCta{id, t});
+    }
+    for (const auto& kv : by_local) {
+      const uint32_t per = geom(kv.second[0]).NP / geom(kv.second[0]).pairs;  // items per k1
+      for (uint32_t i = 0; i < per; ++i)
+        for (uint32_t id : kv.second)
+          for (uint32_t k1 = 0; k1 < geom(id).g.C; ++k1) rows.push_back(BatchCta{id, k1 * per + i});
+    }
+    for (uint32_t id : ids)
+      if (!geom(id).twr) others.push_back(id);
+    const std::vector<BatchCta> packed = pack(others, group, b->nfft, cl);
+    ctas.insert(ctas.end(), packed.begin(), packed.end());
+    ls->nfft = nfft;
+    ls->cluster = cl;
+    ls->beams = (uint32_t)ids.size();
+    ls->n_ctas = (uint32_t)(ctas.size() - o.ctas);
+    ls->n_cols = (uint32_t)(cols.size() - o.cols);
+    ls->n_rows = (uint32_t)(rows.size() - o.rows);
   };
   std::vector<uint32_t> all(b->beams);
   for (uint32_t i = 0; i < b->beams; ++i) all[i] = i;
-  st = make_set(all, 0, &b->all);
-  if (st != SPX_OK) return st;
   std::map<uint32_t, std::vector<uint32_t>, std::greater<uint32_t>> by_size;
   for (uint32_t i = 0; i < b->beams; ++i) by_size[b->nfft[i]].push_back(i);
-  b->per_size.clear();
-  for (auto& kv : by_size) {
-    b->per_size.emplace_back();
-    st = make_set(kv.second, kv.first, &b->per_size.back());
-    if (st != SPX_OK) return st;
+  b->per_size.assign(by_size.size(), LaunchSet{});
+  make_set(all, 0, &b->all);
+  size_t next = 0;
+  for (auto& kv : by_size) make_set(kv.second, kv.first, &b->per_size[next++]);
+  BatchCta *d_ctas = nullptr, *d_cols = nullptr, *d_rows = nullptr;
+  uint32_t* d_lists = nullptr;
+  st = upload(ctx, b, ctas, &d_ctas);
+  if (st == SPX_OK) st = upload(ctx, b, cols, &d_cols);
+  if (st == SPX_OK) st = upload(ctx, b, rows, &d_rows);
+  if (st == SPX_OK) st = upload(ctx, b, lists, &d_lists);
+  if (st != SPX_OK) return st;
+  for (const Offsets& o : offsets) {
+    o.ls->d_ctas = d_ctas + o.ctas;
+    o.ls->d_cols = d_cols + o.cols;
+    o.ls->d_rows = d_rows + o.rows;
+    o.ls->d_beam_list = d_lists + o.list;
   }
   if (b->graph) {  // recorded with the old tables
     cudaGraphExecDestroy(b->graph);
@@ -527,8 +770,35 @@ spx_status launch_set(spx_ctx* ctx, spx_batch* b, const LaunchSet& ls, const voi
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  e = cudaLaunchKernelExC(&cfg, kfn, args);
+  if (ls.n_ctas) e = cudaLaunchKernelExC(&cfg, kfn, args);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "launch fft_batch_kernel");
+  if (ls.n_cols) {
+    const void* kc = (const void*)batch_cols_kernel;
+    const void* kr = (const void*)batch_rows_kernel;
+    e = configure_kernel(kc, kBrColsSmem);
+    if (e == cudaSuccess) e = configure_kernel(kr, kBrRowsSmem);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "configure batch_cols_kernel");
+    BatchArgs ac = a;
+    ac.ahead = ctx->input_on_host ? 0u : resident_ctas(kc, kBrThreads, kBrColsSmem, 1);
+    uint32_t start = b->start, end = b->end;
+    void* cargs[] = {(void*)&ac, (void*)&ls.d_cols};
+    BatchArgs ar = a;
+    ar.ahead = resident_ctas(kr, kBrThreads, kBrRowsSmem, 1);
+    void* rargs[] = {(void*)&ar, (void*)&ls.d_rows, (void*)&start, (void*)&end};
+    cudaLaunchConfig_t cc = {};
+    cc.gridDim = dim3(ls.n_cols, 1, 1);
+    cc.blockDim = dim3(kBrThreads, 1, 1);
+    cc.dynamicSmemBytes = kBrColsSmem;
+    cc.stream = ctx->stream;
+    cudaLaunchAttribute overlap[1];
+    overlap[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    overlap[0].val.programmaticStreamSerializationAllowed = 1;
+    cc.attrs = overlap;
+    cc.numAttrs = ls.n_ctas ? 1 : 0;
+    e = cudaLaunchKernelExC(&cc, kc, cargs);
+    if (e == cudaSuccess) e = cudaLaunchKernel(kr, dim3(ls.n_rows), dim3(kBrThreads), rargs, kBrRowsSmem, ctx->stream);
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "launch batch_cols_kernel / batch_rows_kernel");
+  }
   const TopkArgs tk{reinterpret_cast<MaxValueDev*>(d_out), d_counts, b->K, b->start, b->end, b->refine, b->fs};
   topk_batch_kernel<<<ls.beams, kBtThreads, 0, ctx->stream>>>(b->d_xch, b->d_beams, b->d_geoms, ls.d_beam_list, tk);
   e = cudaGetLastError();
@@ -676,6 +946,11 @@ spx_status spx_batch_capture(spx_ctx* ctx, spx_batch* batch, const void* d_in,
   cudaError_t e = configure_kernel((const void*)fft_batch_kernel, kBpSmem);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "configure fft_batch_kernel");
   resident_ctas((const void*)fft_batch_kernel, kBpThreads, kBpSmem, batch->all.cluster);
+  if (e == cudaSuccess) e = configure_kernel((const void*)batch_cols_kernel, kBrColsSmem);
+  if (e == cudaSuccess) e = configure_kernel((const void*)batch_rows_kernel, kBrRowsSmem);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "configure batch_cols_kernel");
+  resident_ctas((const void*)batch_cols_kernel, kBrThreads, kBrColsSmem, 1);
+  resident_ctas((const void*)batch_rows_kernel, kBrThreads, kBrRowsSmem, 1);
   e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamBeginCapture");
   st = launch_set(ctx, batch, batch->all, d_in, d_out, d_counts);

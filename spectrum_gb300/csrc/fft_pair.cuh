@@ -271,6 +271,15 @@ SPX_DEV float4 ld_stream4(const float2* p) {
   return v;
 }
 
+// Two complex values that are read once (not kept in L1, which holds the
+// twiddles): memory this launch may write later, so not the read-only path.
+SPX_DEV float4 ld_once4(const void* p) {
+  float4 v;
+  asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
+  return v;
+}
+
 // Two table values (volatile: issued where it stands).
 SPX_DEV float2 ld_table2(const float* p) {
   float2 v;

@@ -144,6 +144,7 @@ spx_status spx_destroy(spx_ctx* ctx) {
     cudaStreamSynchronize(ctx->stream);
     ctx->plans.clear();
     for (auto& kv : ctx->windows) cudaFree(kv.second);
+    for (auto& kv : ctx->batch_tables) cudaFree(kv.second);
     for (int i = 0; i < kSlots; ++i)
       if (ctx->d_scratch[i]) cudaFree(ctx->d_scratch[i]);
     if (ctx->d_error) cudaFree(ctx->d_error);

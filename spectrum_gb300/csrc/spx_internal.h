@@ -61,6 +61,7 @@ struct spx_ctx {
   std::string last_error;
   std::map<uint64_t, std::unique_ptr<spx::FftPlan>> plans;  // (ept, points/CTA, nfft)
   std::map<uint32_t, std::pair<uint32_t, uint32_t>> tuning;  // nfft -> (points/thread, points/CTA)
+  std::map<uint32_t, float4*> batch_tables;  // local size -> row-pair twiddles (batch_rows.cuh)
   std::map<uint64_t, float*> windows;  // (window << 32 | n_point) -> table
   // Grow-on-demand device scratch, one buffer per slot (see spx::Slot).
   void* d_scratch[6] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
