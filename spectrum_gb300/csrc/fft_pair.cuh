@@ -569,6 +569,7 @@ SPX_DEV void pair8k_fft_out(float4* s, const Load& load, const float2* __restric
       __syncthreads();
     }
   }
+  if constexpr (Out::kMoves) __syncthreads();  // (every input read before the first output)
   // (the last twiddles all in flight before the outputs, whose square roots
   // would keep the compiler from issuing them early)
   float2 w[16];
@@ -581,27 +582,31 @@ SPX_DEV void pair8k_fft_out(float4* s, const Load& load, const float2* __restric
   }
 }
 
-// Result back into the slots (element i at pair8k_elem(s, i)); only slots this
-// thread read.
-struct Slot8kOut {
-  float4* s;
-  SPX_DEV void operator()(uint32_t e, float2 a, float2 b) const { s[ps(e)] = make_float4(a.x, b.x, a.y, b.y); }
+// Result in natural order (element i is the i-th float2; not the slots' layout),
+// elements beyond `last` left out.
+struct Natural8kOut {
+  static constexpr bool kMoves = true;  // other slots than this thread read
+  float2* s;
+  uint32_t last;
+  SPX_DEV void operator()(uint32_t e, float2 a, float2 b) const {
+    s[e] = a;
+    if (e + 4096 <= last) s[e + 4096] = b;
+  }
 };
-SPX_DEV float2 pair8k_elem(const float4* s, uint32_t i) {
-  const float* f = reinterpret_cast<const float*>(s + ps(i & 4095u)) + (i >> 12);
-  return make_float2(f[0], f[2]);
-}
 
-// Result back into the slots it was read from (element i at pair_elem(s, i)).
+// Result back into the slots it was read from (element i at pair_elem(s, i));
+// SlotOutUpTo leaves elements beyond `last` out.
 struct SlotOut {
   float4* s;
   SPX_DEV void operator()(uint32_t i, C2 z) const { s[ps(i >> 1)] = make_float4(z.x.x, z.x.y, z.y.x, z.y.y); }
 };
-template <int M, typename Load>
-SPX_DEV void pair_local_fft(float4* s, const Load& load, const float4* __restrict__ tw, uint32_t tid) {
-  pair_local_fft_out<M>(s, load, tw, tid, SlotOut{s});
-  __syncthreads();
-}
+struct SlotOutUpTo {
+  float4* s;
+  uint32_t last;
+  SPX_DEV void operator()(uint32_t i, C2 z) const {
+    if (i <= last) SlotOut{s}(i, z);
+  }
+};
 
 // ---- outputs -------------------------------------------------------------------------
 
@@ -683,6 +688,7 @@ struct BinOutPairs<M, kPairOther> {  // any mode, any alignment
 // specialisations of the modes above; every store of a warp is contiguous).
 template <int MODE>
 struct BinOut8k {
+  static constexpr bool kMoves = false;
   void* out;
   uint32_t mode, beam;
   float scale;

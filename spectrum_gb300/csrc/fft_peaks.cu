@@ -464,6 +464,150 @@ fft_group_kernel(FftGeom g, FusedArgs a, uint32_t groups) {
   }  // (the next beam's group_arrive barrier orders these reads of s4 before its first pass)
 }
 
+// ---------------------------------------------------------------------------
+// Top-K of power-of-two beams of 1024 .. 16384 points without a threshold, one
+// CTA per beam in packed arithmetic (fft_pair.cuh): the spectrum stays in shared
+// memory, and bins beyond the search are not written there either.  A lane of the
+// search looks at bins 2j, 2j + 1 (one 16-byte load; at most one of them is a
+// maximum) and gets their outer neighbours from the next lanes; the test is on
+// |X|^2 (sqrt_rn never turns a smaller value into a larger one, so every maximum
+// of |X| passes it), and only bins that pass are tested and listed by |X|.
+// ctx (may be null): [beams][K][5], the bins k - 2 .. k + 2 around each peak, for
+// the learned refinement.  4096 x 8192 top-1: 138 us (the transform into device
+// memory and a search kernel: 165), bound by the two CTAs a SM holds, whose loads,
+// exchanges and arithmetic overlap only between the two (41 % of issue slots, half
+// of the shared-memory port); with one |X| per lane and step it was 161.
+// ---------------------------------------------------------------------------
+template <int M>
+__global__ void __launch_bounds__(M / 32, M >= 16384 ? 1 : M == 8192 ? 2 : M == 4096 ? 4 : 8)
+fft_topk_pair_kernel(FftGeom g, FusedArgs a, float2* __restrict__ ctx) {
+  extern __shared__ float4 s4[];
+  constexpr uint32_t T = M / 32, W = T / 32;
+  uint64_t* lists = reinterpret_cast<uint64_t*>(s4 + ps_len(M));  // [W][32]
+  const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, beam = blockIdx.x;
+  prefetch_future_beam(g, a.in, a.n_point, beam, 0, tid, T);
+  const SamplePairs ld(a.in + (size_t)beam * a.n_point, a.n_point, a.win);
+  if constexpr (M == 8192)
+    pair8k_fft_out(s4, ld, a.tw_local, tid, Natural8kOut{reinterpret_cast<float2*>(s4), a.end + 2});
+  else
+    pair_local_fft_out<M>(s4, ld, a.tw_pair, tid, SlotOutUpTo{s4, a.end + 2});
+  asm volatile("griddepcontrol.launch_dependents;");
+  __syncthreads();
+  auto bin = [&](uint32_t k) {
+    if constexpr (M == 8192) return reinterpret_cast<const float2*>(s4)[k];
+    else return pair_elem(s4, k);
+  };
+  // First each warp lists its R largest maxima only.  The K-th of the merged lists
+  // bounds the answer's K-th from below, so a warp whose R-th entry is not above
+  // it has listed all that it can give; the others (few: R is twice a warp's
+  // share and two) scan again for what is above the bound.
+  uint32_t R = min(a.K, 2 * ((a.K + W - 1) / W) + 2);
+  uint64_t own = 0, floor = 0, mine;
+  bool again = true;
+  for (;;) {
+    if (again) {
+      own = 0;
+      float least2 = 0.f;  // |X|^2 below which no bin is listed
+      // 32 lanes look at 64 bins, the inner 62 of which are this step's candidates
+      for (uint32_t base = ((a.start - 1) >> 1) + 31 * warp; 2 * base + 1 < a.end; base += 31 * W) {
+        const uint32_t j = base + lane, k0 = 2 * j;
+        float c0 = 0.f, c1 = 0.f;
+        if (k0 <= a.end) {
+          if constexpr (M == 8192) {
+            const float4 x = s4[j];
+            c0 = mag2_rn(make_float2(x.x, x.y));
+            c1 = mag2_rn(make_float2(x.z, x.w));
+          } else {
+            const float4 x = s4[ps(j)];
+            c0 = mag2_rn(make_float2(x.x, x.z));
+            c1 = mag2_rn(make_float2(x.y, x.w));
+          }
+        }
+        const float l = __shfl_up_sync(0xffffffffu, c1, 1), r = __shfl_down_sync(0xffffffffu, c0, 1);
+        const bool p0 = lane != 0 && c0 > l && c0 > c1 && k0 >= a.start && k0 < a.end;
+        const bool p1 = lane != 31 && c1 > c0 && c1 > r && k0 + 1 >= a.start && k0 + 1 < a.end;
+        const float c = p0 ? c0 : c1, n = p0 ? fmaxf(l, c1) : fmaxf(c0, r);
+        uint32_t want = __ballot_sync(0xffffffffu, (p0 || p1) && c >= least2);
+        if (!want) continue;
+        const float cm = __fsqrt_rn(c);
+        const uint64_t key = ((uint64_t)__float_as_uint(cm) << 32) | (uint32_t)(~(p0 ? k0 : k0 + 1));
+        uint64_t least = __shfl_sync(0xffffffffu, own, R - 1);
+        least = least > floor ? least : floor;
+        want &= __ballot_sync(0xffffffffu, cm > __fsqrt_rn(n) && key > least);
+        // more than the list holds: the R largest (equal ones from the lowest bin), else all
+        for (uint32_t left = min((uint32_t)__popc(want), R), sift = __popc(want) > R; left; --left) {
+          uint32_t at = want;
+          if (sift) {
+            const uint32_t bits = (want >> lane) & 1 ? __float_as_uint(cm) : 0;
+            at &= __ballot_sync(0xffffffffu, bits == __reduce_max_sync(0xffffffffu, bits));
+          }
+          const int src = __ffs(at) - 1;
+          want &= ~(1u << src);
+          own = warp_list_insert(own, __shfl_sync(0xffffffffu, key, src), lane);
+        }
+        least = __shfl_sync(0xffffffffu, own, R - 1);
+        const float m = __uint_as_float((uint32_t)((least > floor ? least : floor) >> 32));
+        least2 = 0.999999f * (m * m);
+      }
+    }
+    mine = merge_warp_lists(lists, own, W, a.K, warp, lane);
+    if (R == a.K) break;
+    __syncthreads();
+    const uint64_t kth = lists[a.K - 1];
+    again = __shfl_sync(0xffffffffu, own, R - 1) > kth;
+    if (!__syncthreads_or(again)) break;
+    R = a.K;
+    floor = kth ? kth - 1 : 0;
+  }
+  if (warp != 0) return;
+  const uint32_t cnt = __popc(__ballot_sync(0xffffffffu, lane < a.K && mine != 0));
+  if (lane == 0) a.counts[beam] = cnt;
+  if (lane < cnt) {
+    const uint32_t k = ~(uint32_t)mine;
+    const size_t at = (size_t)beam * a.K + lane;
+    a.out[at] = fused_max(k, bin(k), mag_rn(bin(k - 1)), __uint_as_float((uint32_t)(mine >> 32)), mag_rn(bin(k + 1)),
+                          __fdiv_rn(a.fs, (float)g.nfft), a.refine);
+    if (ctx && k >= 2 && k + 2 < g.nfft)
+      for (uint32_t d = 0; d < 5; ++d) ctx[at * 5 + d] = bin(k + d - 2);
+  }
+}
+
+bool topk_pair_supported(const FftPlan& plan) { return plan.d_tw_pair && plan.g.C == 1 && plan.g.ept == 16; }
+
+spx_status launch_topk_pair(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams, uint32_t n_point,
+                            const float* d_win, uint32_t start, uint32_t end, uint32_t k, float fs, uint32_t refine,
+                            spx_max_value* d_out, uint32_t* d_counts, float2* d_ctx) {
+  if (beams == 0) return SPX_OK;
+  FftGeom g = plan.g;
+  FusedArgs a{};
+  a.in = d_in;
+  a.win = d_win;
+  a.tw_local = plan.d_tw_local;
+  a.tw_pair = plan.d_tw_pair;
+  a.out = reinterpret_cast<MaxValueDev*>(d_out);
+  a.counts = d_counts;
+  a.n_point = n_point;
+  a.start = start < end ? start : end;
+  a.end = end;
+  a.K = k;
+  a.refine = refine;
+  a.fs = fs;
+  const void* kfn = g.M == 1024   ? (const void*)fft_topk_pair_kernel<1024>
+                    : g.M == 2048 ? (const void*)fft_topk_pair_kernel<2048>
+                    : g.M == 4096 ? (const void*)fft_topk_pair_kernel<4096>
+                    : g.M == 8192 ? (const void*)fft_topk_pair_kernel<8192>
+                                  : (const void*)fft_topk_pair_kernel<16384>;
+  const uint32_t T = g.M / 32;
+  const size_t smem = ps_len(g.M) * sizeof(float4) + T * sizeof(uint64_t);
+  cudaError_t e = configure_kernel(kfn, smem);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "configure fft_topk_pair_kernel");
+  g.beams = beams;
+  g.ahead = ctx->input_on_host ? 0u : resident_ctas(kfn, T, smem, 1);
+  void* args[] = {(void*)&g, (void*)&a, (void*)&d_ctx};
+  e = cudaLaunchKernel(kfn, dim3(beams), dim3(T), args, smem, ctx->stream);
+  return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch fft_topk_pair_kernel");
+}
+
 // Self-test of the bounded wait: a single CTA arrives at a barrier that
 // expects two arrivals, so the wait ends at its time bound.
 __global__ void group_timeout_probe_kernel(uint32_t* count, uint32_t* err) { group_barrier(count, 2u, err); }

@@ -266,6 +266,18 @@ mlp_tile_kernel(TileArgs a) {
   }
 }
 
+// Parameter i's place in the staged weights (MlpWeights: the layers' matrices as
+// FP32 of their BF16 rounding, the hidden ones transposed), and its value there.
+SPX_DEV void stage_param(MlpWeights* w, uint32_t i, float p, __nv_bfloat16 pb) {
+  const float v = __bfloat162float(pb);
+  if (i < kOffB1) w->w1t[(i % kIn) * kH + i / kIn] = v;
+  else if (i < kOffW2) w->b1[i - kOffB1] = p;
+  else if (i < kOffB2) w->w2t[((i - kOffW2) % kH) * kH + (i - kOffW2) / kH] = v;
+  else if (i < kOffW3) w->b2[i - kOffB2] = p;
+  else if (i < kOffB3) w->w3[i - kOffW3] = v;
+  else w->b3[i - kOffB3] = p;
+}
+
 // The partial sums of `parts` CTAs added in a fixed order: 32 parameters per
 // CTA, eight threads each.  The last "parameter" is the loss (added to *loss).
 // grad != null takes the gradient; else one Adam step of the FP32 masters
@@ -273,6 +285,7 @@ mlp_tile_kernel(TileArgs a) {
 struct AdamArgs {
   float *p, *m, *v;
   __nv_bfloat16* pb;
+  MlpWeights* staged;
   float lr, b1, b2, eps, c1, c2;
 };
 __global__ void __launch_bounds__(256)
@@ -303,12 +316,18 @@ mlp_reduce_kernel(const float* __restrict__ part, uint32_t parts, float* __restr
   ad.v[i] = vi;
   const float pi = ad.p[i] - ad.lr * (mi / ad.c1) / (sqrtf(vi / ad.c2) + ad.eps);
   ad.p[i] = pi;
-  ad.pb[i] = __float2bfloat16_rn(pi);
+  const __nv_bfloat16 b = __float2bfloat16_rn(pi);
+  ad.pb[i] = b;
+  stage_param(ad.staged, i, pi, b);
 }
 
-__global__ void to_bf16_kernel(const float* __restrict__ p, __nv_bfloat16* __restrict__ pb, uint32_t n) {
+__global__ void to_bf16_kernel(const float* __restrict__ p, __nv_bfloat16* __restrict__ pb, MlpWeights* __restrict__ w,
+                               uint32_t n) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) pb[i] = __float2bfloat16_rn(p[i]);
+  if (i >= n) return;
+  const __nv_bfloat16 b = __float2bfloat16_rn(p[i]);
+  pb[i] = b;
+  stage_param(w, i, p[i], b);
 }
 
 // ---- features -------------------------------------------------------------------
@@ -431,15 +450,31 @@ struct RefineSmem {
   float x[kRefineWarps][kIn];
 };
 
+// Bins around the peak at bin k, kept as k - 2 .. k + 2.
+struct CtxBins {
+  const float2* c;
+  uint32_t k;
+  SPX_DEV float2 operator()(uint32_t b) const { return c[b + 2 - k]; }
+};
+
+// CTX: `fft` holds each peak's five bins instead of the spectra, and the launch
+// may begin before the search that writes them has ended (its CTAs that find room
+// beside the search's last wave stage the weights meanwhile).
+template <bool CTX>
 __global__ void __launch_bounds__(kRefineWarps * 32)
-mlp_refine_kernel(const __nv_bfloat16* __restrict__ pb, const float* __restrict__ p,
-                  const float2* __restrict__ fft, uint32_t n_point, uint32_t nfft, uint32_t beams,
-                  uint32_t K, float fs, MaxValueDev* __restrict__ peaks,
+mlp_refine_kernel(const MlpWeights* __restrict__ staged, const float2* __restrict__ fft, uint32_t n_point,
+                  uint32_t nfft, uint32_t beams, uint32_t K, float fs, MaxValueDev* __restrict__ peaks,
                   const uint32_t* __restrict__ counts, float* __restrict__ amp_out,
                   uint32_t* __restrict__ used_mlp) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RefineSmem& s = *reinterpret_cast<RefineSmem*>(smem_raw);
-  mlp_stage(s.w, pb, p, threadIdx.x, blockDim.x);
+  static_assert(sizeof(MlpWeights) % 8 == 0, "copied in pairs of floats");
+  for (uint32_t i = threadIdx.x; i < sizeof(MlpWeights) / 8; i += blockDim.x)
+    reinterpret_cast<float2*>(&s.w)[i] = __ldg(reinterpret_cast<const float2*>(staged) + i);
+  if constexpr (CTX) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("" : "+l"(fft), "+l"(counts), "+l"(peaks)::"memory");  // nothing of them is read earlier
+  }
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint64_t total = (uint64_t)beams * K;
@@ -451,7 +486,10 @@ mlp_refine_kernel(const __nv_bfloat16* __restrict__ pb, const float* __restrict_
     // the features, offset d = lane - 2 on lanes 0..4 (peak_features_at's
     // arithmetic, one offset per lane)
     const uint32_t k = mv.index;
-    const GlobalBins bins{fft + (size_t)beam * nfft};
+    const auto bins = [&] {
+      if constexpr (CTX) return CtxBins{fft + idx * 5, k};
+      else return GlobalBins{fft + (size_t)beam * nfft};
+    }();
     bool good = k >= 2 && k + 2 < nfft;
     float2 c = make_float2(0.f, 0.f);
     float mc = 0.f;
@@ -489,6 +527,7 @@ struct spx_mlp {
   float* d_m = nullptr;           // Adam first moment
   float* d_v = nullptr;           // Adam second moment
   __nv_bfloat16* d_pb = nullptr;  // BF16 copy read by every product
+  MlpWeights* d_staged = nullptr; // the weights as the refine kernel stages them
   float* d_work = nullptr;        // partial sums of the gradients
   size_t work_floats = 0;
   uint64_t step = 0;              // Adam step count
@@ -546,7 +585,7 @@ spx_status backward(spx_ctx* ctx, spx_mlp* m, const TileArgs& a, float* d_loss, 
   AdamArgs ad{};
   if (!d_grad) {
     m->step += 1;
-    ad = AdamArgs{m->d_p, m->d_m, m->d_v, m->d_pb, lr, 0.9f, 0.999f, 1e-8f,
+    ad = AdamArgs{m->d_p, m->d_m, m->d_v, m->d_pb, m->d_staged, lr, 0.9f, 0.999f, 1e-8f,
                   1.f - (float)std::pow(0.9, (double)m->step), 1.f - (float)std::pow(0.999, (double)m->step)};
   }
   mlp_reduce_kernel<<<nblocks(kNParams + 1, 32), 256, 0, ctx->stream>>>(m->d_work, tile_ctas(a.rows), d_grad, d_loss, ad);
@@ -559,7 +598,40 @@ spx_status launch_status(spx_ctx* ctx, const char* what) {
   return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, what);
 }
 
+template <bool CTX>
+spx_status launch_refine(spx_ctx* ctx, const spx_mlp* m, const float2* d_bins, uint32_t beams, uint32_t n_point,
+                         uint32_t nfft, float fs, uint32_t K, spx_max_value* d_peaks, const uint32_t* d_counts,
+                         float* d_amplitude, uint32_t* d_used) {
+  const size_t smem = sizeof(RefineSmem);
+  cudaError_t e = configure_kernel((const void*)mlp_refine_kernel<CTX>, smem);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "spx_mlp_refine: configure");
+  const uint64_t warps = (uint64_t)beams * K;
+  const unsigned grid = (unsigned)std::min<uint64_t>((warps + kRefineWarps - 1) / kRefineWarps,
+                                                     (uint64_t)ctx->sm_count * 8);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kRefineWarps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ctx->stream;
+  cudaLaunchAttribute overlap[1];
+  overlap[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = overlap;
+  cfg.numAttrs = CTX ? 1 : 0;
+  e = cudaLaunchKernelEx(&cfg, mlp_refine_kernel<CTX>, (const MlpWeights*)m->d_staged, d_bins, n_point, nfft, beams, K,
+                         fs, reinterpret_cast<MaxValueDev*>(d_peaks), d_counts, d_amplitude, d_used);
+  return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "spx_mlp_refine");
+}
+
 }  // namespace
+
+namespace spx {
+spx_status launch_mlp_refine_ctx(spx_ctx* ctx, const spx_mlp* m, const float2* d_ctx, uint32_t beams,
+                                 uint32_t n_point, uint32_t nfft, float fs, uint32_t K, spx_max_value* d_peaks,
+                                 const uint32_t* d_counts, float* d_amplitude, uint32_t* d_used) {
+  return launch_refine<true>(ctx, m, d_ctx, beams, n_point, nfft, fs, K, d_peaks, d_counts, d_amplitude, d_used);
+}
+}  // namespace spx
 
 extern "C" {
 
@@ -577,6 +649,7 @@ spx_status spx_mlp_create(spx_ctx* ctx, uint64_t seed, spx_mlp** out) {
   for (float** b : bufs)
     if (e == cudaSuccess) e = cudaMalloc(b, kNParams * sizeof(float));
   if (e == cudaSuccess) e = cudaMalloc(&m->d_pb, kNParams * sizeof(__nv_bfloat16));
+  if (e == cudaSuccess) e = cudaMalloc(&m->d_staged, sizeof(MlpWeights));
   if (e != cudaSuccess) {
     spx_mlp_destroy(m);
     return cuda_fail(ctx, e, "cudaMalloc(mlp parameters)");
@@ -607,6 +680,7 @@ spx_status spx_mlp_destroy(spx_mlp* m) {
   cudaFree(m->d_m);
   cudaFree(m->d_v);
   cudaFree(m->d_pb);
+  cudaFree(m->d_staged);
   cudaFree(m->d_work);
   delete m;
   return SPX_OK;
@@ -620,7 +694,7 @@ spx_status spx_mlp_set_params(spx_ctx* ctx, spx_mlp* m, const float* host_params
   if (e == cudaSuccess) e = cudaMemset(m->d_m, 0, kNParams * sizeof(float));
   if (e == cudaSuccess) e = cudaMemset(m->d_v, 0, kNParams * sizeof(float));
   if (e != cudaSuccess) return cuda_fail(ctx, e, "spx_mlp_set_params");
-  to_bf16_kernel<<<nblocks(kNParams, 256), 256, 0, ctx->stream>>>(m->d_p, m->d_pb, kNParams);
+  to_bf16_kernel<<<nblocks(kNParams, 256), 256, 0, ctx->stream>>>(m->d_p, m->d_pb, m->d_staged, kNParams);
   m->step = 0;
   e = cudaStreamSynchronize(ctx->stream);
   return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "spx_mlp_set_params");
@@ -789,16 +863,8 @@ spx_status spx_mlp_refine(spx_ctx* ctx, spx_mlp* m, const void* d_fft, uint32_t 
   if (nfft < 5 || n_point == 0 || n_point > nfft)
     return fail(ctx, SPX_ERR_INVALID_ARG, "spx_mlp_refine: need 5 <= nfft and 0 < n_point <= nfft");
   DeviceGuard guard(ctx->device);
-  const size_t smem = sizeof(RefineSmem);
-  cudaError_t e = cudaFuncSetAttribute(mlp_refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "spx_mlp_refine: configure");
-  const uint64_t warps = (uint64_t)beams * K;
-  const unsigned grid = (unsigned)std::min<uint64_t>((warps + kRefineWarps - 1) / kRefineWarps,
-                                                     (uint64_t)ctx->sm_count * 8);
-  mlp_refine_kernel<<<grid, kRefineWarps * 32, smem, ctx->stream>>>(
-      m->d_pb, m->d_p, static_cast<const float2*>(d_fft), n_point, nfft, beams, K, sample_rate,
-      reinterpret_cast<MaxValueDev*>(d_peaks), d_counts, d_amplitude, d_used_mlp);
-  return launch_status(ctx, "spx_mlp_refine");
+  return launch_refine<false>(ctx, m, static_cast<const float2*>(d_fft), beams, n_point, nfft, sample_rate, K, d_peaks,
+                              d_counts, d_amplitude, d_used_mlp);
 }
 
 }  // extern "C"

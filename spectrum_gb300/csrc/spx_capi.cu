@@ -452,8 +452,9 @@ spx_status spx_fft_peaks_mlp(spx_ctx* ctx, spx_mlp* mlp, const void* d_in, uint3
   const uint32_t K = params->max_per_beam;
   // One launch while the call is small (at most 2^21 points): each CTA then
   // also stages the network's weights and refines its peaks with one warp,
-  // which pays while launch latency dominates; measured on GB300, 4096 x 8192
-  // top-1 took 0.295 ms in one launch against 0.246 ms in three.
+  // which pays while launch latency dominates; measured on GB300, top-1 and
+  // top-8 of 1 .. 256 beams of 4096 .. 16384 points took 37 .. 42 us per call in
+  // one launch and 40 .. 45 us in two; 4096 x 8192 top-1 290 us against 165.
   const bool one_launch_pays = (uint64_t)beams * nfft <= (1ull << 21);
   if (!plan->big && !plan->bluestein && !plan->huge && one_launch_pays && fused_mlp_supported(plan->g, K)) {
     uint32_t start = params->search_start, end = params->search_end;
@@ -466,6 +467,23 @@ spx_status spx_fft_peaks_mlp(spx_ctx* ctx, spx_mlp* mlp, const void* d_in, uint3
     return launch_fft_peaks(ctx, *plan, static_cast<const float2*>(d_in), beams, n_point, win, SPX_PEAK_TOPK,
                             start, end, K, params->sample_rate, params->refine,
                             thr ? spx_noise_threshold_factor(params->thresh_sigma) : 0.0f, d_out, d_counts, &m);
+  }
+  if (params->thresh_sigma == 0.0f && topk_pair_supported(*plan)) {
+    // larger calls of power-of-two beams up to 16384 points: the search keeps the
+    // spectrum on chip and hands on the five bins of each peak (4096 x 8192 top-1:
+    // 165 us, and 187 us through the spectrum in device memory)
+    uint32_t start = params->search_start, end = params->search_end;
+    resolve_window(nfft, &start, &end);
+    const float* win = nullptr;
+    st = get_window(ctx, window, n_point, &win);
+    void* bins = nullptr;
+    if (st == SPX_OK) st = get_scratch(ctx, kSlotWork, (size_t)beams * K * 5 * sizeof(float2), &bins);
+    if (st == SPX_OK)
+      st = launch_topk_pair(ctx, *plan, static_cast<const float2*>(d_in), beams, n_point, win, start, end, K,
+                            params->sample_rate, params->refine, d_out, d_counts, static_cast<float2*>(bins));
+    if (st != SPX_OK) return st;
+    return launch_mlp_refine_ctx(ctx, mlp, static_cast<const float2*>(bins), beams, n_point, nfft,
+                                 params->sample_rate, K, d_out, d_counts, d_amplitude, d_used_mlp);
   }
   // other sizes: the spectrum in device memory, the search, then the refinement
   void* spec = nullptr;
@@ -518,6 +536,18 @@ spx_status spx_fft_peaks(spx_ctx* ctx, const void* d_in, uint32_t beams, uint32_
       cap = params->max_per_beam;
     }
     const bool thr = params->thresh_sigma > 0.0f;
+    // Top-K of power-of-two beams up to 16384 points without a threshold: one
+    // launch of the packed kernel, faster than the scalar fused kernel and than
+    // the composed path at every size measured (1 .. 4096 beams of 1024 .. 16384
+    // points, K = 1, 8, 32; e.g. 4096 x 8192 top-1: 141 us against 220, 4096 x
+    // 16384 top-32: 409 against 528).
+    if (!all && !thr && topk_pair_supported(*plan)) {
+      const float* win = nullptr;
+      st = get_window(ctx, window, n_point, &win);
+      if (st != SPX_OK) return st;
+      return launch_topk_pair(ctx, *plan, static_cast<const float2*>(d_in), beams, n_point, win, start, end, cap,
+                              params->sample_rate, params->refine, d_out, d_counts, nullptr);
+    }
     // nfft <= 16384 (one CTA per beam): the fused kernel keeps the spectrum
     // on chip, but its search phase holds the SM from the next beam's
     // transform, which pays only while the launch is short.  Measured on

@@ -254,7 +254,9 @@ SPX_DEV uint64_t warp_list_insert(uint64_t mine, uint64_t x, uint32_t lane) {
 
 // Merges the lists of the CTA's nw warps into warp 0's, pairwise in
 // log2(nw) rounds (round s: warp w, a multiple of 2s, takes the list of warp
-// w + s): K log2(nw) insertions on the critical path instead of K (nw - 1).
+// w + s).  Up to four entries are inserted one by one; longer lists as one
+// bitonic step (the larger of entry i and the other list's entry 31 - i are the
+// 32 largest of both) and five exchanges that sort it, whatever K is.
 // The top K of a union does not depend on the order of the merges, so the
 // result is the serial merge's.  lists: nw x 32 words of shared memory, free
 // on entry; every thread of the CTA calls it; warp 0 gets the merged entry.
@@ -264,10 +266,20 @@ SPX_DEV uint64_t merge_warp_lists(uint64_t* lists, uint64_t mine, uint32_t nw, u
   for (uint32_t step = 1; step < nw; step *= 2) {
     __syncthreads();
     if (warp % (2 * step) == 0 && warp + step < nw) {
-      for (uint32_t e = 0; e < K; ++e) {
-        const uint64_t x = lists[(warp + step) * 32 + e];
-        if (x == 0) break;
-        mine = warp_list_insert(mine, x, lane);
+      if (K > 4) {
+        const uint64_t x = lists[(warp + step) * 32 + 31 - lane];
+        mine = mine > x ? mine : x;
+#pragma unroll
+        for (uint32_t o = 16; o > 0; o >>= 1) {
+          const uint64_t y = __shfl_xor_sync(0xffffffffu, mine, o);
+          mine = ((lane & o) != 0) == (mine > y) ? y : mine;
+        }
+      } else {
+        for (uint32_t e = 0; e < K; ++e) {
+          const uint64_t x = lists[(warp + step) * 32 + e];
+          if (x == 0) break;
+          mine = warp_list_insert(mine, x, lane);
+        }
       }
       lists[warp * 32 + lane] = mine;
     }

@@ -164,6 +164,19 @@ spx_status launch_fft_peaks(spx_ctx* ctx, const FftPlan& plan, const float2* d_i
                             uint32_t mode, uint32_t start, uint32_t end, uint32_t cap_or_k,
                             float fs, uint32_t refine, float factor, spx_max_value* d_out,
                             uint32_t* d_counts, const MlpRefineArgs* mlp = nullptr);
+// Top-K without a threshold of plans the packed single-CTA kernel takes
+// (power-of-two, 1024 .. 16384 points): one launch, the spectrum on chip; d_ctx
+// (may be null) receives bins k - 2 .. k + 2 of each peak, [beams][K][5].
+bool topk_pair_supported(const FftPlan& plan);
+spx_status launch_topk_pair(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams,
+                            uint32_t n_point, const float* d_win, uint32_t start, uint32_t end,
+                            uint32_t k, float fs, uint32_t refine, spx_max_value* d_out,
+                            uint32_t* d_counts, float2* d_ctx);
+// spx_mlp_refine on peaks whose neighbourhoods are in d_ctx (launch_topk_pair).
+spx_status launch_mlp_refine_ctx(spx_ctx* ctx, const spx_mlp* m, const float2* d_ctx, uint32_t beams,
+                                 uint32_t n_point, uint32_t nfft, float fs, uint32_t K,
+                                 spx_max_value* d_peaks, const uint32_t* d_counts, float* d_amplitude,
+                                 uint32_t* d_used);
 // The device weights of a network (mlp.cu).
 void mlp_device_params(const spx_mlp* mlp, const void** pb, const float** p, int* device);
 // Output of C spectrum rows per beam (rows[beam][k1][q] = X[k1 + C*q], the

@@ -229,10 +229,10 @@ class MLPRefiner:
         _require_cuda(x, torch.complex64, "x")
         x2 = x.reshape(-1, x.shape[-1])
         beams, n_point = x2.shape
-        out = _zeros((beams, k, 8), torch.int32, x.device)
         counts = torch.empty((beams,), dtype=torch.int32, device=x.device)  # written by the search
-        amp = _zeros((beams, k), torch.float32, x.device)
-        used = _zeros((beams, k), torch.int32, x.device)
+        n = beams * k  # the others cleared in one piece (one launch instead of three)
+        out, amp, used = _zeros((10 * n,), torch.int32, x.device).split((8 * n, n, n))
+        out, amp, used = out.view(beams, k, 8), amp.view(torch.float32).view(beams, k), used.view(beams, k)
         p = _capi.peak_params(PEAK_TOPK, search_start, search_end, 0, k, refine, sample_rate, thresh_sigma)
         self.ctx.bind_stream()
         self.ctx.check(lib.spx_fft_peaks_mlp(self.ctx.h, self.h, _ptr(x2), beams, n_point, int(nfft), int(window),

@@ -129,3 +129,41 @@ def test_chirp_z_in_one_launch_equals_the_launches(spx, nfft):
     for full in (False, True):
         assert _same(spx.fft_r2c(r, nfft, spx.WINDOW_HANN, full),
                      spx.fft_r2c(r, nfft, spx.WINDOW_HANN, full, ctx=general))
+
+
+def _hard_beams(x):
+    """Beams without a maximum, with ties, NaN, infinities and magnitudes whose squares leave FP32."""
+    x[0] = 0
+    x[1] = 1
+    x[2, 0] = complex(float("nan"), 1.0)
+    x[3, -1] = complex(float("inf"), 0.0)
+    x[4] *= 1e25
+    x[5] *= 1e-25
+    x[6, x.shape[1] // 2:] = x[6, :x.shape[1] - x.shape[1] // 2].clone()
+    return x
+
+
+@pytest.mark.parametrize("nfft", [1024, 2048, 4096, 8192, 16384])
+def test_topk_equals_the_scalar_kernels(spx, scalar, nfft):
+    import torch
+    for n, offset, k, lo, hi in ((nfft, 0, 1, 0, 0), (nfft - 1, 0, 8, 1, nfft), (nfft, 1, 32, 2, nfft - 1),
+                                 (nfft // 2, 0, 7, nfft // 2 - 33, nfft // 2 + 33), (nfft, 0, 9, 5, 6), (3, 0, 32, 0, 0),
+                                 (nfft, 0, 4, nfft - 2, nfft - 1), (nfft, 0, 4, 9, 9)):
+        x = _hard_beams(_samples(9, n, offset, nfft + n + k))
+        a, b = (spx.fft_peaks(x, nfft, spx.WINDOW_HANN, spx.PEAK_TOPK, 1e6, lo, hi, max_per_beam=k, refine=1, ctx=c)
+                for c in (None, scalar))
+        assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1]), (nfft, n, k, lo, hi)
+
+
+@pytest.mark.parametrize("nfft,beams,k", [(1024, 2050, 3), (2048, 1030, 32), (4096, 520, 1), (8192, 300, 8), (16384, 130, 2)])
+def test_learned_topk_equals_its_three_steps(spx, nfft, beams, k):
+    import torch
+    from spectrum_gb300.learned import MLPRefiner
+    net = MLPRefiner(seed=5)
+    x = _hard_beams(_samples(beams, nfft, 0, nfft))
+    out, counts, amp, used = net.fft_peaks(x, nfft, spx.WINDOW_HANN, k, 1e6, search_start=1, search_end=nfft)
+    spec = spx.fft(x, nfft, spx.WINDOW_HANN)
+    ref, n = spx.topk(spec, k, sample_rate=1e6, search_start=1, search_end=nfft, refine=1)
+    ramp, rused = net.refine(spec, ref, n, nfft, 1e6)
+    for a, b in ((out, ref), (counts, n), (amp.view(torch.int32), ramp.view(torch.int32)), (used, rused)):
+        assert torch.equal(a, b)
