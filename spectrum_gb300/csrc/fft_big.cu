@@ -60,6 +60,7 @@ big_cols_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __
   constexpr uint32_t HP = W / 2, T = HP * G;
   const uint32_t tid = threadIdx.x, p = tid % HP, t = tid / HP;
   const uint32_t beam = blockIdx.y, c0 = blockIdx.x * W;
+  let_next_launch_begin();
   {  // L2 prefetch of the tile of the CTA `ahead` places later
     const uint64_t f = (uint64_t)blockIdx.y * gridDim.x + blockIdx.x + ahead;
     if (ahead && f < (uint64_t)gridDim.x * gridDim.y) {
@@ -135,13 +136,14 @@ constexpr int kBigComplex = 0, kBigMag = 1, kBigMagPhase = 2, kBigOther = 3;
 
 template <int MODE>
 __global__ void __launch_bounds__(kRows4 * 128, 1)
-big_rows4_kernel(FftGeom g, const float4* __restrict__ tw_pair, const float2* __restrict__ scratch,
+big_rows4_kernel(FftGeom g, const float4* __restrict__ tw_pair, const float2* cols,
                  void* __restrict__ out, uint32_t out_mode, float scale) {
   extern __shared__ float4 s4[];
   constexpr int TG = 128, M = (int)kBigM4;
   const uint32_t tid = threadIdx.x, grp = tid / TG;
   const uint32_t per_beam = g.C / kRows4;
   const uint32_t beam = blockIdx.x / per_beam, r0 = (blockIdx.x - beam * per_beam) * kRows4;
+  const float2* scratch = wait_for_launch_before(cols);
   const float2* row = scratch + (size_t)beam * g.nfft + (size_t)(r0 + grp) * kBigM4;
   // the four rows of the CTA one residency wave later follow this CTA's
   // (CTA b holds elements [b, b + 1) x kRows4 x kBigM4 of the scratch)
@@ -264,7 +266,7 @@ spx_status launch_fft_big(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
     gg.ahead = ctx->input_on_host ? 0u : resident_ctas(kfn, kRows4 * 128, smem, 1);
     const float2* scr_c = scratch;
     void* args[] = {(void*)&gg, (void*)&twp, (void*)&scr_c, (void*)&d_out, (void*)&out_mode, (void*)&scale};
-    e = cudaLaunchKernel(kfn, dim3(beams * (g.C / kRows4)), dim3(kRows4 * 128), args, smem, ctx->stream);
+    e = launch_dependent(kfn, dim3(beams * (g.C / kRows4)), dim3(kRows4 * 128), args, smem, ctx->stream);
     return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch big_rows4_kernel");
   }
   const void* kfn = (const void*)big_rows_kernel;

@@ -339,6 +339,17 @@ SPX_DEV void prefetch_beam_part(const float2* x, uint32_t n_point, uint32_t C, u
   }
 }
 
+// The two ends of launch_dependent: the earlier kernel lets the next one begin
+// (its CTAs become resident once every CTA here has started), the later one waits
+// for the earlier one's results.  p passes through the wait, so that nothing is
+// read through it earlier.
+SPX_DEV void let_next_launch_begin() { asm volatile("griddepcontrol.launch_dependents;"); }
+template <typename T>
+SPX_DEV T* wait_for_launch_before(T* p) {
+  asm volatile("griddepcontrol.wait;" : "+l"(p) : : "memory");
+  return p;
+}
+
 SPX_DEV void prefetch_future_beam(const FftGeom& g, const float2* in, uint32_t n_point, uint32_t beam,
                                   uint32_t c, uint32_t tid, uint32_t T) {
   if (g.ahead == 0 || beam + g.ahead >= g.beams) return;

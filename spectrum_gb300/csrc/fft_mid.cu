@@ -73,6 +73,7 @@ mid_cols_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __
   constexpr uint32_t W = kMidCols<C>, HP = W / 2, G = kMidGroups<C>, U = 16 / G, nfft = C * kMidLocal;
   const uint32_t tid = threadIdx.x, p = tid % HP, g = tid / HP;
   const uint32_t beam = blockIdx.x / (kMidRow / W), c0 = (blockIdx.x - beam * (kMidRow / W)) * W;
+  let_next_launch_begin();
   if (ahead && blockIdx.x + ahead < gridDim.x) {  // L2 prefetch of the tile one residency wave later
     const uint32_t f = blockIdx.x + ahead, fb = f / (kMidRow / W), fc = (f - fb * (kMidRow / W)) * W;
     for (uint32_t r = tid; r < 16 * C; r += HP * G) {
@@ -204,7 +205,9 @@ SPX_DEV void mid_row_fft(float4* s, const float2* row, const float4* __restrict_
 // Beams in descending order (the rows written last by launch 1 may still be
 // in L2), and the L2 prefetch of the rows (contiguous) of the CTA one
 // residency wave later.
-SPX_DEV uint32_t mid_rows_block(const MidRowsArgs& a) {
+SPX_DEV uint32_t mid_rows_block(MidRowsArgs& a) {
+  let_next_launch_begin();
+  a.scratch = wait_for_launch_before(a.scratch);
   const uint32_t bx = gridDim.x - 1 - blockIdx.x;
   if (a.g.ahead && bx >= a.g.ahead && threadIdx.x < kMidRows / 2)
     prefetch_l2(a.scratch + ((size_t)(bx - a.g.ahead) * kMidRows + threadIdx.x * 2) * kMidRow,
@@ -343,7 +346,7 @@ static spx_status launch_mid(spx_ctx* ctx, const FftPlan& plan, const float2* d_
   a.tw = plan.d_tw_rows;
   a.scratch = scratch;
   void* args[] = {(void*)&a};
-  e = cudaLaunchKernel(kfn, dim3(beams * (16 * plan.g.C / kMidRows)), dim3(32 * kMidRows), args, smem, ctx->stream);
+  e = launch_dependent(kfn, dim3(beams * (16 * plan.g.C / kMidRows)), dim3(32 * kMidRows), args, smem, ctx->stream);
   return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch mid_rows_kernel");
 }
 

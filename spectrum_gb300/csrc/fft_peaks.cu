@@ -491,7 +491,7 @@ fft_topk_pair_kernel(FftGeom g, FusedArgs a, float2* __restrict__ ctx) {
     pair8k_fft_out(s4, ld, a.tw_local, tid, Natural8kOut{reinterpret_cast<float2*>(s4), a.end + 2});
   else
     pair_local_fft_out<M>(s4, ld, a.tw_pair, tid, SlotOutUpTo{s4, a.end + 2});
-  asm volatile("griddepcontrol.launch_dependents;");
+  let_next_launch_begin();
   __syncthreads();
   auto bin = [&](uint32_t k) {
     if constexpr (M == 8192) return reinterpret_cast<const float2*>(s4)[k];
@@ -724,7 +724,6 @@ maxima_cluster_kernel(MxArgs a) {
       return smag[i + 1];
     }
   };
-  const float2* sb = a.spec + (size_t)beam * a.nfft;
   if (thr_on) {
     for (uint32_t b = tid; b < (ROWS ? kHist : kHist / 2); b += kMxThreads) hist[b] = 0;
     if (tid == 0) {
@@ -733,6 +732,7 @@ maxima_cluster_kernel(MxArgs a) {
     }
     __syncthreads();
   }
+  const float2* sb = wait_for_launch_before(a.spec) + (size_t)beam * a.nfft;
   // 1. (loads issued kMxBatch at a time per thread, so that enough bytes
   //    are in flight to cover the device-memory latency)
   uint32_t bmin = kHist, bmax = 0;
@@ -1048,7 +1048,7 @@ bool fused_supported(const FftGeom& g, uint32_t mode) {
 spx_status launch_maxima_cluster(spx_ctx* ctx, const float2* d_spec, uint32_t C1, uint32_t M1,
                                  uint32_t beams, uint32_t nfft, uint32_t start, uint32_t end,
                                  uint32_t cap, float fs, uint32_t refine, float factor,
-                                 uint32_t* d_ccount, spx_max_value* d_out, uint32_t* d_counts) {
+                                 uint32_t* d_ccount, spx_max_value* d_out, uint32_t* d_counts, bool after_rows) {
   if (beams == 0) return SPX_OK;
   uint32_t C2 = 1, chunk = 32;
   if (!mx_geometry(end > start ? end - start : 0u, &C2, &chunk))
@@ -1088,13 +1088,15 @@ spx_status launch_maxima_cluster(spx_ctx* ctx, const float2* d_spec, uint32_t C1
   cfg.blockDim = dim3(kMxThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = ctx->stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = C2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_dependent
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = after_rows ? 2 : 1;
   void* args[] = {(void*)&a};
   e = cudaLaunchKernelExC(&cfg, kfn, args);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "launch maxima_cluster_kernel");
@@ -1158,7 +1160,7 @@ spx_status launch_fft_peaks(spx_ctx* ctx, const FftPlan& plan, const float2* d_i
     if (st == SPX_OK) st = launch_fft_mid(ctx, plan, d_in, beams, n_point, d_win, SPX_OUT_COMPLEX, 1.0f, spec);
     if (st != SPX_OK) return st;
     return launch_maxima_cluster(ctx, static_cast<float2*>(spec), 1, g.nfft, beams, g.nfft, start, end, cap_or_k, fs,
-                                 refine, factor, static_cast<uint32_t*>(cnt), d_out, d_counts);
+                                 refine, factor, static_cast<uint32_t*>(cnt), d_out, d_counts, true);
   }
   if (plan.d_tw_rows) {  // spectrum rows over the exchange scratch, then the maxima kernel
     const size_t row_bytes = (size_t)beams * g.nfft * sizeof(float2);
@@ -1170,7 +1172,7 @@ spx_status launch_fft_peaks(spx_ctx* ctx, const FftPlan& plan, const float2* d_i
     if (st != SPX_OK) return st;
     return launch_maxima_cluster(ctx, rows, 16 * g.C, g.nfft / (16 * g.C), beams, g.nfft, start, end, cap_or_k, fs,
                                  refine, factor, reinterpret_cast<uint32_t*>(static_cast<char*>(p) + row_bytes),
-                                 d_out, d_counts);
+                                 d_out, d_counts, true);
   }
   // C > 1: scratch = exchange slots | per-CTA maxima counts | group-barrier arrivals
   const size_t xch_bytes = ((size_t)beams * g.nfft * sizeof(float2) + 255) & ~(size_t)255;

@@ -123,6 +123,25 @@ spx_status launch_fft_big(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
                           uint32_t n_point, const float* d_win, uint32_t out_mode, float scale,
                           void* d_out);
 
+// A launch that may begin while the kernel before it in the stream still runs: its
+// CTAs take the room that the other's last wave leaves, and wait for its results
+// (wait_for_launch_before in fft_core.cuh, ahead of any access to them) after their
+// own prologue.  Saves the drain and start between two launches.
+inline cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, void** args, size_t smem,
+                                    cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute overlap[1];
+  overlap[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  overlap[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = overlap;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, kernel, args);
+}
+
 // Two-launch transforms of 32768 .. 262144 = C x 16384 points (fft_mid.cu).
 // The rows form leaves the spectrum in d_rows [beams][16 C][1024]: bin
 // rho + 16 C q is element q of row rho, defined for bins [klo, khi).
@@ -196,7 +215,8 @@ constexpr uint32_t kMaxClusterSpan = 8u * 32768u;
 spx_status launch_maxima_cluster(spx_ctx* ctx, const float2* d_spec, uint32_t C1, uint32_t M1,
                                  uint32_t beams, uint32_t nfft, uint32_t start, uint32_t end,
                                  uint32_t cap, float fs, uint32_t refine, float factor,
-                                 uint32_t* d_ccount, spx_max_value* d_out, uint32_t* d_counts);
+                                 uint32_t* d_ccount, spx_max_value* d_out, uint32_t* d_counts,
+                                 bool after_rows = false);  // true: launched beside the rows kernel's end
 
 // Kernel launchers (fft_kernels.cu, peak_kernels.cu).
 spx_status launch_fft_out(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
