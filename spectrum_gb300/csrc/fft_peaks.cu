@@ -572,7 +572,41 @@ fft_topk_pair_kernel(FftGeom g, FusedArgs a, float2* __restrict__ ctx) {
   }
 }
 
+// One or two peaks of the same beams (one_two_search) in the same way.
+template <int M>
+__global__ void __launch_bounds__(M / 32, M >= 16384 ? 1 : M == 8192 ? 2 : M == 4096 ? 4 : 8)
+fft_one_two_pair_kernel(FftGeom g, FusedArgs a, uint32_t half, int two_peaks) {
+  extern __shared__ float4 s4[];
+  constexpr uint32_t T = M / 32;
+  const uint32_t tid = threadIdx.x, beam = blockIdx.x;
+  prefetch_future_beam(g, a.in, a.n_point, beam, 0, tid, T);
+  const SamplePairs ld(a.in + (size_t)beam * a.n_point, a.n_point, a.win);
+  if constexpr (M == 8192)
+    pair8k_fft_out(s4, ld, a.tw_local, tid, Natural8kOut{reinterpret_cast<float2*>(s4), 8191});
+  else
+    pair_local_fft_out<M>(s4, ld, a.tw_pair, tid, SlotOut{s4});
+  __syncthreads();
+  one_two_search<T>(
+      [&](uint32_t k) {
+        if constexpr (M == 8192) return reinterpret_cast<const float2*>(s4)[k];
+        else return pair_elem(s4, k);
+      },
+      reinterpret_cast<uint64_t*>(s4 + ps_len(M)), M, half, a.fs, two_peaks, a.out + (size_t)beam * (two_peaks ? 8 : 4));
+}
+
 bool topk_pair_supported(const FftPlan& plan) { return plan.d_tw_pair && plan.g.C == 1 && plan.g.ept == 16; }
+
+// A kernel of the two above over `beams` beams of plan geometry *g (args point at it).
+static spx_status launch_search_pair(spx_ctx* ctx, const void* kfn, FftGeom* g, uint32_t beams, void** args) {
+  const uint32_t T = g->M / 32;
+  const size_t smem = ps_len(g->M) * sizeof(float4) + T * sizeof(uint64_t);  // spectrum | lists [T / 32][32]
+  cudaError_t e = configure_kernel(kfn, smem);
+  if (e != cudaSuccess) return cuda_fail(ctx, e, "configure a search in shared memory");
+  g->beams = beams;
+  g->ahead = ctx->input_on_host ? 0u : resident_ctas(kfn, T, smem, 1);
+  e = cudaLaunchKernel(kfn, dim3(beams), dim3(T), args, smem, ctx->stream);
+  return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch a search in shared memory");
+}
 
 spx_status launch_topk_pair(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams, uint32_t n_point,
                             const float* d_win, uint32_t start, uint32_t end, uint32_t k, float fs, uint32_t refine,
@@ -597,15 +631,31 @@ spx_status launch_topk_pair(spx_ctx* ctx, const FftPlan& plan, const float2* d_i
                     : g.M == 4096 ? (const void*)fft_topk_pair_kernel<4096>
                     : g.M == 8192 ? (const void*)fft_topk_pair_kernel<8192>
                                   : (const void*)fft_topk_pair_kernel<16384>;
-  const uint32_t T = g.M / 32;
-  const size_t smem = ps_len(g.M) * sizeof(float4) + T * sizeof(uint64_t);
-  cudaError_t e = configure_kernel(kfn, smem);
-  if (e != cudaSuccess) return cuda_fail(ctx, e, "configure fft_topk_pair_kernel");
-  g.beams = beams;
-  g.ahead = ctx->input_on_host ? 0u : resident_ctas(kfn, T, smem, 1);
   void* args[] = {(void*)&g, (void*)&a, (void*)&d_ctx};
-  e = cudaLaunchKernel(kfn, dim3(beams), dim3(T), args, smem, ctx->stream);
-  return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch fft_topk_pair_kernel");
+  return launch_search_pair(ctx, kfn, &g, beams, args);
+}
+
+spx_status launch_one_two_pair(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams, uint32_t n_point,
+                               const float* d_win, uint32_t search_range, float fs, int two_peaks,
+                               spx_max_value* d_out) {
+  if (beams == 0) return SPX_OK;
+  FftGeom g = plan.g;
+  FusedArgs a{};
+  a.in = d_in;
+  a.win = d_win;
+  a.tw_local = plan.d_tw_local;
+  a.tw_pair = plan.d_tw_pair;
+  a.out = reinterpret_cast<MaxValueDev*>(d_out);
+  a.n_point = n_point;
+  a.fs = fs;
+  uint32_t half = search_range / 2;
+  const void* kfn = g.M == 1024   ? (const void*)fft_one_two_pair_kernel<1024>
+                    : g.M == 2048 ? (const void*)fft_one_two_pair_kernel<2048>
+                    : g.M == 4096 ? (const void*)fft_one_two_pair_kernel<4096>
+                    : g.M == 8192 ? (const void*)fft_one_two_pair_kernel<8192>
+                                  : (const void*)fft_one_two_pair_kernel<16384>;
+  void* args[] = {(void*)&g, (void*)&a, (void*)&half, (void*)&two_peaks};
+  return launch_search_pair(ctx, kfn, &g, beams, args);
 }
 
 // Self-test of the bounded wait: a single CTA arrives at a barrier that

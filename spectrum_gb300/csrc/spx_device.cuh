@@ -296,5 +296,121 @@ struct MaxValueDev {
 
 // Radians -> degrees with the reference's constant (fft_kernel_sources_rocm.hpp:247).
 constexpr float kRadToDeg = 57.29577951f;
+SPX_DEV float phase_deg(float2 z) { return __fmul_rn(atan2f(z.y, z.x), kRadToDeg); }
+
+// 3-point parabolic offset on magnitudes, clamped to [-0.5, 0.5], 0 when the
+// curvature is below 1e-10 (fft_kernel_sources_rocm.hpp:229-239).
+SPX_DEV bool parabolic(float yl, float yc, float yr, float* fo) {
+  const float denom = __fadd_rn(__fsub_rn(yl, __fmul_rn(2.0f, yc)), yr);
+  if (fabsf(denom) > 1e-10f) {
+    float f = __fdiv_rn(__fmul_rn(0.5f, __fsub_rn(yl, yr)), denom);
+    if (f < -0.5f) f = -0.5f;
+    if (f > 0.5f) f = 0.5f;
+    *fo = f;
+    return true;
+  }
+  *fo = 0.0f;
+  return false;
+}
+
+// ---- one peak / two peaks ------------------------------------------------------
+SPX_DEV uint64_t lane_max_u64(uint64_t v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const uint64_t w = __shfl_xor_sync(0xffffffffu, v, o);
+    v = w > v ? w : v;
+  }
+  return v;
+}
+
+// Argmax key reproducing the reference's reduction order: a range is scanned
+// by 256 threads, thread `lid` visiting offsets lid, lid+256, ... and keeping
+// its first strict maximum; the shared-memory tree then merges local[lid]
+// with local[lid + stride] for stride = 128 ... 1, keeping local[lid] on ties
+// (fft_kernel_sources_rocm.hpp:151-192).  The last merge prefers even lids,
+// the one before lid bit 1 = 0, and so on, so among equal magnitudes the
+// winner has the smallest 8-bit-reversed lid, then the smallest offset.
+// The key orders exactly that way under an unsigned max; NaN never wins (0).
+SPX_DEV uint64_t one_two_key(float mag, uint32_t t) {
+  if (!(mag >= 0.0f)) return 0ull;
+  const uint32_t rev = __brev(t & 255u) & 0xFF000000u;  // bit-reversed lid in the top byte
+  const uint32_t low = ~(rev | ((t >> 8) & 0xFFFFFFu));
+  return ((uint64_t)__float_as_uint(mag) << 32) | low;
+}
+SPX_DEV uint32_t one_two_offset(uint64_t key) {
+  const uint32_t low = ~(uint32_t)key;
+  const uint32_t lid = __brev(low & 0xFF000000u);  // undo the reversal
+  return ((low & 0xFFFFFFu) << 8) | lid;
+}
+
+// Writes the 4 MaxValue of one peak (interpolated, left, center, right)
+// exactly as post_kernel_one_peak does (fft_kernel_sources_rocm.hpp:212-286).
+template <typename Bins>
+SPX_DEV void write_peak4(const Bins& f, uint32_t nfft, uint32_t ci, float fs, bool mirror, MaxValueDev* o) {
+  const float bw = __fdiv_rn(fs, (float)nfft);
+  const float2 cv = f(ci);
+  const float yc = mag_rn(cv);
+  float2 lv = make_float2(0.f, 0.f), rv = make_float2(0.f, 0.f);
+  float yl = 0.f, yr = 0.f;
+  const bool hl = ci > 0, hr = ci < nfft - 1;
+  if (hl) { lv = f(ci - 1); yl = mag_rn(lv); }
+  if (hr) { rv = f(ci + 1); yr = mag_rn(rv); }
+  float fo = 0.f;
+  float rf = __fmul_rn((float)ci, bw);
+  if (hl && hr) {
+    if (parabolic(yl, yc, yr, &fo)) rf = __fmul_rn(__fadd_rn((float)ci, fo), bw);
+  }
+  if (mirror) rf = __fsub_rn(fs, rf);
+  const float pc = phase_deg(cv);
+  o[0] = MaxValueDev{ci, cv.x, cv.y, yc, pc, fo, rf, 0u};
+  float rfl = hl ? __fmul_rn((float)(ci - 1), bw) : 0.f;
+  if (mirror && hl) rfl = __fsub_rn(fs, rfl);
+  o[1] = MaxValueDev{hl ? ci - 1 : 0u, lv.x, lv.y, yl, hl ? phase_deg(lv) : 0.f, 0.f, rfl, 0u};
+  float rfc = __fmul_rn((float)ci, bw);
+  if (mirror) rfc = __fsub_rn(fs, rfc);
+  o[2] = MaxValueDev{ci, cv.x, cv.y, yc, pc, 0.f, rfc, 0u};
+  float rfr = hr ? __fmul_rn((float)(ci + 1), bw) : 0.f;
+  if (mirror && hr) rfr = __fsub_rn(fs, rfr);
+  o[3] = MaxValueDev{hr ? ci + 1 : 0u, rv.x, rv.y, yr, hr ? phase_deg(rv) : 0.f, 0.f, rfr, 0u};
+}
+
+// The search of one beam by a CTA of T threads: the largest |X| of bins [0, half)
+// and of the last `half` bins, and the records of the larger one or of both (each by
+// a thread of its own).  bins(k) is bin k; keys: 2 T / 32 words of shared memory.
+template <uint32_t T, typename Bins>
+SPX_DEV void one_two_search(const Bins& bins, uint64_t* keys, uint32_t nfft, uint32_t half, float fs, int two_peaks,
+                            MaxValueDev* o) {
+  constexpr uint32_t W = T / 32;
+  const uint32_t r0 = nfft - half;
+  uint64_t kl = 0, kr = 0;
+  for (uint32_t t = threadIdx.x; t < half; t += T) {
+    const uint64_t a = one_two_key(mag_rn(bins(t)), t);
+    const uint64_t b = one_two_key(mag_rn(bins(r0 + t)), t);
+    kl = a > kl ? a : kl;
+    kr = b > kr ? b : kr;
+  }
+  kl = lane_max_u64(kl);
+  kr = lane_max_u64(kr);
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (lane == 0) {
+    keys[warp] = kl;
+    keys[W + warp] = kr;
+  }
+  __syncthreads();
+  const bool second = threadIdx.x == T / 2;
+  if (threadIdx.x != 0 && !(second && two_peaks)) return;
+  kl = kr = 0;
+  for (uint32_t w = 0; w < W; ++w) {
+    kl = keys[w] > kl ? keys[w] : kl;
+    kr = keys[W + w] > kr ? keys[W + w] : kr;
+  }
+  // Decode; an empty (or all-NaN) range keeps the reference's initial values.
+  const uint32_t il = kl ? one_two_offset(kl) : 0u;
+  const float ml = kl ? __uint_as_float((uint32_t)(kl >> 32)) : -1.0f;
+  const uint32_t ir = kr ? r0 + one_two_offset(kr) : r0;
+  const float mr = kr ? __uint_as_float((uint32_t)(kr >> 32)) : -1.0f;
+  const bool right = two_peaks ? second : mr > ml;
+  write_peak4(bins, nfft, right ? ir : il, fs, right, second ? o + 4 : o);
+}
 
 }  // namespace spx

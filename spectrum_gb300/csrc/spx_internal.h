@@ -191,6 +191,10 @@ spx_status launch_topk_pair(spx_ctx* ctx, const FftPlan& plan, const float2* d_i
                             uint32_t n_point, const float* d_win, uint32_t start, uint32_t end,
                             uint32_t k, float fs, uint32_t refine, spx_max_value* d_out,
                             uint32_t* d_counts, float2* d_ctx);
+// One or two peaks (launch_one_two) of the same plans, search_range in [2, nfft].
+spx_status launch_one_two_pair(spx_ctx* ctx, const FftPlan& plan, const float2* d_in, uint32_t beams,
+                               uint32_t n_point, const float* d_win, uint32_t search_range, float fs,
+                               int two_peaks, spx_max_value* d_out);
 // spx_mlp_refine on peaks whose neighbourhoods are in d_ctx (launch_topk_pair).
 spx_status launch_mlp_refine_ctx(spx_ctx* ctx, const spx_mlp* m, const float2* d_ctx, uint32_t beams,
                                  uint32_t n_point, uint32_t nfft, float fs, uint32_t K,

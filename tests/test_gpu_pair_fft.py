@@ -155,6 +155,21 @@ def test_topk_equals_the_scalar_kernels(spx, scalar, nfft):
         assert torch.equal(a[0], b[0]) and torch.equal(a[1], b[1]), (nfft, n, k, lo, hi)
 
 
+@pytest.mark.parametrize("nfft", [1024, 2048, 4096, 8192, 16384])
+def test_one_and_two_peaks_equal_the_scalar_kernels(spx, scalar, nfft):
+    import torch
+    for n, offset, rng in ((nfft, 0, 0), (nfft - 1, 0, nfft), (nfft // 2, 1, 2), (5, 0, 77), (nfft, 0, nfft - 1)):
+        x = _hard_beams(_samples(9, n, offset, nfft + n + rng))
+        for mode in (spx.PEAK_ONE, spx.PEAK_TWO):
+            a, b = (spx.fft_peaks(x, nfft, spx.WINDOW_BLACKMAN, mode, 1e6, search_range=rng, ctx=c)[0]
+                    for c in (None, scalar))
+            assert torch.equal(a, b), (nfft, n, rng, mode)
+    for rng in (1, nfft + 1):
+        for c in (None, scalar):
+            with pytest.raises(Exception, match="search_range must be in"):
+                spx.fft_peaks(x, nfft, 0, spx.PEAK_TWO, 1e6, search_range=rng, ctx=c)
+
+
 @pytest.mark.parametrize("nfft,beams,k", [(1024, 2050, 3), (2048, 1030, 32), (4096, 520, 1), (8192, 300, 8), (16384, 130, 2)])
 def test_learned_topk_equals_its_three_steps(spx, nfft, beams, k):
     import torch
