@@ -40,18 +40,20 @@ FS = 1.0
 SIGMA = 6.0
 METRIC = "Msamples/s FFT+|X|+peaks (256x65536 -> nFFT 131072, Hann, all maxima > 6 sigma)"
 # DRAM bytes (read + write) of one step on this workload: the sum of
-# dram__bytes_read.sum + dram__bytes_write.sum of fft_group_kernel<16384> and
-# maxima_cluster_kernel, one ncu capture of each on 160 beams, scaled by
-# 256 / 160 (every beam does the same work).  NCU_TRAFFIC_KERNELS names the
+# dram__bytes_read.sum + dram__bytes_write.sum of mid_cols_kernel<8>,
+# mid_rows_window_kernel and maxima_cluster_kernel, one ncu capture of each on
+# 160 beams, scaled by 256 / 160 (every beam does the same work).  NCU_TRAFFIC_KERNELS names the
 # kernels and the commit the figure was taken at, so a change of either shows
 # that it must be captured again.
-NCU_TRAFFIC_BYTES = 353_151_795
-NCU_TRAFFIC_KERNELS = {"kernels": ["fft_group_kernel<16384>", "maxima_cluster_kernel"], "commit": "ba338c8",
+NCU_TRAFFIC_BYTES = 756_690_944
+NCU_TRAFFIC_KERNELS = {"kernels": ["mid_cols_kernel<8>", "mid_rows_window_kernel", "maxima_cluster_kernel"],
+                       "commit": "ccf0d7c",
                        "beams_captured": 160}
 # What the ncu counters of the step's kernels show bounds them (same capture
 # as NCU_TRAFFIC_BYTES): neither DRAM nor the FP32 pipe is saturated.
-NCU_LIMITER = ("instruction issue and load latency: fft_group_kernel<16384> 45 % issue active, 13.4 % DRAM "
-               "throughput, 30 % FMA pipe, top stall long_scoreboard; maxima_cluster_kernel 18.9 % DRAM")
+NCU_LIMITER = ("load latency and the shared-memory / L1 data path: mid_cols_kernel<8> 45 % issue active, 52 % DRAM "
+               "throughput, top stall long_scoreboard; mid_rows_window_kernel 47 % issue, 49 % FMA pipe, 54 % DRAM; "
+               "maxima_cluster_kernel 48 % issue, 27 % DRAM")
 WORKLOAD = "plain-large: 256 beams x 65536 c64, Hann, nFFT 131072, all local maxima > 6 sigma, parabolic"
 
 
@@ -408,8 +410,8 @@ def run_gpu(args):
 
 
 def time_components(spx, ctx, xs, out, counts, p, stream, steps):
-    """Times a step (the FFT kernel and the maxima kernel, back to back on one
-    stream) with CUDA events on the launching stream, plus the composed path
+    """Times a step (the FFT's two kernels and the maxima kernel, back to back on
+    one stream) with CUDA events on the launching stream, plus the composed path
     (spx_fft to a spectrum in device memory, then spx_all_maxima)."""
     import ctypes as C
 
@@ -450,21 +452,21 @@ def time_components(spx, ctx, xs, out, counts, p, stream, steps):
     # algorithmic bytes: samples read once + maxima and counts written
     algo = BEAMS * N_POINT * 8 + n_max * 32 + BEAMS * 4
     return {
-        "path": "spx_fft_peaks: fft_group_kernel<16384> (persistent cooperative launch, 19 groups of 8 CTAs x "
-                "1024 threads, one CTA per SM; per beam: window, zero pad, 131072-point FFT with a device-memory "
-                "group barrier, the search window's bins in row layout into the beam's L2 exchange slot) then "
-                "maxima_cluster_kernel (one cluster of 8 CTAs x 256 threads per beam, 5 CTAs per SM: |X|, noise "
-                "histogram merged through DSMEM, 6-sigma threshold, maxima, ranks)",
+        "path": "spx_fft_peaks: mid_cols_kernel<8> (window, zero pad, the 8-point cross stage and the first radix-16 "
+                "pass of 32 columns per CTA into 128 rows of scratch per beam), mid_rows_window_kernel (the 1024-point "
+                "FFT of each row by one warp, the search window's elements written back over the row), "
+                "maxima_cluster_kernel (one cluster of 8 CTAs x 256 threads per beam: |X|, noise histogram merged "
+                "through DSMEM, 6-sigma threshold, maxima, ranks)",
         "components_ms": {"fused_step": round(f, 4), "composed_fft_complex": round(statistics.median(fft_ms), 4),
                           "composed_peaks": round(statistics.median(peak_ms), 4)},
-        "roofline": {"bound": "hbm", "kernel": "fft_group_kernel + maxima_cluster_kernel (one step)",
+        "roofline": {"bound": "hbm", "kernel": "mid_cols_kernel + mid_rows_window_kernel + maxima_cluster_kernel (one step)",
                      "achieved": round(algo / (f * 1e-3) / 1e9, 1),
                      "unit": "GB/s", "traffic": NCU_TRAFFIC_BYTES,
                      "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch of each "
                                        "kernel of the step", "traffic_captured": NCU_TRAFFIC_KERNELS,
                      "algorithmic_bytes_per_launch": algo,
                      "maxima_per_launch": n_max},
-        "launches_per_step": 2,
+        "launches_per_step": 3,
         "fp64": fp,
     }
 
@@ -554,7 +556,7 @@ def fp64_error(xs, specs, nfft, kind) -> dict:
 
 def bench_workloads(spx, ctx, stream, dev, hbm):
     """The other workloads of the path, each timed on the device with inputs
-    resident: small (8 x 4096 top-5), uneven (1024 beams, one launch vs one
+    resident: small (8 x 4096 top-5), uneven (1024 beams, one batch vs one
     launch pair per size), precision (64 x 2^20 Blackman-Harris, error vs an
     FP64 FFT on two beams) and learned (training time; inference on 4096 x
     8192 against the plain parabolic path, with frequency RMS errors)."""
@@ -636,8 +638,9 @@ def bench_workloads(spx, ctx, stream, dev, hbm):
     res["uneven"] = {"config": "1024 beams, n_point U[1000,100000], nFFT = next 2^a3^b, Hann, top-8",
                      "samples": samples, "distinct_nfft": len(first),
                      "ms_batch_run": round(ms_one, 4), "ms_graph_replay": round(ms_graph, 4),
-                     "batch_run": "spx_batch_run: one launch of every beam's FFT (clusters), then one "
-                                  "top-K launch; the autotuner's local sizes and cluster size",
+                     "batch_run": "spx_batch_run: the column and row launches of the C x M-point beams beside "
+                                  "one launch of the rest (clusters), then one top-K launch; the autotuner's "
+                                  "local sizes and cluster size",
                      "batch_plans": {"cluster": int(b.cluster), "changed_by_autotune": int(tune_changed)},
                      "ms_plain_per_beam_eager": round(ms_plain, 4),
                      "ms_plain_per_beam_graph": round(ms_plain_graph, 4),
@@ -743,12 +746,12 @@ def bench_workloads(spx, ctx, stream, dev, hbm):
                       "final_loss": float(losses[-1]),
                       "ms_plain_fft_topk": round(ms_plain, 4), "ms_spx_fft_peaks_topk": round(ms_fused, 4),
                       "ms_spx_fft_peaks_mlp": round(ms_one, 4),
-                      "spx_fft_peaks_mlp_path": "2^25 points per call: spx_fft, spx_topk and spx_mlp_refine "
-                                                "(one fused launch only up to 2^21 points per call)",
+                      "spx_fft_peaks_mlp_path": "2^25 points per call: transform and top-K in one launch, the "
+                                                "refinement of the peaks' five bins in a second (one launch up to "
+                                                "2^21 points per call)",
                       "small_128x8192": {"ms_spx_fft_peaks_mlp_one_launch": round(ms_one_small, 4),
                                          "ms_three_steps": round(ms_three_small, 4)},
-                      "spx_fft_peaks_path": "spectrum to device memory + topk_kernel (the single-CTA fused "
-                                            "kernel is taken up to 2^23 points per call)",
+                      "spx_fft_peaks_path": "one launch, the spectrum on chip (fft_topk_pair_kernel)",
                       "ms_with_learned_refine": round(ms_ref, 4),
                       "ms_refine_kernel": round(ms_kernel, 4),
                       "Msamples_per_s_with_refine": round(4096 * nl / (ms_ref * 1e-3) / 1e6, 1),

@@ -28,7 +28,7 @@
  *                              src/fft_func/src/all_maxima_pipeline_rocm.cpp:258-472)
  *   spx_topk               -> (no reference counterpart: top-K of local maxima)
  *   spx_fft_peaks          -> ISpectrumProcessor::ProcessFromGPU / FindAllMaximaFromGPUPipeline
- *                             fused: one launch up to nfft 16384, FFT + maxima launch
+ *                             fused: one launch up to nfft 16384, FFT + maxima launches
  *                             above (include/spectrum/interface/i_spectrum_processor.hpp:95-129)
  */
 #ifndef SPX_H_
@@ -167,16 +167,17 @@ uint32_t spx_next_pow2(uint32_t n);
 /* Smallest 2^a*3^b >= n (extension for beams of uneven length). */
 uint32_t spx_next_smooth23(uint32_t n);
 /* 1 if this build can transform nfft points; else 0.  2^a*3^b in
- * [2, 262144]: one pass (cluster of <= 16 CTAs); 2^19 and 2^20: two
+ * [2, 16384]: one launch, up to 262144: two; 2^19 and 2^20: two
  * launches, 2^21: three; 2^a*3^b above 2^21 up to 2^28 that split into two factors
  * <= 16384 (every power of two): four steps with transposes; any other
- * length up to 2^27: Bluestein's chirp-z transform.  The reference takes any
+ * length up to 2^27: Bluestein's chirp-z transform (one launch up to 8192
+ * points).  The reference takes any
  * nextPow2(n_point) * repeat_count (fft_processor_rocm.cpp:673-677). */
 int spx_fft_size_supported(uint32_t nfft);
 /* Tuning for transforms of nfft points: points each thread holds per pass
  * (16: more resident warps; 32: more work per thread) and, above 16384
  * points, the preferred points per CTA of a beam's cluster (1024..16384;
- * 0 = default 16384: one CTA per SM; 8192 allows two).  No reference counterpart (hipFFT
+ * 0 = default 16384).  Sizes at the defaults run the packed kernels.  No reference counterpart (hipFFT
  * chooses internally); set by the autotuner or by hand. */
 spx_status spx_set_fft_tuning(spx_ctx* ctx, uint32_t nfft, uint32_t points_per_thread,
                               uint32_t points_per_cta);
@@ -270,10 +271,12 @@ spx_status spx_all_maxima_noalloc(spx_ctx* ctx, const float* d_mag, const void* 
                                   spx_max_value* d_out, uint32_t* d_counts);
 
 /* ---- fused: raw samples -> peaks ---------------------------------------- */
-/* Window + zero-pad + FFT + |X| + peak search.  nfft <= 16384 (ALL, TOPK):
- * one launch, the spectrum never goes to device memory.  ALL with nfft >
- * 16384: the FFT writes only the search window's bins (device scratch), then
- * one maxima launch.  Other cases: spx_fft, then the peak function.
+/* Window + zero-pad + FFT + |X| + peak search.  Power-of-two nfft
+ * from 1024 to 16384 (ONE, TWO, TOPK without a threshold) and small calls of
+ * other nfft <= 16384 (ALL, TOPK): one launch, the spectrum never goes to
+ * device memory.  ALL with nfft > 16384: the FFT writes only the search
+ * window's bins (device scratch), then one maxima launch.  Other cases:
+ * spx_fft, then the peak function.
  * params->mode selects ONE/TWO/ALL/TOPK with the layouts of
  * spx_peaks_one_two / spx_all_maxima / spx_topk.  d_counts may be NULL for
  * ONE/TWO; d_out may be NULL for ALL when the capacity is 0. */
@@ -433,8 +436,9 @@ spx_status spx_mlp_refine(spx_ctx* ctx, spx_mlp* mlp, const void* d_fft, uint32_
  * spectrum's shared memory (2^a 3^b nfft from about 2600 to 16384 points),
  * and the call is small (beams x nfft <= 2^21), this is ONE launch:
  * transform, top-K search and the network on each peak, the spectrum never
- * written to device memory; otherwise the three steps run (faster once many
- * CTAs queue: one launch holds each SM while it stages the weights).  No reference counterpart (the
+ * written to device memory.  Larger calls that spx_fft_peaks searches on chip
+ * take two launches, the search handing on five bins per peak; otherwise the
+ * three steps run (one launch holds each SM while it stages the weights).  No reference counterpart (the
  * reference refines with the parabola, fft_kernel_sources_rocm.hpp:228-239). */
 spx_status spx_fft_peaks_mlp(spx_ctx* ctx, spx_mlp* mlp, const void* d_in, uint32_t beams,
                              uint32_t n_point, uint32_t nfft, uint32_t window,

@@ -227,15 +227,10 @@ struct ExchangeLoader {
 };
 
 // Output of a last local pass into a row of device memory: row[i] = Z[i]
-// (L2-kept stores for rows read again in the same launch or the next one,
-// streaming stores otherwise).
+// (L2-kept stores: rows are read again in the same launch or the next one).
 struct RowOut {
   float2* row;
   SPX_DEV void operator()(uint32_t i, float2 z) const { __stcg(row + i, z); }
-};
-struct RowOutStream {
-  float2* row;
-  SPX_DEV void operator()(uint32_t i, float2 z) const { __stcs(row + i, z); }
 };
 
 // First Stockham pass (Ns = 1) reading its inputs from device memory.

@@ -24,7 +24,7 @@
 // L1, and the spectrum comes out in bin order without a transpose.
 // 256 beams of 65536 samples in 131072 bins: launch 1 0.068 ms (5.0 TB/s of
 // samples and scratch), bound by device memory; launch 2 0.066 ms (6.0 TB/s),
-// bound by the L1's data path (82 % of its wavefronts: two exchanges, twiddles,
+// bound by the L1's data path (77 % of its wavefronts: two exchanges, twiddles,
 // loads).  In bin order launch 2 takes 0.10 ms: runs of four bins cost the L1
 // as much as the rest.
 //

@@ -743,13 +743,6 @@ SPX_DEV void pair_cross_stage(float2* __restrict__ slot, uint32_t c, const Sampl
   }
 }
 
-// Four complex values, one 32-byte store (p on a 32-byte boundary).
-SPX_DEV void st256(float2* p, float2 a, float2 b, float2 c, float2 d) {
-  asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(b.x),
-               "f"(b.y), "f"(c.x), "f"(c.y), "f"(d.x), "f"(d.y)
-               : "memory");
-}
-
 // Elements i, i + 1 into a 16-byte aligned row of device memory.
 struct RowOutPairs {
   float2* row;

@@ -14,6 +14,8 @@
 //                      compacted in bin order.
 //   TOPK (C == 1)    : the K largest strict local maxima (optionally above the
 //                      threshold), |X| descending, ties by lower bin.
+//   ONE, TWO (C == 1): power-of-two sizes of the packed kernels, see
+//                      fft_one_two_pair_kernel; other sizes go through spx_fft.
 // Results are bit-identical to spx_fft (COMPLEX) followed by spx_all_maxima /
 // spx_topk: the same FFT code, |X| = sqrt_rn(re*re + im*im), the same
 // histogram-median threshold and the same comparisons.

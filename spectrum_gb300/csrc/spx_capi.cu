@@ -555,14 +555,13 @@ spx_status spx_fft_peaks(spx_ctx* ctx, const void* d_in, uint32_t beams, uint32_
       return launch_topk_pair(ctx, *plan, static_cast<const float2*>(d_in), beams, n_point, win, start, end, cap,
                               params->sample_rate, params->refine, d_out, d_counts, nullptr);
     }
-    // nfft <= 16384 (one CTA per beam): the fused kernel keeps the spectrum
-    // on chip, but its search phase holds the SM from the next beam's
-    // transform, which pays only while the launch is short.  Measured on
-    // GB300 (8 .. 4096 beams of 4096 .. 16384 points, top-1/8 and 6-sigma
-    // all maxima), fused is faster for top-K at 4096 points or up to 2^23
-    // points in all, and for all maxima up to 2^21 points in all; beyond, the
-    // spectrum in device memory and a separate search kernel win (e.g. 4096
-    // x 16384 top-8: 0.597 vs 0.463 ms).  Both give the same bits.
+    // Otherwise nfft <= 16384 in one CTA per beam (thresholds, all maxima, 3-smooth
+    // sizes): the scalar fused kernel keeps the spectrum on chip, but its search
+    // phase holds the SM from the next beam's transform, which pays only while the
+    // launch is short.  Measured on GB300 (8 .. 4096 beams of 4096 .. 16384 points):
+    // fused is faster for top-K at 4096 points or up to 2^23 points in all, and for
+    // all maxima up to 2^21 points in all; beyond, the spectrum in device memory and
+    // a separate search kernel win.  Both give the same bits.
     const uint64_t pts = (uint64_t)beams * nfft;
     const bool single_cta_pays =
         plan->g.C > 1 || (all ? pts <= (1ull << 21) : (nfft <= 4096 || pts <= (1ull << 23)));

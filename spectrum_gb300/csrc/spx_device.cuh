@@ -30,7 +30,6 @@ SPX_DEV float2 cmul(float2 a, float2 w) {
   return make_float2(fmaf(a.x, w.x, -a.y * w.y), fmaf(a.x, w.y, a.y * w.x));
 }
 SPX_DEV float2 mul_neg_i(float2 a) { return make_float2(a.y, -a.x); }  // a * (-i)
-SPX_DEV float2 mul_pos_i(float2 a) { return make_float2(-a.y, a.x); }  // a * (+i)
 
 // |z| and |z|^2 with every operation rounded separately (no FMA contraction),
 // i.e. sqrt_rn(re*re + im*im) exactly as a CPU evaluates it in FP32.  Peak
