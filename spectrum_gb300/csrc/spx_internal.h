@@ -142,6 +142,12 @@ inline cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, v
   return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 
+// Two beams per CTA: 2^a 3^b points, not a power of two, 1024 .. 8192 (fft_twin.cu).
+bool twin_supported(const FftGeom& g);
+cudaError_t launch_fft_twin(const FftPlan& plan, const float2* d_in, uint32_t beams, uint32_t n_point,
+                            const float* d_win, uint32_t out_mode, float scale, void* d_out,
+                            cudaStream_t stream, bool prefetch);
+
 // Two-launch transforms of 32768 .. 262144 = C x 16384 points (fft_mid.cu).
 // The rows form leaves the spectrum in d_rows [beams][16 C][1024]: bin
 // rho + 16 C q is element q of row rho, defined for bins [klo, khi).

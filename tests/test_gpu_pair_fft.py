@@ -182,3 +182,32 @@ def test_learned_topk_equals_its_three_steps(spx, nfft, beams, k):
     ramp, rused = net.refine(spec, ref, n, nfft, 1e6)
     for a, b in ((out, ref), (counts, n), (amp.view(torch.int32), ramp.view(torch.int32)), (used, rused)):
         assert torch.equal(a, b)
+
+
+TWIN_SIZES = [n for n in (2 ** a * 3 ** b for a in range(13) for b in range(1, 9)) if 1024 < n < 8192]
+
+
+@pytest.mark.parametrize("nfft", sorted(TWIN_SIZES))
+def test_two_beams_per_cta_equal_the_scalar_kernels(spx, nfft):
+    import torch
+    from spectrum_gb300._capi import lib
+    other = spx.Context(0)
+    other.check(lib.spx_set_fft_tuning(other.h, nfft, 32, 0))
+    for beams, n, offset, window in ((1, nfft, 0, spx.WINDOW_HANN), (2, nfft - 1, 1, spx.WINDOW_BLACKMAN),
+                                     (5, nfft // 2 + 1, 0, spx.WINDOW_NONE), (4, 1, 1, 0)):
+        x = _samples(beams, n, offset, nfft + n)
+        x[beams - 1, 0] = complex(float("inf"), 0.0)  # (stays in its beam)
+        for out in MODES:
+            a, b = (spx.fft(x, nfft, window, out, 0.25, ctx=c) for c in (None, other))
+            assert _same(a, b), (nfft, beams, n, out)
+    x = _samples(3, nfft, 0, nfft)
+    ref = spx.ifft(x, ctx=other)
+    assert _same(spx.ifft(x), ref)
+    y = torch.empty(3 * nfft + 1, dtype=torch.complex64, device="cuda")[1:].reshape(3, nfft)
+    assert _same(spx.ifft(x, out=y), ref)
+    z = x.clone()
+    spx.ifft(z, out=z)
+    assert _same(z, ref)
+    r = x.real.contiguous()
+    for full in (False, True):
+        assert _same(spx.fft_r2c(r, nfft, 1, full), spx.fft_r2c(r, nfft, 1, full, ctx=other))
