@@ -300,6 +300,10 @@ SPX_DEV uint64_t br_scan(const float2* rows, uint32_t C, uint32_t L, uint32_t st
 // the |X| of the neighbours).
 // Six CTAs per SM (42 registers, 48 bytes spilled): more loads of the
 // beams' rows in flight than at four (no spill); uneven step 0.759 -> 0.744 ms.
+// ITEMS: the set holds beams of batch_rows.cuh; sets without them run a kernel
+// without their scan, whose registers cost the other scans spills (69 beams:
+// 44.9 -> 48.2 us).
+template <bool ITEMS>
 __global__ void __launch_bounds__(kBtThreads, 6)
 topk_batch_kernel(const float2* __restrict__ xch, const BatchBeam* __restrict__ beams,
                   const BatchGeom* __restrict__ geoms, const uint32_t* __restrict__ beam_list, TopkArgs a) {
@@ -311,7 +315,7 @@ topk_batch_kernel(const float2* __restrict__ xch, const BatchBeam* __restrict__ 
   if (end >= nfft) end = nfft - 1;
   const uint32_t C = geoms[bm.geom].g.C, M = geoms[bm.geom].g.M;
   const RowBins bins{xch + bm.spec_off, M};
-  const bool br = geoms[bm.geom].twr != nullptr;
+  const bool br = ITEMS && geoms[bm.geom].twr != nullptr;
   const uint32_t R0 = geoms[bm.geom].R0, L = geoms[bm.geom].L, NP = geoms[bm.geom].NP;
   const uint32_t cmagic = 0xFFFFFFFFu / C + 1u;  // k div C = umulhi(k, cmagic) (k * C < 2^32)
   auto bin = [&](uint32_t k) -> float2 {
@@ -800,7 +804,8 @@ spx_status launch_set(spx_ctx* ctx, spx_batch* b, const LaunchSet& ls, const voi
     if (e != cudaSuccess) return cuda_fail(ctx, e, "launch batch_cols_kernel / batch_rows_kernel");
   }
   const TopkArgs tk{reinterpret_cast<MaxValueDev*>(d_out), d_counts, b->K, b->start, b->end, b->refine, b->fs};
-  topk_batch_kernel<<<ls.beams, kBtThreads, 0, ctx->stream>>>(b->d_xch, b->d_beams, b->d_geoms, ls.d_beam_list, tk);
+  const auto topk = ls.n_cols ? topk_batch_kernel<true> : topk_batch_kernel<false>;
+  topk<<<ls.beams, kBtThreads, 0, ctx->stream>>>(b->d_xch, b->d_beams, b->d_geoms, ls.d_beam_list, tk);
   e = cudaGetLastError();
   return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch topk_batch_kernel");
 }
