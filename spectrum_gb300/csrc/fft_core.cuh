@@ -461,6 +461,15 @@ struct CtPlan {
     return p == 0 ? 0 : twoff(p - 1) + (int)tw_entries((uint32_t)radix(p - 1), (uint32_t)ns(p - 1));
   }
   static_assert(M == (1 << a) * ct_pow3(b) && M <= 16384, "M must be 2^a 3^b <= 16384");
+  // Where elements lie between two passes.  Powers of two: element i at sw(i).
+  // Plans with a factor of 3: ahead of pass p in blocks of ns(p) elements, one
+  // unused element after each block of a first radix-16 pass (sw's positions
+  // there), so that the passes on both sides reach their elements by constant
+  // offsets; sw costs their strides an index computation per element and pass.
+  // (Not behind a first radix-8 pass: its blocks need more room than sw_len.)
+  // Only plans whose last pass hands its outputs on (ct_local_fft_out) may use it.
+  static constexpr bool blocks = b > 0 && !lead8;
+  static constexpr int pad(int p) { return p == 1 && radix(0) % 2 == 0 ? 1 : 0; }
 };
 
 // Barriers of a local FFT: the whole CTA's, or one group of N consecutive
@@ -487,7 +496,10 @@ SPX_DEV void ct_first(float2* s, const Load& load, uint32_t tid) {
 #pragma unroll
       for (int r = 0; r < R; ++r) v[r] = load(j + r * B);
       Dft<R>::run(v);
-      if constexpr (16 % R == 0) {
+      if constexpr (P::blocks) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) s[j * (R + P::pad(1)) + r] = v[r];
+      } else if constexpr (16 % R == 0) {
         // base = R j: base mod 16 + r < 16, so sw(base + r) = sw(base) + r
         const uint32_t sb = sw(j * R);
 #pragma unroll
@@ -513,9 +525,15 @@ SPX_DEV void ct_pass(float2* s, const float2* __restrict__ tw, uint32_t tid) {
   for (int q = 0; q < Q; ++q) {
     const uint32_t j = tid + q * T;
     if (B % T == 0 || q + 1 < Q || j < (uint32_t)B) {
-      const uint32_t sj = sw(j);
+      if constexpr (PL::blocks) {
+        const float2* p = s + j + PL::pad(P) * (j / Ns);
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[q][r] = s[(B % 16 == 0) ? sj + sw(r * B) : sw(j + r * B)];
+        for (int r = 0; r < R; ++r) v[q][r] = p[r * (B + PL::pad(P) * (B / Ns))];
+      } else {
+        const uint32_t sj = sw(j);
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[q][r] = s[(B % 16 == 0) ? sj + sw(r * B) : sw(j + r * B)];
+      }
     }
   }
   if constexpr (P + 1 < PL::npass) Sync::wait();
@@ -534,9 +552,15 @@ SPX_DEV void ct_pass(float2* s, const float2* __restrict__ tw, uint32_t tid) {
       }
       Dft<R>::run(v[q]);
       const uint32_t base = (j - k) * R + k;
-      const uint32_t sb = sw(base);
+      if constexpr (PL::blocks) {
+        static_assert(P + 1 < PL::npass, "the last pass writes other elements than it read");
 #pragma unroll
-      for (int r = 0; r < R; ++r) s[(Ns % 16 == 0) ? sb + sw(r * Ns) : sw(base + r * Ns)] = v[q][r];
+        for (int r = 0; r < R; ++r) s[base + PL::pad(P + 1) * (j / Ns) + r * Ns] = v[q][r];
+      } else {
+        const uint32_t sb = sw(base);
+#pragma unroll
+        for (int r = 0; r < R; ++r) s[(Ns % 16 == 0) ? sb + sw(r * Ns) : sw(base + r * Ns)] = v[q][r];
+      }
     }
   }
   Sync::wait();
@@ -565,9 +589,15 @@ SPX_DEV void ct_last_pass_out(const float2* s, const float2* __restrict__ tw, ui
   for (int q = 0; q < Q; ++q) {
     const uint32_t j = tid + q * T;
     if (B % T == 0 || q + 1 < Q || j < (uint32_t)B) {
-      const uint32_t sj = sw(j);
+      if constexpr (PL::blocks) {
+        const float2* p = s + j + PL::pad(P) * (j / Ns);
 #pragma unroll
-      for (int r = 0; r < R; ++r) v[q][r] = s[(B % 16 == 0) ? sj + sw(r * B) : sw(j + r * B)];
+        for (int r = 0; r < R; ++r) v[q][r] = p[r * (B + PL::pad(P) * (B / Ns))];
+      } else {
+        const uint32_t sj = sw(j);
+#pragma unroll
+        for (int r = 0; r < R; ++r) v[q][r] = s[(B % 16 == 0) ? sj + sw(r * B) : sw(j + r * B)];
+      }
     }
   }
 #pragma unroll
