@@ -552,8 +552,9 @@ spx_status launch_fft_out(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
     e = launch_pair(plan, d_in, beams, n_point, d_win, out_mode, scale, d_out, ctx->stream, !ctx->input_on_host);
     return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch fft_pair_kernel");
   }
-  // 2^a 3^b sizes from 1024 to 8192: two beams per CTA, faster at every size and
-  // number of beams measured (1 .. 29000 beams, all modes; figures in fft_twin.cu)
+  // the other 2^a 3^b sizes above 1024 (two beams per CTA up to 8192): faster at
+  // every size and number of beams measured (1 .. 29000 beams, all modes; figures
+  // in fft_twin.cu)
   if (twin_supported(g)) {
     e = launch_fft_twin(plan, d_in, beams, n_point, d_win, out_mode, scale, d_out, ctx->stream, !ctx->input_on_host);
     return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch fft_twin_kernel");

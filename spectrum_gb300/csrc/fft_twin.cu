@@ -1,5 +1,5 @@
-// fft_twin.cu — batched transforms of 2^a 3^b points, not a power of two, from
-// 1024 to 8192: two beams per CTA in packed arithmetic.
+// fft_twin.cu — batched transforms of 2^a 3^b points, not a power of two: from
+// 1024 to 8192 two beams per CTA in packed arithmetic, up to 16384 one.
 //
 // The odd strides of these plans leave no neighbours to pair inside a beam
 // (fft_pair.cuh), so the two values of a pair are the same element of two beams:
@@ -189,10 +189,32 @@ fft_twin_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __
   }
 }
 
+// 8748 .. 15552 points: pairs of beams would not fit the register file, so one
+// beam per CTA in scalar arithmetic, at the compile-time plan (fft_core.cuh),
+// where fft_out_kernel runs the passes with run-time radices and strides.  2^25
+// points, complex: 8748 398 -> 290 us, 9216 301 -> 216, 12288 285 -> 205, 15552 313
+// -> 237; inverse 286 -> 213 at 12288.
+template <int M>
+__global__ void __launch_bounds__(CtPlan<M>::T)
+fft_solo_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __restrict__ win, FftGeom g,
+                const float2* __restrict__ tw, void* __restrict__ out, uint32_t out_mode, float scale) {
+  extern __shared__ float2 s2[];
+  const uint32_t tid = threadIdx.x, beam = blockIdx.x;
+  prefetch_future_beam(g, in, n_point, beam, 0, tid, CtPlan<M>::T);
+  const SampleLoader ld{in + (size_t)beam * n_point, n_point, win};
+  if (out_mode == SPX_OUT_COMPLEX) {
+    float2* o = reinterpret_cast<float2*>(out) + (size_t)beam * M;
+    ct_local_fft_out<M>(s2, ld, tw, tid, [=](uint32_t k, float2 z) { o[k] = z; });
+  } else {
+    ct_local_fft_out<M>(s2, ld, tw, tid, BinOut{out, out_mode, scale, &g, beam});
+  }
+}
+
 template <int M>
 static const void* twin_kernel(uint32_t m) {
-  if (m == M) return (const void*)fft_twin_kernel<M>;
-  return nullptr;
+  if (m != M) return nullptr;
+  if constexpr (M > 8192) return (const void*)fft_solo_kernel<M>;
+  else return (const void*)fft_twin_kernel<M>;
 }
 static const void* twin_kernel_of(uint32_t m) {
   const void* k = nullptr;
@@ -200,7 +222,9 @@ static const void* twin_kernel_of(uint32_t m) {
 #define SPX_TWIN(n) std::integral_constant<int, n>()
   any(SPX_TWIN(1152), SPX_TWIN(1296), SPX_TWIN(1458), SPX_TWIN(1536), SPX_TWIN(1728), SPX_TWIN(1944), SPX_TWIN(2187),
       SPX_TWIN(2304), SPX_TWIN(2592), SPX_TWIN(2916), SPX_TWIN(3072), SPX_TWIN(3456), SPX_TWIN(3888), SPX_TWIN(4374),
-      SPX_TWIN(4608), SPX_TWIN(5184), SPX_TWIN(5832), SPX_TWIN(6144), SPX_TWIN(6561), SPX_TWIN(6912), SPX_TWIN(7776));
+      SPX_TWIN(4608), SPX_TWIN(5184), SPX_TWIN(5832), SPX_TWIN(6144), SPX_TWIN(6561), SPX_TWIN(6912), SPX_TWIN(7776),
+      SPX_TWIN(8748), SPX_TWIN(9216), SPX_TWIN(10368), SPX_TWIN(11664), SPX_TWIN(12288), SPX_TWIN(13122),
+      SPX_TWIN(13824), SPX_TWIN(15552));
 #undef SPX_TWIN
   return k;
 }
@@ -213,14 +237,16 @@ cudaError_t launch_fft_twin(const FftPlan& plan, const float2* d_in, uint32_t be
   FftGeom g = plan.g;
   const void* kfn = twin_kernel_of(g.M);
   const uint32_t threads = ((g.M + 15) / 16 + 31) / 32 * 32;
-  const size_t smem = (size_t)(g.M + (g.radix[0] % 2 == 0 ? g.M / g.radix[0] : 0)) * sizeof(float4);  // TwinPlan::slots
+  const uint32_t per_cta = g.M > 8192 ? 1 : 2;
+  const size_t smem = per_cta == 1 ? (size_t)sw_len(g.M) * sizeof(float2)
+                                   : (size_t)(g.M + (g.radix[0] % 2 == 0 ? g.M / g.radix[0] : 0)) * sizeof(float4);  // TwinPlan::slots
   cudaError_t e = configure_kernel(kfn, smem);
   if (e != cudaSuccess) return e;
   g.beams = beams;
   g.ahead = prefetch ? resident_ctas(kfn, threads, smem, 1) : 0u;
   void* args[] = {(void*)&d_in, (void*)&n_point, (void*)&d_win, (void*)&g,
                   (void*)&plan.d_tw_local, (void*)&d_out, (void*)&out_mode, (void*)&scale};
-  return cudaLaunchKernel(kfn, dim3((beams + 1) / 2), dim3(threads), args, smem, stream);
+  return cudaLaunchKernel(kfn, dim3((beams + per_cta - 1) / per_cta), dim3(threads), args, smem, stream);
 }
 
 }  // namespace spx

@@ -142,7 +142,7 @@ inline cudaError_t launch_dependent(const void* kernel, dim3 grid, dim3 block, v
   return cudaLaunchKernelExC(&cfg, kernel, args);
 }
 
-// Two beams per CTA: 2^a 3^b points, not a power of two, 1024 .. 8192 (fft_twin.cu).
+// 2^a 3^b points, not a power of two, 1024 .. 16384, at their compile-time plans (fft_twin.cu).
 bool twin_supported(const FftGeom& g);
 cudaError_t launch_fft_twin(const FftPlan& plan, const float2* d_in, uint32_t beams, uint32_t n_point,
                             const float* d_win, uint32_t out_mode, float scale, void* d_out,

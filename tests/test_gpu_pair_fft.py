@@ -184,7 +184,7 @@ def test_learned_topk_equals_its_three_steps(spx, nfft, beams, k):
         assert torch.equal(a, b)
 
 
-TWIN_SIZES = [n for n in (2 ** a * 3 ** b for a in range(13) for b in range(1, 9)) if 1024 < n < 8192]
+TWIN_SIZES = [n for n in (2 ** a * 3 ** b for a in range(13) for b in range(1, 9)) if 1024 < n < 16384]
 
 
 @pytest.mark.parametrize("nfft", sorted(TWIN_SIZES))
