@@ -67,7 +67,7 @@ struct BatchBeam {
 constexpr uint32_t kIdle = 0xFFFFFFFFu;
 struct BatchCta {
   uint32_t beam;  // kIdle: this CTA has no work
-  uint32_t c;     // rank within the beam's CTAs
+  uint32_t c;     // rank within the beam's CTAs (batch_rows.cuh: tile or row item)
 };
 struct BatchGeom {
   FftGeom g;
@@ -233,13 +233,15 @@ SPX_DEV uint64_t bt_scan(const Bins& bins, uint32_t start, uint32_t end, uint32_
 }
 
 // The same for a beam of batch_rows.cuh: element q of row (k1, r0), at
-// (k1 2 NP + r0) L + q, is bin rho + C R0 q, rho = k1 + C r0.  A lane owns column
+// k1 br_pitch(M) + r0 L + q, is bin rho + C R0 q, rho = k1 + C r0.  A lane owns column
 // q and walks its C R0 consecutive bins, R0 loads (256 bytes a warp) at a time;
 // the bins before and after the column come from the neighbouring columns.
 template <uint32_t R0>
-SPX_DEV uint64_t br_scan(const float2* rows, uint32_t C, uint32_t L, uint32_t start, uint32_t end, uint32_t K,
+SPX_DEV uint64_t br_scan(const float2* rows, uint32_t C, uint32_t L, uint32_t M, uint32_t start, uint32_t end, uint32_t K,
                          uint32_t lane, uint32_t warp) {
-  constexpr uint32_t NP2 = 2 * ((R0 + 1) / 2), U = R0 == 9 ? 9 : 8;
+  constexpr uint32_t U = R0 == 9 ? 9 : 8;
+  // (even R0: M = R0 L is its own pitch)
+  auto row = [=](uint32_t k1, uint32_t r0) { return R0 % 2 ? k1 * br_pitch(M) + r0 * L : (k1 * R0 + r0) * L; };
   const uint32_t CB = C * R0, q_lo = start / CB, q_hi = (end - 1) / CB;
   uint64_t mine = 0;
   // |X|^2 below which no bin's rounded square root reaches the list's K-th entry
@@ -252,7 +254,7 @@ SPX_DEV uint64_t br_scan(const float2* rows, uint32_t C, uint32_t L, uint32_t st
     const bool in = q <= q_hi;
     const float2* col = rows + q;
     float l = 0.f, c = 0.f;  // |X|^2 of bins k - 1 and k
-    if (in && q * CB >= start) l = mag2_rn(__ldg(rows + (size_t)((C - 1) * NP2 + R0 - 1) * L + q - 1));
+    if (in && q * CB >= start) l = mag2_rn(__ldg(rows + row(C - 1, R0 - 1) + q - 1));
     if (in) c = mag2_rn(__ldg(col));
     // bins of the column in the window: [klo, khi), none for lanes past the end
     const uint32_t klo = max(start, q * CB), khi = in ? min(end, (q + 1) * CB) : 0u;
@@ -266,7 +268,7 @@ SPX_DEV uint64_t br_scan(const float2* rows, uint32_t C, uint32_t L, uint32_t st
           ++r0;
         }
         z[u] = make_float2(0.f, 0.f);
-        if (in && k + u < end) z[u] = r0 < R0 ? __ldg(col + (k1 * NP2 + r0) * L) : __ldg(col + 1);
+        if (in && k + u < end) z[u] = r0 < R0 ? __ldg(col + row(k1, r0)) : __ldg(col + 1);
       }
 #pragma unroll
       for (uint32_t u = 0; u < U; ++u, ++k) {
@@ -316,17 +318,17 @@ topk_batch_kernel(const float2* __restrict__ xch, const BatchBeam* __restrict__ 
   const uint32_t C = geoms[bm.geom].g.C, M = geoms[bm.geom].g.M;
   const RowBins bins{xch + bm.spec_off, M};
   const bool br = ITEMS && geoms[bm.geom].twr != nullptr;
-  const uint32_t R0 = geoms[bm.geom].R0, L = geoms[bm.geom].L, NP = geoms[bm.geom].NP;
+  const uint32_t R0 = geoms[bm.geom].R0, L = geoms[bm.geom].L;
   const uint32_t cmagic = 0xFFFFFFFFu / C + 1u;  // k div C = umulhi(k, cmagic) (k * C < 2^32)
   auto bin = [&](uint32_t k) -> float2 {
     const uint32_t q = C == 1 ? k : __umulhi(k, cmagic), k1 = k - q * C;
-    return br ? __ldg(xch + bm.spec_off + (size_t)(k1 * 2 * NP + q % R0) * L + q / R0) : bins(k1, q);
+    return br ? __ldg(xch + bm.spec_off + (k1 * br_pitch(M) + (q % R0) * L) + q / R0) : bins(k1, q);
   };
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint64_t mine = 0;
   if (start < end && br) {  // (the same for the whole CTA)
     const float2* rows = xch + bm.spec_off;
-    mine = R0 == 9 ? br_scan<9>(rows, C, L, start, end, a.K, lane, warp) : br_scan<16>(rows, C, L, start, end, a.K, lane, warp);
+    mine = R0 == 9 ? br_scan<9>(rows, C, L, M, start, end, a.K, lane, warp) : br_scan<16>(rows, C, L, M, start, end, a.K, lane, warp);
   } else if (start < end) {
     switch (C) {  // the same for the whole CTA
       case 1: mine = bt_scan<1, kBtThreads>(bins, start, end, a.K, lane, warp); break;
@@ -420,7 +422,7 @@ __global__ void __launch_bounds__(kBrThreads, 4) batch_cols_kernel(BatchArgs a, 
   const BatchSamples ld{a.in + bm.in_off, bm.n_point, make_window_gen(a.window, bm.n_point)};
   const uint32_t M = bg->g.M, L = bg->L;
   const float2* twc = bg->twc;
-  float4* slot = reinterpret_cast<float4*>(a.xch + bm.spec_off);
+  float2* slot = a.xch + bm.spec_off;
   auto go = [&](auto c, auto r) {
     constexpr int C = decltype(c)::value, R = decltype(r)::value;
     br_cols<C, R>(s4, ld, M, L, d.c * 2 * br_hw(C, R), twc, slot);
@@ -458,8 +460,10 @@ batch_rows_kernel(BatchArgs a, const BatchCta* __restrict__ items, uint32_t star
   if (a.ahead && blockIdx.x + a.ahead < gridDim.x && threadIdx.x < 2) {  // L2 prefetch of the pairs one residency wave later
     const BatchCta f = items[blockIdx.x + a.ahead];
     const BatchBeam fb = a.beams[f.beam];
-    const uint32_t fl = a.geoms[fb.geom].L, n = (uint32_t)a.geoms[fb.geom].pairs * fl;  // elements x 2 of an item
-    prefetch_l2(a.xch + fb.spec_off + (size_t)f.c * n * 2 + threadIdx.x * n, (size_t)n * sizeof(float2), 0, 1);
+    const BatchGeom* fg = a.geoms + fb.geom;
+    const uint32_t n = fg->pairs, r0 = (2 * (f.c & 255) + threadIdx.x) * n;
+    if (r0 < fg->R0)  // half of the item's rows (an odd R0's last row is alone)
+      prefetch_l2(a.xch + fb.spec_off + ((f.c >> 8) * br_pitch(fg->g.M) + r0 * fg->L), (size_t)n * fg->L * sizeof(float2), 0, 1);
   }
   br_switch(bg->g.M, [&](auto m) {
     br_rows<decltype(m)::value>(s4, d.c, a.xch + bm.spec_off, bg->twr, qlo, qhi);
@@ -658,9 +662,9 @@ spx_status build(spx_ctx* ctx, spx_batch* b) {
     beams[i] = BatchBeam{in_off, spec_off, b->n_point[i], b->nfft[i], geom_of[b->nfft[i]], 0};
     group[i] = geoms[geom_of[b->nfft[i]]].g.C;
     in_off += b->n_point[i];
-    const BatchGeom& bg = geoms[geom_of[b->nfft[i]]];
-    const uint32_t slot = bg.twr ? bg.g.C * 2 * bg.NP * bg.L : b->nfft[i];
-    spec_off += (slot + 31u) & ~31u;  // 256-byte aligned spectra
+    // 256-byte aligned slots that hold the beam at any plan: every later choice of
+    // local sizes fits the scratch that spx_batch_create allocates
+    spec_off += (br_slot(b->nfft[i]) + 31u) & ~31u;
   }
   b->in_total = in_off;
   b->spec_total = spec_off;
@@ -706,7 +710,7 @@ spx_status build(spx_ctx* ctx, spx_batch* b) {
       const uint32_t per = geom(kv.second[0]).NP / geom(kv.second[0]).pairs;  // items per k1
       for (uint32_t i = 0; i < per; ++i)
         for (uint32_t id : kv.second)
-          for (uint32_t k1 = 0; k1 < geom(id).g.C; ++k1) rows.push_back(BatchCta{id, k1 * per + i});
+          for (uint32_t k1 = 0; k1 < geom(id).g.C; ++k1) rows.push_back(BatchCta{id, k1 << 8 | i});
     }
     for (uint32_t id : ids)
       if (!geom(id).twr) others.push_back(id);

@@ -13,11 +13,15 @@
 //     FFT over j in row coordinates whose twiddles depend on r0.
 // Rows r0 = 2i, 2i + 1 of one k1 run as a pair in packed arithmetic
 // (fft_pair.cuh): one value of each row in a register pair, so any radix and any
-// odd stride will do.  Between the launches a beam's slot holds, for k1 and i, the
-// pair's L elements as float4 {re, re, im, im}; launch 2 leaves the rows there as
-// complex values: bin k1 + C (r0 + R0 q) is element q of row (k1, r0), at
-// (k1 2 NP + r0) L + q, NP = ceil(R0 / 2) (R0 = 9: the last pair holds row 8
-// twice).
+// odd stride will do.  A beam's slot holds C blocks, one per k1, br_pitch(M)
+// elements apart.  Between the launches a block holds for i = 0, 1, ... the pair's L
+// elements as float4 {re, re, im, im}, then for R0 = 9 row 8 as complex values
+// (launch 2 runs it with zeros beside it); launch 2 leaves the rows there as complex
+// values: bin k1 + C (r0 + R0 q) is element q of row (k1, r0), at k1 br_pitch(M) +
+// r0 L + q.  A slot's length (br_slot) does not depend on the plan: a batch's scratch
+// is allocated once, and local sizes may change later.  (A whole row behind row 8,
+// so that it runs as a pair like the others: 574 us for 577 on 1024 beams of 1000 ..
+// 100000 samples, but slots of these plans a tenth longer than of others.)
 //
 // Where the last two passes multiply to 18 or less (972, 1458 and 864 points)
 // launch 2 runs them in registers, one exchange fewer (rows 0.213 -> 0.20 ms on
@@ -69,6 +73,19 @@ __host__ __device__ __forceinline__ void br_switch(uint32_t M, F&& f) {
   }
 }
 constexpr uint32_t kBrThreads = 128;
+// Elements from one k1's rows to the next one's: M up to 32-byte sectors.
+__host__ __device__ constexpr uint32_t br_pitch(uint32_t M) { return (M + 3) & ~3u; }
+// Elements of a beam's slot at whatever plan (of the local sizes only 6561 and its
+// double are no multiples of 4).
+constexpr uint32_t br_slot(uint32_t nfft) { return nfft + (nfft % 6561 == 0 ? 3 * (nfft / 6561) : 0u); }
+constexpr uint32_t kBrMaxC = 9;
+constexpr bool br_slots_fit() {
+  for (uint32_t M = 6561; M <= 16384; ++M)
+    for (uint32_t C = 2; br_size(M) && C <= kBrMaxC; ++C)
+      if (C * br_pitch(M) > br_slot(C * M)) return false;
+  return true;
+}
+static_assert(br_slots_fit(), "a slot holds its beam at every plan");
 
 // ---- windows, two samples at a time ---------------------------------------------------
 // window_at's operations (fft_core.cuh) on samples a and b, the polynomials in
@@ -147,7 +164,6 @@ struct BatchSamples {
 // ---- launch 1 ----------------------------------------------------------------------
 // Column pairs per tile: columns p and p + HW of 2 HW.
 constexpr int br_hw(int C, int R0) { return R0 == 9 ? (C <= 4 ? 32 : 16) : C == 2 ? 64 : C <= 4 ? 32 : 16; }
-constexpr uint32_t kBrMaxC = 9;
 // bytes of the largest tile (C = 9, R0 = 16) and its window values
 constexpr uint32_t kBrTile = kBrMaxC * 16 * 16 * 16, kBrColsSmem = kBrTile + kBrTile / 2;
 
@@ -156,8 +172,8 @@ constexpr uint32_t kBrTile = kBrMaxC * 16 * 16 * 16, kBrColsSmem = kBrTile + kBr
 // unrolled into every load).
 template <int C, int R0>
 SPX_DEV void br_cols(float4* s4, const BatchSamples& load, uint32_t M, uint32_t L, uint32_t j0, const float2* __restrict__ twc,
-                     float4* __restrict__ slot) {
-  constexpr int HW = br_hw(C, R0), T = (int)kBrThreads, NI = R0 * HW, U = (NI + T - 1) / T, NP = (R0 + 1) / 2;
+                     float2* __restrict__ slot) {
+  constexpr int HW = br_hw(C, R0), T = (int)kBrThreads, NI = R0 * HW, U = (NI + T - 1) / T, NP = R0 / 2;
   static_assert(C * R0 * HW * 16 <= (int)kBrTile, "tile");
   float2* wt = reinterpret_cast<float2*>(s4 + kBrTile / 16);  // [C R0][HW]: windows of columns p, p + HW
   const uint32_t tid = threadIdx.x;
@@ -214,30 +230,36 @@ SPX_DEV void br_cols(float4* s4, const BatchSamples& load, uint32_t M, uint32_t 
 #pragma unroll 1
   for (uint32_t i = tid; i < (uint32_t)(C * HW); i += T) {
     const uint32_t p = i % HW, k1 = i / HW, ja = j0 + p, jb = ja + HW;
-    C2 b[R0 + 1];
+    C2 b[R0];
 #pragma unroll
     for (int r = 0; r < R0; ++r) {
       const float4 a = s4[(k1 * R0 + r) * HW + p];
       b[r] = C2{make_float2(a.x, a.y), make_float2(a.z, a.w)};
     }
     PDft<R0>::run(b);
-    if (R0 % 2) b[R0] = b[R0 - 1];
-    float4* o = slot + (size_t)k1 * NP * L;
+    float2* block = slot + (size_t)k1 * br_pitch(M);
+    float4* o = reinterpret_cast<float4*>(block);
 #pragma unroll
     for (int q = 0; q < NP; ++q) {
       const C2 e = b[2 * q], f = b[2 * q + 1];
       if (ja < L) __stcg(o + (size_t)q * L + ja, make_float4(e.x.x, f.x.x, e.y.x, f.y.x));
       if (jb < L) __stcg(o + (size_t)q * L + jb, make_float4(e.x.y, f.x.y, e.y.y, f.y.y));
     }
+    if constexpr (R0 % 2 != 0) {
+      float2* r = block + (size_t)(R0 - 1) * L;
+      if (ja < L) __stcg(r + ja, first_of(b[R0 - 1]));
+      if (jb < L) __stcg(r + jb, second_of(b[R0 - 1]));
+    }
   }
 }
 
 // ---- launch 2 ----------------------------------------------------------------------
 // Pass P of the plan on one row pair by threads t < T: from the slots in device
-// memory (the first), else from shared memory; the last hands element q of both
-// rows to out(q, z).
+// memory (the first; `alone`: src is one row of complex values), else from shared
+// memory; the last hands element q of both rows to out(q, z).
 template <int M, int P, typename Sync, typename Out>
-SPX_DEV void br_pass(float4* s, const float4* src, const float4* __restrict__ tw, uint32_t t, const Out& out) {
+SPX_DEV void br_pass(float4* s, const float2* src, bool alone, const float4* __restrict__ tw, uint32_t t,
+                     const Out& out) {
   using PL = CtPlan<M>;
   using S = BrSize<M>;
   constexpr int T = S::T, R = PL::radix(P), Nr = PL::ns(P) / S::R0, B = S::L / R, Q = (B + T - 1) / T;
@@ -245,11 +267,19 @@ SPX_DEV void br_pass(float4* s, const float4* src, const float4* __restrict__ tw
   const float4* tp = tw + S::off(P);
   auto have = [&](int q) { return B % T == 0 || q + 1 < Q || t + q * T < (uint32_t)B; };
   auto load = [&](C2* v, uint32_t j) {
+    float4 a[R];
+    if (first && S::R0 % 2 != 0 && alone) {  // (into the register pairs themselves: a wider load's moves would wait for it)
 #pragma unroll
-    for (int r = 0; r < R; ++r) {
-      const float4 a = first ? ld_once4(src + j + r * B) : s[ps(j + r * B)];
-      v[r] = C2{make_float2(a.x, a.y), make_float2(a.z, a.w)};
+      for (int r = 0; r < R; ++r) {
+        const float* z = reinterpret_cast<const float*>(src + j + r * B);
+        a[r] = make_float4(ld_value(z), 0.f, ld_value(z + 1), 0.f);
+      }
+    } else {
+#pragma unroll
+      for (int r = 0; r < R; ++r) a[r] = first ? ld_once4(src + 2 * (j + r * B)) : s[ps(j + r * B)];
     }
+#pragma unroll
+    for (int r = 0; r < R; ++r) v[r] = C2{make_float2(a[r].x, a[r].y), make_float2(a[r].z, a[r].w)};
   };
   auto butterfly = [&](C2* v, uint32_t k) {
     if constexpr (R == 4) {
@@ -327,7 +357,7 @@ SPX_DEV void br_pass(float4* s, const float4* src, const float4* __restrict__ tw
         s[ps(base + r * Nr)] = make_float4(v[q][r].x.x, v[q][r].x.y, v[q][r].y.x, v[q][r].y.y);
     }
     Sync::wait();
-    br_pass<M, P + 1, Sync>(s, src, tw, t, out);
+    br_pass<M, P + 1, Sync>(s, src, alone, tw, t, out);
   }
 }
 
@@ -337,7 +367,7 @@ constexpr uint32_t br_slots = BrSize<M>::L + (BrSize<M>::L + 15) / 16 + 1;
 constexpr uint32_t kBrRowsSmem = 2 * (1024 + 65) * 16;  // the largest: two pairs of 1024
 static_assert(br_slots<13122> * 16 <= kBrRowsSmem && 2 * br_slots<13824> * 16 <= kBrRowsSmem, "shared memory");
 
-// Item `part` of a beam: row pair part (T = 128), or pairs 2 part, 2 part + 1.
+// Item k1 << 8 | j of a beam: row pair j of k1 (T = 128), or pairs 2 j and 2 j + 1.
 // Elements [qlo, qhi) of the rows are left in the slot.
 template <int M>
 SPX_DEV void br_rows(float4* s4, uint32_t part, float2* __restrict__ slot, const float4* __restrict__ tables,
@@ -345,16 +375,17 @@ SPX_DEV void br_rows(float4* s4, uint32_t part, float2* __restrict__ slot, const
   using S = BrSize<M>;
   constexpr uint32_t L = S::L, T = S::T;
   const uint32_t t = threadIdx.x % T, h = threadIdx.x / T;
-  const uint32_t pair = part * (kBrThreads / T) + h, i = pair % S::NP;
-  float2* rows = slot + (size_t)pair * 2 * L;  // rows 2i and 2i + 1 of k1 = pair / NP
+  const uint32_t k1 = part >> 8, i = (part & 255) * (kBrThreads / T) + h;
+  const bool alone = S::R0 % 2 != 0 && i == S::NP - 1;
+  float2* rows = slot + (size_t)k1 * br_pitch(M) + 2 * i * L;  // rows 2i and 2i + 1 of k1
   auto out = [=](uint32_t q, C2 z) {
     if (q >= qlo && q < qhi) {
       __stcg(rows + q, first_of(z));
-      __stcg(rows + L + q, second_of(z));
+      if (!alone) __stcg(rows + L + q, second_of(z));
     }
   };
   using Sync = std::conditional_t<T == kBrThreads, CtaSync, GroupSync<(int)T>>;
-  br_pass<M, 1, Sync>(s4 + h * br_slots<M>, reinterpret_cast<const float4*>(rows), tables + i * S::entries, t, out);
+  br_pass<M, 1, Sync>(s4 + h * br_slots<M>, rows, alone, tables + i * S::entries, t, out);
 }
 
 }  // namespace spx

@@ -279,6 +279,11 @@ SPX_DEV float4 ld_once4(const void* p) {
                : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p) : "memory");
   return v;
 }
+SPX_DEV float ld_value(const float* p) {
+  float v;
+  asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p) : "memory");
+  return v;
+}
 
 // Two table values (volatile: issued where it stands).
 SPX_DEV float2 ld_table2(const float* p) {
