@@ -638,14 +638,22 @@ spx_status build(spx_ctx* ctx, spx_batch* b) {
     geom_of[kv.first] = (uint32_t)geoms.size();
     BatchGeom bg{plan->g, plan->d_tw_local, plan->d_tw_cross, nullptr, 0, 0, 0, 0};
     if (item_points >= kBrMinPoints && plan->g.ept == 16 && by_items(kv.first, plan->g.M)) {
-      float4*& table = ctx->batch_tables[plan->g.M];
-      if (!table) {
+      float4* table = nullptr;
+      const auto known = ctx->batch_tables.find(plan->g.M);
+      if (known != ctx->batch_tables.end()) {
+        table = known->second;
+      } else {
         std::vector<float2> twl(plan->g.M);
         fill_local_twiddles(plan->g, twl.data());
         const std::vector<float4> t = br_tables(plan->g, twl.data());
         cudaError_t e = cudaMalloc(&table, t.size() * sizeof(float4));
-        if (e == cudaSuccess) e = cudaMemcpy(table, t.data(), t.size() * sizeof(float4), cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "batch row twiddles");
+        e = cudaMemcpy(table, t.data(), t.size() * sizeof(float4), cudaMemcpyHostToDevice);
+        if (e != cudaSuccess) {  // the context keeps complete tables only
+          cudaFree(table);
+          return cuda_fail(ctx, e, "batch row twiddles");
+        }
+        ctx->batch_tables[plan->g.M] = table;
       }
       bg.twr = table;
       bg.R0 = plan->g.radix[0];
