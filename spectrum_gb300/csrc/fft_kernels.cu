@@ -366,11 +366,12 @@ spx_status get_plan(spx_ctx* ctx, uint32_t nfft, const FftPlan** out) {
 }
 
 // The window table of one (window, n_point): w[n] = window_at(n) (fft_core.cuh),
-// the evaluation the uneven batch makes per sample.
+// the evaluation the uneven batch makes per sample, and a zero behind the last
+// (the packed kernels read values in pairs).
 __global__ void window_table_kernel(uint32_t window, uint32_t n_point, float* __restrict__ w) {
   const WindowGen g = make_window_gen(window, n_point);
-  for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n < n_point; n += gridDim.x * blockDim.x)
-    w[n] = window_at(g, n);
+  for (uint32_t n = blockIdx.x * blockDim.x + threadIdx.x; n <= n_point; n += gridDim.x * blockDim.x)
+    w[n] = n < n_point ? window_at(g, n) : 0.f;
 }
 
 spx_status get_window(spx_ctx* ctx, uint32_t window, uint32_t n_point, const float** out) {
@@ -387,7 +388,7 @@ spx_status get_window(spx_ctx* ctx, uint32_t window, uint32_t n_point, const flo
     return SPX_OK;
   }
   float* d = nullptr;
-  cudaError_t e = cudaMalloc(&d, std::max<size_t>(1, n_point) * sizeof(float));
+  cudaError_t e = cudaMalloc(&d, ((size_t)n_point + 1) * sizeof(float));
   if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(window)");
   const uint32_t blocks = std::min<uint32_t>((n_point + 255) / 256, 4096);
   window_table_kernel<<<std::max(blocks, 1u), 256, 0, ctx->stream>>>(window, n_point, d);
