@@ -1148,7 +1148,15 @@ spx_status launch_maxima_cluster(spx_ctx* ctx, const float2* d_spec, uint32_t C1
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;  // as launch_dependent
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = after_rows ? 2 : 1;
+  // Beside the end of the rows kernel (attr[1]) where that was faster: thresholded
+  // searches of few CTAs (8 x 131072 bins 43.5 -> 40.4 us a call) or of all the SMs
+  // hold (256 x 131072 from half as many samples 198 -> 196).  In between the CTAs
+  // pack onto the SMs that fall free first and leave the others idle (42 x 98304 51
+  // -> 53), and without a threshold one CTA of a beam writes most of its records
+  // (85 x 49152 59 -> 72; from 2^25 points on within 1 % either way, or 3 % slower).
+  const uint32_t ctas = beams * C2, sms = (uint32_t)ctx->sm_count;
+  const bool beside = after_rows && factor > 0.0f && (ctas <= sms / 2 || ctas >= sms * (rows ? 4 : kMxMinBlocks));
+  cfg.numAttrs = beside ? 2 : 1;
   void* args[] = {(void*)&a};
   e = cudaLaunchKernelExC(&cfg, kfn, args);
   if (e != cudaSuccess) return cuda_fail(ctx, e, "launch maxima_cluster_kernel");

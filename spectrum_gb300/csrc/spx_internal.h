@@ -226,7 +226,7 @@ spx_status launch_maxima_cluster(spx_ctx* ctx, const float2* d_spec, uint32_t C1
                                  uint32_t beams, uint32_t nfft, uint32_t start, uint32_t end,
                                  uint32_t cap, float fs, uint32_t refine, float factor,
                                  uint32_t* d_ccount, spx_max_value* d_out, uint32_t* d_counts,
-                                 bool after_rows = false);  // true: launched beside the rows kernel's end
+                                 bool after_rows = false);  // true: d_spec is written by the launch before, a rows kernel
 
 // Kernel launchers (fft_kernels.cu, peak_kernels.cu).
 spx_status launch_fft_out(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
