@@ -1214,13 +1214,30 @@ spx_status launch_fft_peaks(spx_ctx* ctx, const FftPlan& plan, const float2* d_i
   // the cluster transform: 49152 0.305 -> 0.262 ms, 98304 0.314 -> 0.250, 147456
   // 0.351 -> 0.267, 196608 0.481 -> 0.274
   if (plan.d_tw_rows && !mx_rows(16 * g.C)) {
-    void *spec = nullptr, *cnt = nullptr;
-    spx_status st = get_scratch(ctx, kSlotSpectrum, (size_t)beams * g.nfft * sizeof(float2), &spec);
-    if (st == SPX_OK) st = get_scratch(ctx, kSlotWork, (size_t)beams * kMxMaxC2 * sizeof(uint32_t), &cnt);
-    if (st == SPX_OK) st = launch_fft_mid(ctx, plan, d_in, beams, n_point, d_win, SPX_OUT_COMPLEX, 1.0f, spec);
-    if (st != SPX_OK) return st;
-    return launch_maxima_cluster(ctx, static_cast<float2*>(spec), 1, g.nfft, beams, g.nfft, start, end, cap_or_k, fs,
-                                 refine, factor, static_cast<uint32_t*>(cnt), d_out, d_counts, true);
+    // Two buffers of a spectrum each, where the cluster transform needs one: out of
+    // memory, the call runs in parts whose buffers hold no more than that (in halves
+    // always: 341 x 98304 275 -> 297 us).
+    const size_t beam_bytes = (size_t)g.nfft * sizeof(float2);
+    uint32_t group = beams;
+    void *spec = nullptr, *xch = nullptr, *cnt = nullptr;
+    spx_status st;
+    for (;; group = (group + 1) / 2) {
+      st = get_scratch(ctx, kSlotWork, (size_t)group * kMxMaxC2 * sizeof(uint32_t), &cnt);
+      if (st == SPX_OK) st = get_scratch(ctx, kSlotSpectrum, group * beam_bytes, &spec);
+      if (st == SPX_OK) st = get_scratch(ctx, kSlotExchange, group * beam_bytes, &xch);
+      if (st != SPX_ERR_OUT_OF_MEMORY || group == 1) break;
+      free_scratch(ctx, kSlotSpectrum);
+      free_scratch(ctx, kSlotExchange);
+    }
+    for (uint32_t b = 0; b < beams && st == SPX_OK; b += group) {
+      const uint32_t n = std::min(group, beams - b);
+      st = launch_fft_mid(ctx, plan, d_in + (size_t)b * n_point, n, n_point, d_win, SPX_OUT_COMPLEX, 1.0f, spec);
+      if (st == SPX_OK)
+        st = launch_maxima_cluster(ctx, static_cast<float2*>(spec), 1, g.nfft, n, g.nfft, start, end, cap_or_k, fs,
+                                   refine, factor, static_cast<uint32_t*>(cnt), d_out + (size_t)b * cap_or_k,
+                                   d_counts + b, true);
+    }
+    return st;
   }
   if (plan.d_tw_rows) {  // spectrum rows over the exchange scratch, then the maxima kernel
     const size_t row_bytes = (size_t)beams * g.nfft * sizeof(float2);

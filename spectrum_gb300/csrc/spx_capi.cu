@@ -24,14 +24,17 @@ spx_status cuda_fail(spx_ctx* ctx, cudaError_t e, const char* what) {
                            cudaGetErrorString(e) + ")");
 }
 
+void free_scratch(spx_ctx* ctx, int slot) {
+  if (!ctx->d_scratch[slot]) return;
+  cudaFree(ctx->d_scratch[slot]);
+  ctx->d_scratch[slot] = nullptr;
+  ctx->scratch_bytes[slot] = 0;
+}
+
 spx_status get_scratch(spx_ctx* ctx, int slot, size_t bytes, void** out) {
   if (bytes == 0) bytes = 256;
   if (ctx->scratch_bytes[slot] < bytes) {
-    if (ctx->d_scratch[slot]) {
-      cudaFree(ctx->d_scratch[slot]);
-      ctx->d_scratch[slot] = nullptr;
-      ctx->scratch_bytes[slot] = 0;
-    }
+    free_scratch(ctx, slot);
     size_t sz = bytes + bytes / 4;  // headroom so slowly growing sizes do not thrash
     cudaError_t e = cudaMalloc(&ctx->d_scratch[slot], sz);
     if (e != cudaSuccess) {

@@ -101,6 +101,7 @@ constexpr int kSlots = 6;
 // Ensures at least `bytes` in `slot`; returns its device pointer.  Growing a
 // slot frees the old buffer (cudaFree waits for the device first).
 spx_status get_scratch(spx_ctx* ctx, int slot, size_t bytes, void** out);
+void free_scratch(spx_ctx* ctx, int slot);
 
 // Raises a kernel's dynamic shared-memory limit (and allows clusters of
 // up to 16) once per (device, kernel).
