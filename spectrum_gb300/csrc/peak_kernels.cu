@@ -450,7 +450,10 @@ topk_kernel(const float* __restrict__ mag, const float2* __restrict__ fft, uint3
       }
     }
   }
-  mine = merge_warp_lists(&lists[0][0], mine, kTkWarps, K, warp, lane);
+  // the lists of the warps that had a bin to look at (top-5 of 131072 spectra of 256
+  // bins: 551 -> 187 us, of 32768 of 1024: 172 -> 158)
+  const uint32_t bins = end > start ? end - start : 0u;
+  mine = merge_warp_lists(&lists[0][0], mine, min(kTkWarps, (bins + 32 * kTkRun - 1) / (32 * kTkRun)), K, warp, lane);
   if (warp != 0) return;
   const uint32_t n = __popc(__ballot_sync(0xffffffffu, lane < K && mine != 0));
   if (lane == 0) counts[beam] = n;
