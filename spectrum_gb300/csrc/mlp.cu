@@ -58,6 +58,7 @@ constexpr int kTile = 32, kTp = kTile + 4;  // rows per tile; row pitch of [unit
 constexpr int kWp = kH + 4;                 // row pitch of W2
 constexpr int kW1p = 12;                    // row pitch of W1
 constexpr uint32_t kMaxTileCtas = 304;      // two per SM
+constexpr uint32_t kChain = 16;             // tiles (512 rows) added up in one FP32 chain
 constexpr uint32_t kPart = kNParams + 2;    // floats of a partial sum: gradients, loss, padding
 
 struct TileSmem {
@@ -108,7 +109,9 @@ mlp_tile_kernel(TileArgs a) {
   auto f4 = [](const float* p) { return *reinterpret_cast<const float4*>(p); };
   const uint32_t r4 = 4 * (tid & 7), up = tid >> 3;  // four rows, two units of the layers
   const uint32_t to = tid & 15, ti = tid >> 4;       // W2 gradient: units to + 16 j, inputs ti + 16 k
-  float gw2[4][4] = {}, gw1[3] = {}, gw3 = 0.f, loss = 0.f;
+  // sums of up to kChain tiles, and of those sums
+  float gw2[4][4] = {}, gw1[3] = {}, gw3 = 0.f, sw2[4][4] = {}, sw1[3] = {}, sw3 = 0.f, loss = 0.f;
+  uint32_t chain = 0;
   const uint32_t tiles = (a.rows + kTile - 1) / kTile;
 #pragma unroll 1
   for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
@@ -238,6 +241,23 @@ mlp_tile_kernel(TileArgs a) {
           gw1[e] = dot4(f4(s.g1 + o * kTp + r), i < (uint32_t)kIn ? f4(s.x + i * kTp + r) : make_float4(1.f, 1.f, 1.f, 1.f),
                         gw1[e]);
       }
+      if (++chain == kChain) {
+        chain = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            sw2[j][k] += gw2[j][k];
+            gw2[j][k] = 0.f;
+          }
+#pragma unroll
+        for (int e = 0; e < 3; ++e) {
+          sw1[e] += gw1[e];
+          gw1[e] = 0.f;
+        }
+        sw3 += gw3;
+        gw3 = 0.f;
+      }
     }
     __syncthreads();  // the tile's arrays are rewritten by the next one
   }
@@ -246,13 +266,14 @@ mlp_tile_kernel(TileArgs a) {
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int k = 0; k < 4; ++k) g[kOffW2 + (to + 16 * j) * kH + ti + 16 * k] = gw2[j][k];
+      for (int k = 0; k < 4; ++k) g[kOffW2 + (to + 16 * j) * kH + ti + 16 * k] = sw2[j][k] + gw2[j][k];
 #pragma unroll
     for (int e = 0; e < 3; ++e) {
       const uint32_t i = (tid + 256 * e) / kH, o = tid % kH;
-      if (i < (uint32_t)kIn) g[kOffW1 + o * kIn + i] = gw1[e];
-      if (i == (uint32_t)kIn) g[kOffB1 + o] = gw1[e];
+      if (i < (uint32_t)kIn) g[kOffW1 + o * kIn + i] = sw1[e] + gw1[e];
+      if (i == (uint32_t)kIn) g[kOffB1 + o] = sw1[e] + gw1[e];
     }
+    gw3 += sw3;
     if (tid < kOut * kH) g[kOffW3 + tid] = gw3;
     else if (tid < kOut * kH + kH) g[kOffB2 + tid - kOut * kH] = gw3;
     else if (tid < kOut * kH + kH + kOut) g[kOffB3 + tid - kOut * kH - kH] = gw3;
