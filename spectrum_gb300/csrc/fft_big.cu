@@ -120,7 +120,7 @@ big_rows_kernel(FftGeom g, const float4* __restrict__ tw_pair, float2* __restric
   if (g.ahead && blockIdx.x + g.ahead < gridDim.x)  // the row the CTA one wave later reads
     prefetch_l2(row + (size_t)g.ahead * g.M, (size_t)g.M * sizeof(float2), tid, 512);
   // the row is read by this CTA alone (first pass, before its barrier)
-  pair_local_fft_out<(int)kBigM>(s4, ExchangePairs{row}, tw_pair, tid, RowOutPairs{row});
+  pair_local_fft_out<(int)kBigM>(s4, ExchangePairs<>{row}, tw_pair, tid, RowOutPairs{row});
 }
 
 // Four rows k1 = r0 .. r0+3 of 4096 points per CTA in packed arithmetic
@@ -137,7 +137,7 @@ constexpr int kBigComplex = 0, kBigMag = 1, kBigMagPhase = 2, kBigOther = 3;
 template <int MODE>
 __global__ void __launch_bounds__(kRows4 * 128, 1)
 big_rows4_kernel(FftGeom g, const float4* __restrict__ tw_pair, const float2* cols,
-                 void* __restrict__ out, uint32_t out_mode, float scale) {
+                 void* __restrict__ out, uint32_t out_mode, float scale, bool last) {
   extern __shared__ float4 s4[];
   constexpr int TG = 128, M = (int)kBigM4;
   const uint32_t tid = threadIdx.x, grp = tid / TG;
@@ -151,7 +151,10 @@ big_rows4_kernel(FftGeom g, const float4* __restrict__ tw_pair, const float2* co
     prefetch_l2(scratch + (size_t)(blockIdx.x + g.ahead) * (kRows4 * kBigM4), kRows4 * kBigM4 * sizeof(float2), tid,
                 kRows4 * TG);
   float4* s = s4 + grp * kRowPitch4;
-  pair_first<M, TG, GroupSync<TG>>(s, ExchangePairs{row}, tid - grp * TG);
+  if (last)
+    pair_first<M, TG, GroupSync<TG>>(s, ExchangePairs<true>{row}, tid - grp * TG);
+  else
+    pair_first<M, TG, GroupSync<TG>>(s, ExchangePairs<>{row}, tid - grp * TG);
   pair_passes_until_last<M, 1, TG, GroupSync<TG>>(s, tw_pair, tid - grp * TG);
   __syncthreads();
   const uint32_t q = tid % kRows4, k1 = r0 + q;
@@ -265,7 +268,13 @@ spx_status launch_fft_big(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
     if (e != cudaSuccess) return cuda_fail(ctx, e, "configure big_rows4_kernel");
     gg.ahead = ctx->input_on_host ? 0u : resident_ctas(kfn, kRows4 * 128, smem, 1);
     const float2* scr_c = scratch;
-    void* args[] = {(void*)&gg, (void*)&twp, (void*)&scr_c, (void*)&d_out, (void*)&out_mode, (void*)&scale};
+    // While the scratch and the spectrum fit L2 together (129 MB), the scratch leaves
+    // it as it is read: else the spectrum is driven out, and a search behind the
+    // transform is slower (top-5 of 8 x 2^20 points 565 -> 478 us, of 16 x 2^19 320 ->
+    // 274; complex spectra alone 74.5 -> 73.5).  From 96 MB of scratch on, 1 .. 5 %
+    // slower that way.
+    const bool last = (size_t)beams * g.nfft * sizeof(float2) <= (64u << 20);
+    void* args[] = {(void*)&gg, (void*)&twp, (void*)&scr_c, (void*)&d_out, (void*)&out_mode, (void*)&scale, (void*)&last};
     e = launch_dependent(kfn, dim3(beams * (g.C / kRows4)), dim3(kRows4 * 128), args, smem, ctx->stream);
     return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch big_rows4_kernel");
   }

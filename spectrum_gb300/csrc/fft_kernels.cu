@@ -143,7 +143,7 @@ fft_group_out_kernel(const float2* __restrict__ in, uint32_t n_point, const floa
     // row c was read by this CTA alone: it takes the CTA's spectrum row
     // (row[i] = X[c + C*i]) from the last pass's registers;
     // rows_transpose_kernel writes the output
-    pair_local_fft_out<M>(s4, ExchangePairs{row}, tw_pair, tid, RowOutPairs{row});
+    pair_local_fft_out<M>(s4, ExchangePairs<>{row}, tw_pair, tid, RowOutPairs{row});
   }  // (the next beam's group barrier orders these reads of s4 before its local FFT)
 }
 

@@ -391,14 +391,17 @@ struct ChirpPairs {
 };
 
 // Elements n, n + 1 of a row written earlier by other CTAs (exchange slots):
-// L2-coherent 16-byte loads (rows start on 16-byte boundaries).
+// L2-coherent 16-byte loads (rows start on 16-byte boundaries).  LAST: no one reads
+// the row again, and it leaves the L2 first.
+template <bool LAST = false>
 struct ExchangePairs {
   const float2* row;
   template <int R>
   SPX_DEV void load(C2 (&v)[R], uint32_t n0, uint32_t step) const {
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      const float4 a = __ldcg(reinterpret_cast<const float4*>(row + n0 + r * step));
+      const float4* p = reinterpret_cast<const float4*>(row + n0 + r * step);
+      const float4 a = LAST ? __ldcs(p) : __ldcg(p);
       v[r] = C2{make_float2(a.x, a.z), make_float2(a.y, a.w)};
     }
   }

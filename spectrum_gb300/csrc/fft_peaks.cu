@@ -461,7 +461,7 @@ fft_group_kernel(FftGeom g, FusedArgs a, uint32_t groups) {
     // the last pass writes the window's bins of the row straight from its
     // registers (no store to shared memory, barrier and reload)
     const WindowRows w = window_rows(g, c, a.start, a.end);
-    pair_local_fft_out<M>(s4, ExchangePairs{row}, a.tw_pair, tid, WindowRowOutPairs{row, w});
+    pair_local_fft_out<M>(s4, ExchangePairs<>{row}, a.tw_pair, tid, WindowRowOutPairs{row, w});
     discard_outside_window(row, g, w, tid, T);
   }  // (the next beam's group_arrive barrier orders these reads of s4 before its first pass)
 }
