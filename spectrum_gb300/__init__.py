@@ -259,7 +259,7 @@ def fft_peaks(x, nfft: int, window: int = WINDOW_NONE, mode: int = PEAK_ALL,
     """Raw samples [beams, n_point] -> peaks in one call (layouts as the peak functions)."""
     torch = _torch()
     _require_cuda(x, torch.complex64, "x")
-    x2 = x if x.dim() == 2 else x.reshape(-1, x.shape[-1])
+    x2 = x if x.dim() == 2 and x.shape[1] else x.reshape(-1, x.shape[-1])
     beams, n_point = x2.shape
     # every row of ONE / TWO and every count of ALL / TOPK is written by the search
     if mode in (PEAK_ONE, PEAK_TWO):
