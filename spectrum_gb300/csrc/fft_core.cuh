@@ -472,7 +472,7 @@ struct CtPlan {
   static constexpr int pad(int p) { return p == 1 && radix(0) % 2 == 0 ? 1 : 0; }
 };
 
-// Barriers of a local FFT: the whole CTA's, or one group of N consecutive
+// Barriers of the packed passes: the whole CTA's, or one group of N consecutive
 // threads' (N a multiple of 32; groups of one CTA use different hardware
 // barriers, 1 + their number).
 struct CtaSync {
@@ -484,7 +484,7 @@ struct GroupSync {
 };
 
 // First pass (Ns = 1) from `load`, results into shared memory.
-template <int M, int T = CtPlan<M>::T, typename Sync = CtaSync, typename Load>
+template <int M, int T = CtPlan<M>::T, typename Load>
 SPX_DEV void ct_first(float2* s, const Load& load, uint32_t tid) {
   using P = CtPlan<M>;
   constexpr int R = P::radix(0), B = M / R, Q = (B + T - 1) / T;
@@ -510,13 +510,13 @@ SPX_DEV void ct_first(float2* s, const Load& load, uint32_t tid) {
       }
     }
   }
-  Sync::wait();
+  __syncthreads();
 }
 
 // Pass P >= 1 in shared memory.  The last pass (Ns = M / R = B) writes each
 // butterfly's outputs to the elements it read (base = j), so it needs no
 // barrier between its loads and its stores.
-template <int M, int P, int T, typename Sync = CtaSync>
+template <int M, int P, int T>
 SPX_DEV void ct_pass(float2* s, const float2* __restrict__ tw, uint32_t tid) {
   using PL = CtPlan<M>;
   constexpr int R = PL::radix(P), Ns = PL::ns(P), B = M / R, Q = (B + T - 1) / T;
@@ -536,7 +536,7 @@ SPX_DEV void ct_pass(float2* s, const float2* __restrict__ tw, uint32_t tid) {
       }
     }
   }
-  if constexpr (P + 1 < PL::npass) Sync::wait();
+  if constexpr (P + 1 < PL::npass) __syncthreads();
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
     const uint32_t j = tid + q * T;
@@ -563,14 +563,14 @@ SPX_DEV void ct_pass(float2* s, const float2* __restrict__ tw, uint32_t tid) {
       }
     }
   }
-  Sync::wait();
+  __syncthreads();
 }
 
-template <int M, int P, int T, typename Sync = CtaSync>
+template <int M, int P, int T>
 SPX_DEV void ct_passes_from(float2* s, const float2* __restrict__ tw, uint32_t tid) {
   if constexpr (P < CtPlan<M>::npass) {
-    ct_pass<M, P, T, Sync>(s, tw, tid);
-    ct_passes_from<M, P + 1, T, Sync>(s, tw, tid);
+    ct_pass<M, P, T>(s, tw, tid);
+    ct_passes_from<M, P + 1, T>(s, tw, tid);
   }
 }
 
@@ -627,12 +627,12 @@ SPX_DEV void ct_passes_until_last(float2* s, const float2* __restrict__ tw, uint
   }
 }
 
-// Whole local FFT of M points (first pass from `load`) by T threads (a CTA,
-// or a group of one with its own barrier), ending with a barrier.
-template <int M, int T = CtPlan<M>::T, typename Sync = CtaSync, typename Load>
+// Whole local FFT of M points (first pass from `load`) by a CTA of T threads,
+// ending with a barrier.
+template <int M, int T = CtPlan<M>::T, typename Load>
 SPX_DEV void ct_local_fft(float2* s, const Load& load, const float2* __restrict__ tw, uint32_t tid) {
-  ct_first<M, T, Sync>(s, load, tid);
-  ct_passes_from<M, 1, T, Sync>(s, tw, tid);
+  ct_first<M, T>(s, load, tid);
+  ct_passes_from<M, 1, T>(s, tw, tid);
 }
 
 // The local FFT of ct_local_fft with the last pass's outputs handed to
@@ -677,7 +677,9 @@ SPX_DEV bool ct_menu_fft(uint32_t M, float2* s, const Load& load, const float2* 
     case 13122: ct_local_fft_ool<13122, T ? T : CtPlan<13122>::T>(s, load, tw, tid, out); return true;
     case 13824: ct_local_fft_ool<13824, T ? T : CtPlan<13824>::T>(s, load, tw, tid, out); return true;
     case 15552: ct_local_fft_ool<15552, T ? T : CtPlan<15552>::T>(s, load, tw, tid, out); return true;
-    case 16384: ct_local_fft_ool<16384, T ? T : CtPlan<16384>::T>(s, load, tw, tid, out); return true;
+    case 16384:  // (fft_mid.cu takes the others' C x 16384 points)
+      if constexpr (T != 0) ct_local_fft_ool<16384, T>(s, load, tw, tid, out);
+      return T != 0;
     default: return false;
   }
 }

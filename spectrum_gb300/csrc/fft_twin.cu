@@ -13,7 +13,7 @@
 // -> 200, {|X|, phase} 306 -> 263; about 340 beams 21 .. 24 -> 17 .. 19.  Bound by
 // the one or two CTAs an SM holds above 4096 points (128 KB of slots and the
 // register file), by issue below.  Pairing alone gave a tenth; the rest came with
-// the layout of TwinPlan, which needs no index computation per element.
+// the layout of CtPlan's blocks, which needs no index computation per element.
 #include <algorithm>
 
 #include "fft_core.cuh"
@@ -56,23 +56,15 @@ struct TwinSamples {
   }
 };
 
-// The slots between pass P - 1 and pass P: blocks of ns(P) elements, one unused
-// slot after each behind a first pass of even radix, whose outputs would else
-// meet in one bank.  Both passes then reach their elements by constant offsets
-// (the layout of every 16th element padded costs these plans' strides an index
-// computation per element).
-template <int M>
-struct TwinPlan : CtPlan<M> {
-  using C = CtPlan<M>;
-  static constexpr int pad(int p) { return p == 1 && C::radix(0) % 2 == 0 ? 1 : 0; }
-  static constexpr int slots = M + pad(1) * (M / C::radix(0));
-};
+// The slots between pass P - 1 and pass P lie in CtPlan's blocks: blocks of ns(P)
+// elements, one unused slot (CtPlan::pad) after each behind a first pass of even
+// radix, whose outputs would else meet in one bank.
 SPX_DEV void twin_put(float4* s, C2 z) { *s = make_float4(z.x.x, z.x.y, z.y.x, z.y.y); }
 
 // ct_first, ct_pass and ct_last_pass_out on pairs.
 template <int M>
 SPX_DEV void twin_first(float4* s, const TwinSamples& load, uint32_t tid) {
-  using P = TwinPlan<M>;
+  using P = CtPlan<M>;
   constexpr int R = P::radix(0), B = M / R, T = P::T, Q = (B + T - 1) / T;
 #pragma unroll
   for (int q = 0; q < Q; ++q) {
@@ -89,7 +81,7 @@ SPX_DEV void twin_first(float4* s, const TwinSamples& load, uint32_t tid) {
 }
 template <int M, int P, typename Out>
 SPX_DEV void twin_pass(float4* s, const float2* __restrict__ tw, uint32_t tid, const Out& out) {
-  using PL = TwinPlan<M>;
+  using PL = CtPlan<M>;
   constexpr int R = PL::radix(P), Ns = PL::ns(P), B = M / R, T = PL::T, Q = (B + T - 1) / T;
   constexpr bool last = P + 1 == PL::npass;
   C2 v[Q][R];
@@ -239,7 +231,7 @@ cudaError_t launch_fft_twin(const FftPlan& plan, const float2* d_in, uint32_t be
   const uint32_t threads = ((g.M + 15) / 16 + 31) / 32 * 32;
   const uint32_t per_cta = g.M > 8192 ? 1 : 2;
   const size_t smem = per_cta == 1 ? (size_t)sw_len(g.M) * sizeof(float2)
-                                   : (size_t)(g.M + (g.radix[0] % 2 == 0 ? g.M / g.radix[0] : 0)) * sizeof(float4);  // TwinPlan::slots
+                                   : (size_t)(g.M + (g.radix[0] % 2 == 0 ? g.M / g.radix[0] : 0)) * sizeof(float4);
   cudaError_t e = configure_kernel(kfn, smem);
   if (e != cudaSuccess) return e;
   g.beams = beams;
