@@ -132,12 +132,12 @@ big_rows_kernel(FftGeom g, const float4* __restrict__ tw_pair, float2* __restric
 // in slots: the four lanes of one element and two neighbouring slots of each
 // hit eight different 16-byte banks.
 constexpr uint32_t kRowPitch4 = ps_len(kBigM4) + 2;
-constexpr int kBigComplex = 0, kBigMag = 1, kBigMagPhase = 2, kBigOther = 3;
+constexpr int kBigComplex = 0, kBigMag = 1, kBigMagPhase = 2, kBigOther = 3, kBigReversed = 4, kBigHalf = 5;
 
-template <int MODE>
+template <int MODE, bool LAST = false>
 __global__ void __launch_bounds__(kRows4 * 128, 1)
 big_rows4_kernel(FftGeom g, const float4* __restrict__ tw_pair, const float2* cols,
-                 void* __restrict__ out, uint32_t out_mode, float scale, bool last) {
+                 void* __restrict__ out, uint32_t out_mode, float scale) {
   extern __shared__ float4 s4[];
   constexpr int TG = 128, M = (int)kBigM4;
   const uint32_t tid = threadIdx.x, grp = tid / TG;
@@ -151,28 +151,19 @@ big_rows4_kernel(FftGeom g, const float4* __restrict__ tw_pair, const float2* co
     prefetch_l2(scratch + (size_t)(blockIdx.x + g.ahead) * (kRows4 * kBigM4), kRows4 * kBigM4 * sizeof(float2), tid,
                 kRows4 * TG);
   float4* s = s4 + grp * kRowPitch4;
-  if (last)
-    pair_first<M, TG, GroupSync<TG>>(s, ExchangePairs<true>{row}, tid - grp * TG);
-  else
-    pair_first<M, TG, GroupSync<TG>>(s, ExchangePairs<>{row}, tid - grp * TG);
+  pair_first<M, TG, GroupSync<TG>>(s, ExchangePairs<LAST>{row}, tid - grp * TG);
   pair_passes_until_last<M, 1, TG, GroupSync<TG>>(s, tw_pair, tid - grp * TG);
   __syncthreads();
   const uint32_t q = tid % kRows4, k1 = r0 + q;
   float4* sq = s4 + q * kRowPitch4;
-  if constexpr (MODE == kBigOther || MODE == kBigMagPhase) {
-    // through shared memory: the last pass's registers leave no room for the
-    // long output functions
+  if constexpr (MODE == kBigOther) {
+    // mirrored real-input spectra: through shared memory, the general output
+    // function having no room beside the last pass's registers
     pair_last<M, TG>(sq, tw_pair, tid / kRows4, SlotOut{sq});
     __syncthreads();
 #pragma unroll 4
     for (uint32_t p = tid / kRows4; p < kBigM4 / 2; p += TG) {
       const float4 z = sq[ps(p)];
-      if constexpr (MODE == kBigMagPhase) {
-        float2* o = reinterpret_cast<float2*>(out) + (size_t)beam * g.nfft + k1 + (size_t)g.C * (2 * p);
-        o[0] = make_float2(mag_rn(make_float2(z.x, z.z)), atan2f(z.z, z.x));
-        o[g.C] = make_float2(mag_rn(make_float2(z.y, z.w)), atan2f(z.w, z.y));
-        continue;
-      }
       store_bin(out, out_mode, scale, g, beam, k1 + g.C * (2 * p), make_float2(z.x, z.z));
       store_bin(out, out_mode, scale, g, beam, k1 + g.C * (2 * p + 1), make_float2(z.y, z.w));
     }
@@ -183,6 +174,24 @@ big_rows4_kernel(FftGeom g, const float4* __restrict__ tw_pair, const float2* co
       if constexpr (MODE == kBigComplex) {
         reinterpret_cast<float2*>(out)[at] = a;
         reinterpret_cast<float2*>(out)[at + g.C] = b;
+      } else if constexpr (MODE == kBigMagPhase) {
+        // one phase after another: their registers would not fit side by side (through
+        // shared memory instead, 64 x 2^19 points 270 us for 263)
+        float2* o = reinterpret_cast<float2*>(out) + at;
+        o[0] = make_float2(mag_rn(a), atan2f(a.y, a.x));
+        asm volatile("" ::: "memory");
+        o[g.C] = make_float2(mag_rn(b), atan2f(b.y, b.x));
+        asm volatile("" ::: "memory");
+      } else if constexpr (MODE == kBigHalf) {
+        const uint32_t k = k1 + g.C * e, half = g.nfft / 2;
+        float2* o = reinterpret_cast<float2*>(out) + (size_t)beam * (half + 1) + k;
+        if (k <= half) o[0] = a;
+        if (k + g.C <= half) o[g.C] = b;
+      } else if constexpr (MODE == kBigReversed) {
+        const uint32_t k = k1 + g.C * e;
+        float2* o = reinterpret_cast<float2*>(out) + (size_t)beam * g.nfft;
+        o[(g.nfft - k) & (g.nfft - 1)] = make_float2(__fmul_rn(a.x, scale), __fmul_rn(a.y, scale));
+        o[g.nfft - k - g.C] = make_float2(__fmul_rn(b.x, scale), __fmul_rn(b.y, scale));
       } else {
         float* o = reinterpret_cast<float*>(out);
         const float a2 = mag2_rn(a), b2 = mag2_rn(b);
@@ -258,23 +267,26 @@ spx_status launch_fft_big(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
   FftGeom gg = g;
   gg.beams = beams;
   if (M == kBigM4) {  // four rows per CTA, bin order written directly
-    const void* kfn = out_mode == SPX_OUT_COMPLEX ? (const void*)big_rows4_kernel<kBigComplex>
+    // While the scratch and a complex spectrum fit L2 together (129 MB), the scratch
+    // leaves it as it is read: else the spectrum is driven out, and a search behind
+    // the transform is slower (top-5 of 8 x 2^20 points 565 -> 478 us, of 16 x 2^19
+    // 320 -> 274; the spectra alone 74.5 -> 73.5).  From 96 MB of scratch on, 1 .. 5 %
+    // slower that way.
+    const bool last = (size_t)beams * g.nfft * sizeof(float2) <= (64u << 20);
+    const void* kfn = out_mode == SPX_OUT_COMPLEX ? (last ? (const void*)big_rows4_kernel<kBigComplex, true>
+                                                          : (const void*)big_rows4_kernel<kBigComplex>)
                       : out_mode == SPX_OUT_MAG || out_mode == SPX_OUT_MAG2
                           ? (const void*)big_rows4_kernel<kBigMag>
-                      : out_mode == SPX_OUT_MAGPHASE ? (const void*)big_rows4_kernel<kBigMagPhase>
-                                                     : (const void*)big_rows4_kernel<kBigOther>;
+                      : out_mode == SPX_OUT_MAGPHASE    ? (const void*)big_rows4_kernel<kBigMagPhase>
+                      : out_mode == kOutComplexReversed ? (const void*)big_rows4_kernel<kBigReversed>
+                      : out_mode == kOutR2CHalf         ? (const void*)big_rows4_kernel<kBigHalf>
+                                                        : (const void*)big_rows4_kernel<kBigOther>;
     const size_t smem = (size_t)kRows4 * kRowPitch4 * sizeof(float4);
     e = configure_kernel(kfn, smem);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "configure big_rows4_kernel");
     gg.ahead = ctx->input_on_host ? 0u : resident_ctas(kfn, kRows4 * 128, smem, 1);
     const float2* scr_c = scratch;
-    // While the scratch and the spectrum fit L2 together (129 MB), the scratch leaves
-    // it as it is read: else the spectrum is driven out, and a search behind the
-    // transform is slower (top-5 of 8 x 2^20 points 565 -> 478 us, of 16 x 2^19 320 ->
-    // 274; complex spectra alone 74.5 -> 73.5).  From 96 MB of scratch on, 1 .. 5 %
-    // slower that way.
-    const bool last = (size_t)beams * g.nfft * sizeof(float2) <= (64u << 20);
-    void* args[] = {(void*)&gg, (void*)&twp, (void*)&scr_c, (void*)&d_out, (void*)&out_mode, (void*)&scale, (void*)&last};
+    void* args[] = {(void*)&gg, (void*)&twp, (void*)&scr_c, (void*)&d_out, (void*)&out_mode, (void*)&scale};
     e = launch_dependent(kfn, dim3(beams * (g.C / kRows4)), dim3(kRows4 * 128), args, smem, ctx->stream);
     return e == cudaSuccess ? SPX_OK : cuda_fail(ctx, e, "launch big_rows4_kernel");
   }
