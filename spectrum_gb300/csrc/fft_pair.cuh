@@ -298,8 +298,10 @@ SPX_DEV float2 ld_table2(const float* p) {
 // two 8-byte loads that keep the line in L1 for the second.  Window values come
 // in pairs on both paths (n is even; the table has a zero behind its last value),
 // all of them and the samples in flight before the first product: read one by one
-// between the products, 64 x 2^19 points 8 bytes off a boundary took 304 us instead
-// of 256, 8192 x 4096 points 142 instead of 100.
+// between the products, 64 x 2^19 points 8 bytes off a boundary took 297 us instead
+// of 226, 8192 x 4096 points 140 instead of 95.  The products stand once behind both
+// paths: the kernels are long and run once per CTA, and instruction fetch counts
+// (two copies: 256 x 131072 points 226 us for 214, 64 x 2^19 241 for 225).
 struct SamplePairs {
   const float2* __restrict__ x;
   uint32_t n_point;
@@ -310,9 +312,9 @@ struct SamplePairs {
   template <int R>
   SPX_DEV void load(C2 (&v)[R], uint32_t n0, uint32_t step) const {
     float4 a[R];
-    if (vec) {
-      if (win) {
-        float2 w[R];
+    if (win) {
+      float2 w[R];
+      if (vec) {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const uint32_t n = n0 + r * step;
@@ -323,38 +325,32 @@ struct SamplePairs {
             w[r] = ld_table2(win + n);
           }
         }
-#pragma unroll
-        for (int r = 0; r < R; ++r)
-          if (n0 + r * step < n_point)
-            a[r] = make_float4(__fmul_rn(a[r].x, w[r].x), __fmul_rn(a[r].y, w[r].x), __fmul_rn(a[r].z, w[r].y),
-                               __fmul_rn(a[r].w, w[r].y));
       } else {
 #pragma unroll
         for (int r = 0; r < R; ++r) {
           const uint32_t n = n0 + r * step;
-          a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (n < n_point) a[r] = ld_stream4(x + n);
+          float2 b = make_float2(0.f, 0.f), c = b;
+          w[r] = b;
+          if (n < n_point) {
+            b = ld_table2(reinterpret_cast<const float*>(x + n));
+            w[r] = ld_table2(win + n);
+          }
+          if (n + 1 < n_point) c = ld_table2(reinterpret_cast<const float*>(x + n + 1));
+          a[r] = make_float4(b.x, b.y, c.x, c.y);
         }
-      }
-    } else if (win) {
-      float2 w[R];
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        const uint32_t n = n0 + r * step;
-        float2 b = make_float2(0.f, 0.f), c = b;
-        w[r] = b;
-        if (n < n_point) {
-          b = ld_table2(reinterpret_cast<const float*>(x + n));
-          w[r] = ld_table2(win + n);
-        }
-        if (n + 1 < n_point) c = ld_table2(reinterpret_cast<const float*>(x + n + 1));
-        a[r] = make_float4(b.x, b.y, c.x, c.y);
       }
 #pragma unroll
       for (int r = 0; r < R; ++r)
         if (n0 + r * step < n_point)
           a[r] = make_float4(__fmul_rn(a[r].x, w[r].x), __fmul_rn(a[r].y, w[r].x), __fmul_rn(a[r].z, w[r].y),
                              __fmul_rn(a[r].w, w[r].y));
+    } else if (vec) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const uint32_t n = n0 + r * step;
+        a[r] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (n < n_point) a[r] = ld_stream4(x + n);
+      }
     } else {
 #pragma unroll
       for (int r = 0; r < R; ++r) {
