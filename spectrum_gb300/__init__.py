@@ -259,8 +259,9 @@ def fft_peaks(x, nfft: int, window: int = WINDOW_NONE, mode: int = PEAK_ALL,
     """Raw samples [beams, n_point] -> peaks in one call (layouts as the peak functions)."""
     torch = _torch()
     _require_cuda(x, torch.complex64, "x")
-    x2 = x if x.dim() == 2 and x.shape[1] else x.reshape(-1, x.shape[-1])
-    beams, n_point = x2.shape
+    shape = x.shape
+    x2 = x if len(shape) == 2 and shape[1] else x.reshape(-1, shape[-1])
+    beams, n_point = x2.shape if x2 is not x else shape
     # every row of ONE / TWO and every count of ALL / TOPK is written by the search
     if mode in (PEAK_ONE, PEAK_TWO):
         o = torch.empty((beams, 4 if mode == PEAK_ONE else 8, 8), dtype=torch.int32, device=x.device)
