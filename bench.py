@@ -45,15 +45,15 @@ METRIC = "Msamples/s FFT+|X|+peaks (256x65536 -> nFFT 131072, Hann, all maxima >
 # 160 beams, scaled by 256 / 160 (every beam does the same work).  NCU_TRAFFIC_KERNELS names the
 # kernels and the commit the figure was taken at, so a change of either shows
 # that it must be captured again.
-NCU_TRAFFIC_BYTES = 756_690_944
+NCU_TRAFFIC_BYTES = 753_811_866
 NCU_TRAFFIC_KERNELS = {"kernels": ["mid_cols_kernel<8>", "mid_rows_window_kernel", "maxima_cluster_kernel"],
-                       "commit": "ccf0d7c",
+                       "commit": "657d2fe",
                        "beams_captured": 160}
 # What the ncu counters of the step's kernels show bounds them (same capture
 # as NCU_TRAFFIC_BYTES): neither DRAM nor the FP32 pipe is saturated.
-NCU_LIMITER = ("load latency and the shared-memory / L1 data path: mid_cols_kernel<8> 45 % issue active, 52 % DRAM "
-               "throughput, top stall long_scoreboard; mid_rows_window_kernel 47 % issue, 49 % FMA pipe, 54 % DRAM; "
-               "maxima_cluster_kernel 48 % issue, 27 % DRAM")
+NCU_LIMITER = ("load latency and the shared-memory / L1 data path: mid_cols_kernel<8> 46 % issue active, 56 % DRAM "
+               "throughput, top stall long_scoreboard; mid_rows_window_kernel 47 % issue, 49 % FMA pipe, 55 % DRAM; "
+               "maxima_cluster_kernel 48 % issue, 26 % DRAM")
 WORKLOAD = "plain-large: 256 beams x 65536 c64, Hann, nFFT 131072, all local maxima > 6 sigma, parabolic"
 
 

@@ -170,8 +170,8 @@ uint32_t spx_next_smooth23(uint32_t n);
  * [2, 16384]: one launch, up to 262144: two; 2^19 and 2^20: two
  * launches, 2^21: three; 2^a*3^b above 2^21 up to 2^28 that split into two factors
  * <= 16384 (every power of two): four steps with transposes; any other
- * length up to 2^27: Bluestein's chirp-z transform (one launch up to 8192
- * points).  The reference takes any
+ * length up to 2^27: Bluestein's chirp-z transform (257 .. 8192 points: one
+ * launch).  The reference takes any
  * nextPow2(n_point) * repeat_count (fft_processor_rocm.cpp:673-677). */
 int spx_fft_size_supported(uint32_t nfft);
 /* Tuning for transforms of nfft points: points each thread holds per pass
@@ -274,9 +274,11 @@ spx_status spx_all_maxima_noalloc(spx_ctx* ctx, const float* d_mag, const void* 
 /* Window + zero-pad + FFT + |X| + peak search.  Power-of-two nfft
  * from 1024 to 16384 (ONE, TWO, TOPK without a threshold) and small calls of
  * other nfft <= 16384 (ALL, TOPK): one launch, the spectrum never goes to
- * device memory.  ALL with nfft > 16384: the FFT writes only the search
- * window's bins (device scratch), then one maxima launch.  Other cases:
- * spx_fft, then the peak function.
+ * device memory.  ALL with 2^a*3^b nfft from 16385 to 262144: the FFT writes
+ * only the search window's bins (over its scratch of beams x nfft complex
+ * values), then one maxima launch; for 49152, 98304, 147456 and 196608 it writes
+ * the whole spectrum into a second buffer of that size (out of memory, the call
+ * runs on parts of the beams).  Other cases: spx_fft, then the peak function.
  * params->mode selects ONE/TWO/ALL/TOPK with the layouts of
  * spx_peaks_one_two / spx_all_maxima / spx_topk.  d_counts may be NULL for
  * ONE/TWO; d_out may be NULL for ALL when the capacity is 0. */

@@ -20,8 +20,8 @@
 //   1a. batch_cols_kernel, beside it, and batch_rows_kernel (batch_rows.cuh):
 //      the beams of C x M points, C >= 2, with M one of the common local sizes
 //      (96 % of the points of lengths U[1000, 100000]), once they hold
-//      kBrMinPoints: 1024 such beams, Hann, top-8: 0.733 -> 0.564 ms
-//      (columns 0.27 ms, rows 0.20, top-K 0.09).
+//      kBrMinPoints: 1024 such beams, Hann, top-8: 0.733 -> 0.572 ms
+//      (columns 0.27 ms, rows 0.19, top-K 0.085).
 //   2. topk_batch_kernel: the K largest strict local maxima of every beam,
 //      one CTA per beam, reading bin k from row k mod C of the beam's slot (or
 //      from the rows of 1a).
@@ -502,7 +502,7 @@ std::vector<float4> br_tables(const FftGeom& g, const float2* twl) {
 // ---------------------------------------------------------------------------
 using namespace spx;
 
-struct LaunchSet {  // one FFT launch (packed CTA table, cluster size) and its top-K launch
+struct LaunchSet {  // one run's launches (packed CTA table and cluster size, items) and its top-K
   uint32_t nfft = 0;  // 0: every beam of the batch, else the beams of this nfft
   BatchCta* d_ctas = nullptr;
   uint32_t* d_beam_list = nullptr;  // the top-K launch's beams, largest spectra first

@@ -34,7 +34,7 @@
 // launch 1 by issue (42 % active; straight-line code of ~2000 instructions that
 // each CTA runs once misses the instruction caches) and its loads' latency,
 // launch 2 by the latency of its first loads and the L1's data path (57 %).
-// Five CTAs per SM (96 registers, spills) 0.564 -> 0.588 ms, not kept.
+// Five CTAs per SM (96 registers, spills) 0.564 -> 0.588 ms on the same beams, not kept.
 #pragma once
 
 #include <type_traits>

@@ -16,10 +16,10 @@
 //     room for four rows, and stride-Cb stores straight from the row kernel
 //     kept its SMs waiting on the store queue: 0.63 ms for 64 x 2^20 points).
 // Both kernels run in packed arithmetic (fft_pair.cuh).  Measured, complex
-// output: 64 x 2^20 0.581 -> 0.512 ms (columns 0.317 -> 0.263, bound by the
-// latency of their loads at 15 warps per SM; rows 0.259 -> 0.25, one CTA per
-// SM whose phases do not overlap), 64 x 2^19 0.257 -> 0.247, 16 x 2^21 0.393 ->
-// 0.358.  Not kept: 32-byte stores per thread in the row kernel (32 x 2^20
+// output: 64 x 2^20 0.581 -> 0.467 ms (columns 0.317 -> 0.221, bound by the
+// latency of their loads at 15 warps per SM; rows 0.259 -> 0.234, one CTA per
+// SM whose phases do not overlap), 64 x 2^19 0.257 -> 0.222, 16 x 2^21 0.393 ->
+// 0.342.  Not kept: 32-byte stores per thread in the row kernel (32 x 2^20
 // 0.269 -> 0.294), five column CTAs per SM (96 registers, spills: 0.305).
 // All twiddles are FP64-generated and stored in FP32, which is what the
 // 120 dB dynamic range of the precision workload needs: W_N^{n2 k1}, k1 =

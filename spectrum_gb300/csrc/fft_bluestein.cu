@@ -14,9 +14,9 @@
 // m-point transform (the library's own plan), the product with FFT_m(b) (made
 // once per plan on the device), the m-point inverse transform (the forward
 // plan with the reversing 1/m epilogue of spx_ifft), and the post-multiply
-// with the output epilogue of spx_fft (any output mode): one launch up to m =
-// 16384, four up to 262144, one per step (a few more inside the transforms)
-// beyond.  w is FP64-generated
+// with the output epilogue of spx_fft (any output mode): one launch for m = 1024
+// .. 16384, four up to 262144, one per step (a few more inside the transforms)
+// below and beyond.  w is FP64-generated
 // (n^2 reduced mod 2N exactly in integers) and stored FP32.  Error: a few
 // FP32 transforms of m points, ~1e-6 of the peak.
 #include <cmath>

@@ -46,7 +46,7 @@ fft_out_kernel(const float2* __restrict__ in, uint32_t n_point, const float* __r
 // registers (64 of them the butterflies), 16 warps per SM at every size.
 // Measured against fft_out_kernel<16> (same bits): 8192 x 4096 |X|^2 0.133 ->
 // 0.089 ms, 2048 x 16384 inverse 0.191 -> 0.153 ms; with the window loaded beside
-// the samples 8192 x 4096 0.080 ms (5.0 TB/s of input and output); 4096 x 8192
+// the samples 8192 x 4096 0.079 ms (5.1 TB/s of input and output); 4096 x 8192
 // complex 0.163 -> 0.114, inverse 0.167 -> 0.104 with the two-exchange plan
 // (0.136 before it and the window loads).  16384 points: one CTA per SM, whose
 // load, exchange and store phases do not overlap (33 % of the issue slots, 50 %
@@ -571,9 +571,9 @@ spx_status launch_fft_out(spx_ctx* ctx, const FftPlan& plan, const float2* d_in,
   }
   // C x 16384 points at the default plan: two launches of small CTAs against
   // the beam groups (C a power of two) or clusters and the transpose, 2^25
-  // points in all: 32768 0.323 -> 0.247 ms, 65536 0.324 -> 0.230, 131072 0.326 ->
-  // 0.233, 262144 0.354 -> 0.250; 49152 0.402 -> 0.229, 98304 0.407 -> 0.224, 147456
-  // 0.423 -> 0.212, 196608 0.579 -> 0.231
+  // points in all: 32768 0.323 -> 0.241 ms, 65536 0.324 -> 0.226, 131072 0.326 ->
+  // 0.214, 262144 0.354 -> 0.210; 49152 0.402 -> 0.226, 98304 0.407 -> 0.215, 147456
+  // 0.423 -> 0.204, 196608 0.579 -> 0.209
   if (plan.d_tw_rows) return launch_fft_mid(ctx, plan, d_in, beams, n_point, d_win, out_mode, scale, d_out);
   const size_t xch_bytes = ((size_t)beams * g.nfft * sizeof(float2) + 255) & ~(size_t)255;
   void* xch = nullptr;

@@ -22,11 +22,11 @@
 // shared-memory traffic).  Tiles of 4096 points leave five CTAs per SM in
 // different phases, the rows need only warp barriers, the twiddles of a row fit
 // L1, and the spectrum comes out in bin order without a transpose.
-// 256 beams of 65536 samples in 131072 bins: launch 1 0.068 ms (5.0 TB/s of
-// samples and scratch), bound by device memory; launch 2 0.066 ms (6.0 TB/s),
-// bound by the L1's data path (77 % of its wavefronts: two exchanges, twiddles,
-// loads).  In bin order launch 2 takes 0.10 ms: runs of four bins cost the L1
-// as much as the rest.
+// 256 beams of 65536 samples in 131072 bins: launch 1 0.065 ms (6.2 TB/s of
+// samples and scratch), bound by device memory and load latency; launch 2 0.066 ms
+// (6.0 TB/s), bound by the L1's data path (77 % of its wavefronts: two exchanges,
+// twiddles, loads).  In bin order launch 2 takes 0.12 ms: runs of four bins cost the
+// L1 as much as the rest.
 //
 // Replaces hipfftExecC2C's multi-pass plans
 // (src/fft_func/src/fft_processor_rocm.cpp:176-193).

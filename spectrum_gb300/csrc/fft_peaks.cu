@@ -1208,7 +1208,7 @@ spx_status launch_fft_peaks(spx_ctx* ctx, const FftPlan& plan, const float2* d_i
   }
   // power-of-two sizes at the default local size.  256 beams of 65536 points in
   // 131072 bins, 6 sigma: 0.275 ms with the beam groups (FFT 0.192, search of
-  // their rows 0.080) -> 0.205 (columns 0.068, rows 0.066, search 0.066)
+  // their rows 0.080) -> 0.193 (columns 0.065, rows 0.066, search 0.06)
   // C = 3, 6, 9, 12: the spectrum in bin order (rows of 48 .. 192 columns are not
   // what the column-by-column search takes).  All maxima of 2^25 points against
   // the cluster transform: 49152 0.305 -> 0.262 ms, 98304 0.314 -> 0.250, 147456

@@ -464,7 +464,7 @@ spx_status spx_fft_peaks_mlp(spx_ctx* ctx, spx_mlp* mlp, const void* d_in, uint3
   // also stages the network's weights and refines its peaks with one warp,
   // which pays while launch latency dominates; measured on GB300, top-1 and
   // top-8 of 1 .. 256 beams of 4096 .. 16384 points took 37 .. 42 us per call in
-  // one launch and 40 .. 45 us in two; 4096 x 8192 top-1 290 us against 165.
+  // one launch and 40 .. 45 us in two; 4096 x 8192 top-1 290 us against 147.
   const bool one_launch_pays = (uint64_t)beams * nfft <= (1ull << 21);
   if (!plan->big && !plan->bluestein && !plan->huge && one_launch_pays && fused_mlp_supported(plan->g, K)) {
     uint32_t start = params->search_start, end = params->search_end;
@@ -481,7 +481,7 @@ spx_status spx_fft_peaks_mlp(spx_ctx* ctx, spx_mlp* mlp, const void* d_in, uint3
   if (params->thresh_sigma == 0.0f && topk_pair_supported(*plan)) {
     // larger calls of power-of-two beams up to 16384 points: the search keeps the
     // spectrum on chip and hands on the five bins of each peak (4096 x 8192 top-1:
-    // 165 us, and 187 us through the spectrum in device memory)
+    // 147 us, and 167 us through the spectrum in device memory)
     uint32_t start = params->search_start, end = params->search_end;
     resolve_window(nfft, &start, &end);
     const float* win = nullptr;
@@ -549,7 +549,7 @@ spx_status spx_fft_peaks(spx_ctx* ctx, const void* d_in, uint32_t beams, uint32_
     // Top-K of power-of-two beams up to 16384 points without a threshold: one
     // launch of the packed kernel, faster than the scalar fused kernel and than
     // the composed path at every size measured (1 .. 4096 beams of 1024 .. 16384
-    // points, K = 1, 8, 32; e.g. 4096 x 8192 top-1: 141 us against 220, 4096 x
+    // points, K = 1, 8, 32; e.g. 4096 x 8192 top-1: 139 us against 220, 4096 x
     // 16384 top-32: 409 against 528).
     if (!all && !thr && topk_pair_supported(*plan)) {
       const float* win = nullptr;
